@@ -1,0 +1,46 @@
+"""Rows that do not start on a chunk or vector boundary: the chunk-wise ragged kernels at the sizes where a row's first and
+last chunk are shared with its neighbours in every way, and at rows too wide for shared memory."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import CASES, case_id, case_ok, make_w, to_product_blob
+
+pytestmark = pytest.mark.gpu
+
+# one chunk or less, one more than a chunk, half-chunk boundaries, more chunks than lanes, more rows than warps in the
+# grid, and (49154) x read from global memory
+SHAPES = [(7, 5), (40, 33), (37, 48), (19, 1022), (9, 1070), (9001, 46), (3, 49154)]
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[1] == 0], ids=case_id)
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_ragged_rows(wv, case, shape):
+    rows, cols = shape
+    if not case_ok(case, rows, cols):
+        pytest.skip("layout needs aligned cols")
+    f, bw, dt = case
+    w, x = make_w(rows * 7 + cols, rows, cols)
+    ob = O.pack(f, w, rows, cols, bw, dt)
+    y = np.zeros(rows, np.float32)
+    wv.dense.MatVecPackedBlob(to_product_blob(wv, ob), x, y)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    ref, den = wd @ x, np.abs(wd) @ np.abs(x)
+    # float32: at most 24 roundings inside a chunk and over the lanes plus one per 1024 columns, each 2^-24 of sum |w x|;
+    # twice that for the formats with a min, whose |code * scale| may exceed |w|
+    assert np.all(np.abs(y - ref) <= 2 * (24 + cols / 1024) * 2.0 ** -24 * den + 1e-30)
+
+
+def test_ragged_batch_and_neighbours(wv):
+    """Batch rows, and a neighbour's non-finite scale that shares a chunk but no half of it with the row."""
+    rows, cols, batch = 5, 48, 3
+    w, _ = make_w(5, rows, cols)
+    X = np.random.default_rng(6).normal(0, 1, (batch, cols)).astype(np.float32)
+    ob = O.pack("IQ3_S", w, rows, cols)
+    ob.scales[0:3] = np.inf          # row 0 is groups 0 - 2; group 3, in the same chunk as group 2, is row 1's
+    st = wv.weights.FromBlob(to_product_blob(wv, ob))
+    pre, _ = wv.dense.Forward(wv.dense.Layer(cols, rows, wv.dense.ActivationLinear, st), X)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)[1:]
+    ref, den = X @ wd.T, np.abs(X) @ np.abs(wd).T
+    assert np.all(np.isfinite(pre[:, 1:])) and np.all(np.abs(pre[:, 1:] - ref) <= 50 * 2.0 ** -24 * den)
+    assert not np.any(np.isfinite(pre[:, 0]))

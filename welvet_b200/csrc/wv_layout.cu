@@ -199,12 +199,12 @@ int wv_launch_unpack_rows(const WvDevBlob& b, int row, int nrows, float* d_out, 
   return cudaGetLastError() == cudaSuccess ? WV_OK : WV_ECUDA;
 }
 
-// ---------------------------------------------------------------- ragged-shape GEMV
+// ---------------------------------------------------------------- weight-by-weight GEMV
 // One warp per output row, lanes stride over columns, exact dequant + f32 multiply-add,
-// shuffle reduction. Used only when rows are not chunk aligned (cols % 32*J != 0); the
-// config shapes all take the chunked kernels in wv_gemv.cu.
-__global__ void gemv_ragged_kernel(WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
-                                   int batch, int row_begin, int row_end) {
+// shuffle reduction. Left for affine groups that are no multiple of 32 weights; every other ragged
+// shape takes the chunk-wise kernels of wv_gemv_ragged.cu.
+__global__ void gemv_flat_kernel(WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
+                                 int batch, int row_begin, int row_end) {
   const WvFmtInfo fi = wv_fmt_info(b.format);
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -219,12 +219,12 @@ __global__ void gemv_ragged_kernel(WvDevBlob b, const float* __restrict__ x, flo
   }
 }
 
-int wv_launch_gemv_ragged(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end,
-                          cudaStream_t st) {
+int wv_launch_gemv_flat(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end,
+                        cudaStream_t st) {
   long long items = (long long)(row_end - row_begin) * batch;
   if (items <= 0) return WV_OK;
   long long nb = (items + 7) / 8;
   if (nb > 148 * 8) nb = 148 * 8;
-  gemv_ragged_kernel<<<(unsigned)nb, 256, 0, st>>>(b, dx, dy, batch, row_begin, row_end);
+  gemv_flat_kernel<<<(unsigned)nb, 256, 0, st>>>(b, dx, dy, batch, row_begin, row_end);
   return cudaGetLastError() == cudaSuccess ? WV_OK : WV_ECUDA;
 }
