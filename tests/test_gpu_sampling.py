@@ -74,3 +74,20 @@ def test_topk_sample_limits_and_distribution(wv):
     assert set(picks) <= set(top.tolist())
     freq = np.array([(picks == t).mean() for t in top])
     assert np.abs(freq - p).max() < 2e-3
+
+
+@pytest.mark.parametrize("n", [8192, 8193, 8199, 327680, 327681])
+def test_pickers_at_the_cluster_edges(wv, n):
+    """One CTA up to 8192 logits, eight beyond, logits kept in shared memory up to 327680: winners and ties that sit in
+    the last CTA's part, on both sides of a boundary between CTAs, and all over the vector."""
+    per = -(-n // 8)
+    rng = np.random.default_rng(n)
+    cases = [rng.normal(0, 3, n).astype(np.float32), np.zeros(n, np.float32)]
+    c = rng.normal(0, 1, n).astype(np.float32); c[[per - 1, per, n - 1]] = 9.0; cases.append(c)
+    c = np.full(n, -np.inf, np.float32); c[-1] = 1.0; c[n // 2:n // 2 + 30] = 0.5; cases.append(c)
+    for v in cases:
+        d = torch.from_numpy(v).cuda()
+        assert wv.sampling.ArgMaxCUDA(d.data_ptr(), n) == O.argmax(v)
+        for k in (2, 33, 1024):
+            for u in (0.0, 0.4, 1.0):
+                assert wv.sampling.SampleTopKCUDA(d.data_ptr(), n, k, 0.9, False, u) == O.topk_sample(v, k, 0.9, False, u), (k, u)

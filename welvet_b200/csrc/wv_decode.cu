@@ -6,8 +6,11 @@
 // layers/mha/attn.go:15-120, simd/silu.go:14-27, model/transformer/scratch.go:33-41); here sums that
 // decide a normalisation are kept in float64 and the rest is float32.
 #include "wv_common.cuh"
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdlib.h>
+
+namespace cg = cooperative_groups;
 
 // ------------------------------------------------------------------ RMSNorm
 // y[i] = x[i] * inv * gamma[i], inv = 1 / sqrt(sum(x^2) / dim + eps)  (rmsnorm/cpu.go:76-85).
@@ -398,58 +401,110 @@ int wv_launch_residual_add(float* ddst, const float* dadd, int n, cudaStream_t s
 // open; here equal values go by rising index. A NaN logit is ordered by its bit pattern (the reference's order with
 // NaN is whatever its sort happens to do).
 //
-// One CTA. Each logit becomes a 64-bit word (ordered value bits : ~index), all distinct; a most-significant-digit
-// radix select (8 bits a pass, stopping as soon as a bucket holds exactly what is still needed) finds the K-th
-// largest word, the K words at or above it are gathered and sorted by a bitonic network in shared memory, and
-// thread 0 does the two short sequential float64 walks so that the sums round as the reference's do.
+// Each logit becomes a 64-bit word (ordered value bits : ~index), all distinct; a most-significant-digit radix select
+// (11 bits a pass, stopping as soon as a bucket holds exactly what is still needed) finds the K-th largest word, the K
+// words at or above it are gathered and sorted by a bitonic network in shared memory, and one thread does the two short
+// sequential float64 walks so that the sums round as the reference's do.
+//
+// Bound: latency; 128256 logits are 0.5 MB. One cluster of eight CTAs shares the work without any scratch in global
+// memory: a CTA keeps its eighth of the logits in shared memory for all passes, the histograms are added up over
+// distributed shared memory by every CTA for itself (so all take the same decision), and the candidates go to CTA 0.
+// Eleven bits reach two bits into the mantissa, so that a pass's shared-memory atomics spread over more than the few
+// exponents that logits have, and 40 of 128256 are found in two or three passes. One CTA that read the logits from L2
+// in each of its 8-bit passes took 117 us for 40 of 128256 and 18.5 us for 40 of 8192 (back to back on a stream); now
+// 17.0 and 10.7 us.
 #define TOPK_MAX 1024
-__device__ __forceinline__ unsigned long long topk_word(float v, float temperature, int i) {
-  const float val = __fdiv_rn(v, temperature);
-  unsigned u = __float_as_uint(val);
-  u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  return ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)i);
+#define TOPK_THREADS 1024
+#define TOPK_BITS 11
+#define TOPK_BINS (1 << TOPK_BITS)
+#define TOPK_CLUSTER 8
+#define TOPK_SMALL 8192                 // up to here one CTA: a cluster's barriers cost more than eight logits per thread
+#define TOPK_CACHE_BYTES (160 * 1024)   // logits kept in shared memory per CTA (327680 over a cluster); beyond, they are read again
+__device__ __forceinline__ unsigned topk_key(float v, float temperature) {
+  const unsigned u = __float_as_uint(__fdiv_rn(v, temperature));
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-__global__ void __launch_bounds__(1024, 1) topk_sample_kernel(const float* __restrict__ v, int n, int k, float temperature, double u01,
-                                                              int* __restrict__ out) {
-  __shared__ unsigned s_hist[256];
+__global__ void __launch_bounds__(TOPK_THREADS, 1) topk_sample_kernel(const float* __restrict__ v, int n, int k, float temperature, double u01,
+                                                                      int* __restrict__ out, int per, int cached) {
+  extern __shared__ unsigned s_key[];                     // this CTA's keys: logits rank * per ... (+ per), when cached
+  __shared__ __align__(16) unsigned s_hist[2][TOPK_BINS];
   __shared__ unsigned long long s_cand[TOPK_MAX];
   __shared__ double s_p[TOPK_MAX];
+  __shared__ unsigned s_warp[TOPK_THREADS / 32];
   __shared__ unsigned long long s_prefix;
   __shared__ unsigned s_need, s_done, s_count;
-  const int tid = threadIdx.x;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ncta = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = min(n, rank * per), mine = min(n, i0 + per) - i0;
   if (tid == 0) { s_prefix = 0ull; s_need = (unsigned)k; s_done = 0u; s_count = 0u; }
+  for (int i = tid; i < TOPK_BINS; i += TOPK_THREADS) s_hist[0][i] = 0u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (cached) {
+    // eight loads in flight per thread: the copy is one round trip to L2 per 8192 logits
+    for (int b = tid; b < mine; b += 8 * TOPK_THREADS) {
+      float x[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) if (b + q * TOPK_THREADS < mine) x[q] = v[i0 + b + q * TOPK_THREADS];
+#pragma unroll
+      for (int q = 0; q < 8; q++) if (b + q * TOPK_THREADS < mine) s_key[b + q * TOPK_THREADS] = topk_key(x[q], temperature);
+    }
+  }
+  auto word = [&](int i) {                                // i counts from i0
+    const unsigned key = cached ? s_key[i] : topk_key(v[i0 + i], temperature);
+    return ((unsigned long long)key << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)(i0 + i));
+  };
   __syncthreads();
   unsigned long long thresh = 0ull;
-  for (int pass = 0; pass < 8; pass++) {
-    const int shift = 56 - 8 * pass;
-    if (tid < 256) s_hist[tid] = 0u;
-    __syncthreads();
-    const unsigned long long prefix = s_prefix;
-    const unsigned long long himask = pass == 0 ? 0ull : (~0ull << (shift + 8));
-    for (int i = tid; i < n; i += 1024) {
-      const unsigned long long w = topk_word(v[i], temperature, i);
-      if ((w & himask) == prefix) atomicAdd(&s_hist[(unsigned)(w >> shift) & 255u], 1u);
+  int hi = 64;                                            // bits below `hi` are still open
+  for (int pass = 0; hi > 0; pass++) {
+    const int shift = hi > TOPK_BITS ? hi - TOPK_BITS : 0;
+    unsigned* hist = s_hist[pass & 1];
+    const unsigned dmask = (1u << (hi - shift)) - 1u;
+    const unsigned long long prefix = s_prefix, himask = hi == 64 ? 0ull : (~0ull << hi);
+    for (int i = tid; i < mine; i += TOPK_THREADS) {
+      const unsigned long long w = word(i);
+      if ((w & himask) == prefix) atomicAdd(&hist[(unsigned)(w >> shift) & dmask], 1u);
     }
+    cluster.sync();
+    // every CTA is past the previous pass's sums: its histogram may be cleared for the next pass
+    for (int i = tid; i < TOPK_BINS; i += TOPK_THREADS) s_hist[(pass & 1) ^ 1][i] = 0u;
+    // from the top digit down: the bucket where the running count reaches what is still needed. A thread holds two
+    // neighbouring digits, the higher one first.
+    const int d0 = TOPK_BINS - 1 - 2 * tid;
+    unsigned c0 = 0u, c1 = 0u;
+    for (int r = 0; r < ncta; r++) {
+      const uint2 c = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(hist, r) + d0 - 1);
+      c0 += c.y; c1 += c.x;
+    }
+    unsigned incl = c0 + c1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+    if (lane == 31) s_warp[warp] = incl;
+    const unsigned need = s_need;
     __syncthreads();
-    if (tid == 0) {
-      unsigned need = s_need, d = 255u;
-      for (;; d--) {               // from the top digit down: the bucket where the running count reaches `need`
-        const unsigned c = s_hist[d];
-        if (c >= need || d == 0u) { if (c == need) s_done = 1u; break; }
-        need -= c;
-      }
-      s_need = need;
-      s_prefix = prefix | ((unsigned long long)d << shift);
+    for (int q = 0; q < warp; q++) incl += s_warp[q];
+    const unsigned above = incl - c0 - c1;                // candidates in higher digits than this thread's
+    if (above < need && incl >= need) {
+      const bool first = above + c0 >= need;
+      const unsigned left = need - above - (first ? 0u : c0), c = first ? c0 : c1;
+      s_need = left;
+      s_done = c == left;
+      s_prefix = prefix | ((unsigned long long)(first ? d0 : d0 - 1) << shift);
     }
     __syncthreads();
     thresh = s_prefix;             // low digits still zero: every word of the chosen bucket is >= thresh
+    hi = shift;
     if (s_done) break;
   }
-  for (int i = tid; i < n; i += 1024) {
-    const unsigned long long w = topk_word(v[i], temperature, i);
-    if (w >= thresh) { const unsigned slot = atomicAdd(&s_count, 1u); if (slot < TOPK_MAX) s_cand[slot] = w; }
+  unsigned* count0 = cluster.map_shared_rank(&s_count, 0);
+  unsigned long long* cand0 = cluster.map_shared_rank(s_cand, 0);
+  for (int i = tid; i < mine; i += TOPK_THREADS) {
+    const unsigned long long w = word(i);
+    if (w >= thresh) { const unsigned slot = atomicAdd(count0, 1u); if (slot < TOPK_MAX) cand0[slot] = w; }
   }
-  __syncthreads();
+  cluster.sync();
+  if (rank != 0) return;           // nobody reads the other CTAs' memory from here on
   const int cnt = min((int)s_count, TOPK_MAX);   // == k by construction
   int p2 = 1;
   while (p2 < cnt) p2 <<= 1;
@@ -487,6 +542,23 @@ __global__ void __launch_bounds__(1024, 1) topk_sample_kernel(const float* __res
   }
 }
 int wv_launch_topk_sample(const float* d_logits, int n, int k, float temperature, double u01, int* d_out, cudaStream_t st) {
-  topk_sample_kernel<<<1, 1024, 0, st>>>(d_logits, n, k, temperature, u01, d_out);
-  return cudaGetLastError() == cudaSuccess ? WV_OK : WV_ECUDA;
+  static unsigned long long attr_mask = 0;     // the attribute is set once per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(attr_mask & (1ull << dev))) {
+    if (cudaFuncSetAttribute(topk_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TOPK_CACHE_BYTES) != cudaSuccess) return WV_ECUDA;
+    if (dev < 64) attr_mask |= 1ull << dev;
+  }
+  const int ncta = n <= TOPK_SMALL ? 1 : TOPK_CLUSTER;
+  const int per = (n + ncta - 1) / ncta;
+  const int cached = (long long)per * 4 <= TOPK_CACHE_BYTES;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncta); cfg.blockDim = dim3(TOPK_THREADS); cfg.dynamicSmemBytes = cached ? (size_t)per * 4 : 0; cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)ncta; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, topk_sample_kernel, d_logits, n, k, temperature, u01, d_out, per, cached) == cudaSuccess ? WV_OK : WV_ECUDA;
 }
