@@ -1,0 +1,56 @@
+"""Two to five activation rows: every packed layout on whichever kernel takes it, batches that fill a CTA's rows unevenly,
+bands of less than a tile, one and several column warps, and rows up to and beyond the width that leaves the integer-dot
+rows kernel room for its records."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import CASES, case_id, case_ok, make_w
+from test_gpu_batched import _run
+
+pytestmark = pytest.mark.gpu
+
+# rows x cols: fewer rows than SMs, a partial last tile, one column warp, a partial last column warp (1280 = 40 chunks),
+# 4608 (formats that the tensor pipe takes up to 4096), 6144 (the widest in most formats), 14336 (row by row)
+SHAPES = [(5, 512), (300, 1024), (149, 1280), (450, 4096), (40, 4608), (64, 6144), (40, 14336)]
+
+
+def _bound(ob, x):
+    """float32 scales and sums over at most 16 column warps (64 roundings are ample), and an activation off by at most
+    amax / 65024 of its 32-column chunk under 16-bit records."""
+    wd = np.abs(O.unpack(ob).reshape(ob.rows, ob.cols).astype(np.float64))
+    amax = np.abs(x).reshape(-1, 32).max(1).repeat(32)
+    return wd @ (np.abs(x) * 64 * 2.0 ** -24 + amax / 65024) + 1e-30
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[0] != "none"], ids=case_id)
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_rows_every_format(wv, case, shape):
+    rows, cols = shape
+    if not case_ok(case, rows, cols):
+        pytest.skip("layout needs aligned cols")
+    f, bw, dt = case
+    w, _ = make_w(rows + cols, rows, cols)
+    ob = O.pack(f, w, rows, cols, bw, dt)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    rng = np.random.default_rng(cols)
+    for batch in (2, 3, 5):
+        x = rng.normal(0, 1, (batch, cols)).astype(np.float32)
+        x[-1] *= 1e-20
+        x[0, ::97] *= 1e4             # outliers: 24-bit records for this row only
+        y, _ = _run(wv, ob, x)
+        for m in range(batch):
+            err = np.abs(y[m] - wd @ x[m].astype(np.float64))
+            assert np.all(err <= 2 * _bound(ob, x[m])), (batch, m, float(np.max(err / _bound(ob, x[m]))))
+
+
+def test_rows_keep_their_own_infinities(wv):
+    """A non-finite activation makes its own row's outputs NaN and leaves the others alone."""
+    rows, cols = 64, 2048
+    w, _ = make_w(3, rows, cols)
+    ob = O.pack("Q4_K", w, rows, cols)
+    x = np.random.default_rng(4).normal(0, 1, (4, cols)).astype(np.float32)
+    clean, _ = _run(wv, ob, x)
+    x[2, 700] = np.inf
+    y, _ = _run(wv, ob, x)
+    assert np.all(np.isnan(y[2])) and np.array_equal(y[[0, 1, 3]], clean[[0, 1, 3]])

@@ -36,6 +36,7 @@ SOURCES = {
     "wv_gemv_tma.cu": [],
     "wv_gemv_mma.cu": [],
     "wv_gemv_ragged.cu": [],
+    "wv_gemv_rows.cu": [],
     "wv_decode.cu": [],
     "wv_gemv_tc.cu": [],
     "wv_gemm_tcgen05.cu": [],

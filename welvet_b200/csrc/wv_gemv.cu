@@ -721,6 +721,7 @@ static int launch_gemv_regs(const WvDevBlob& b, const float* dx, float* dy, int 
   return WV_EFORMAT;
 }
 
+int wv_launch_gemv_rows(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st);      // wv_gemv_rows.cu
 int wv_launch_gemm_tcgen05(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st);   // wv_gemm_tcgen05.cu
 // Development switch (libraries built with the hooks only): WV_BATCH_LOOP=1 in the environment keeps batches on the
 // one-row-at-a-time kernels, for timing one path against the other.
@@ -748,12 +749,19 @@ int wv_launch_gemv(const WvDevBlob& b, const float* dx, float* dy, int batch, in
   if (row_end <= row_begin || batch <= 0) return WV_OK;
   const WvPeers* pp = wv_cur_peers;
   if (pp && batch != 1) return WV_ESHAPE;
-  // Measured at 4096 x 4096 (L2-resident): the tensor-core kernel costs 17-20 us whatever the batch, a batch-1 launch
-  // 5 us per row, so small batches of a matrix that stays in L2 run row by row; a matrix that does not fit L2 would
-  // be streamed from HBM once per row, so there the tensor-core kernel takes every batch.
+  const bool batched = batch >= 2 && !pp && !wv_cur_fuse && !g_tune_r && !wv_tma_tuning_rt() && !batch_loop_forced();   // a kernel forced by a tuning code keeps the batch on it
+  // A few rows: up to four per pass over W on the integer-dot kernel, which is more precise than the tensor cores' TF32.
+  // At 4096 x 4096 in Q4_K four rows take 11.1 us there, 22.8 on the tensor-core kernel, 18.8 row by row; from six rows
+  // (two passes, 18.9) the tensor-core kernel's time, which hardly depends on the batch, is the better one.
+  if (batched && batch < batch_min()) {
+    const int rc = wv_launch_gemv_rows(b, dx, dy, batch, row_begin, row_end, st);
+    if (rc != 1) return rc;
+  }
+  // What that kernel does not take of a matrix that does not fit L2 would be streamed from HBM once per row, so there the
+  // tensor-core kernel takes every batch.
   const WvFmtInfo bfi = wv_fmt_info(b.format);
   const bool big = (double)b.n * (bfi.bits_lo + bfi.bits_hi) / 8.0 > 64e6;
-  if ((batch >= batch_min() || (batch >= 2 && big)) && !pp && !wv_cur_fuse && !g_tune_r && !wv_tma_tuning_rt() && !batch_loop_forced()) {   // a kernel forced by a tuning code keeps the batch on it
+  if (batched && (batch >= batch_min() || big)) {
     // Several activation rows: the tensor-core kernel streams and dequantises the matrix once for up to 256 of
     // them. What it does not take (FormatNone, ragged rows) runs row by row below.
     int rc = wv_launch_gemm_tcgen05(b, dx, dy, batch < 256 ? batch : 256, row_begin, row_end, st);
