@@ -144,3 +144,40 @@ def test_host_pointer_calls_from_threads(wv):
         t.join()
     assert not errors, errors[:3]
     assert wv._lib.lib().wv_device_status() == 0
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[0] != "none"], ids=case_id)
+@pytest.mark.parametrize("shape", [(130, 96), (40, 544), (200, 1056), (140, 1536), (129, 4352)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_batched_column_orders(wv, case, shape):
+    """Chunk counts that leave the four producer groups unequal runs, a part of a load unit or nothing at all, rows that do
+    not start on a load unit (17 and 33 chunks), and one and two rounds of stages (batches up to 64 and beyond)."""
+    rows, cols = shape
+    if not case_ok(case, rows, cols):
+        pytest.skip("layout needs aligned cols")
+    f, bw, dt = case
+    w = np.random.default_rng(cols).normal(0, 0.02, rows * cols).astype(np.float32)
+    ob = O.pack(f, w, rows, cols, bw, dt)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    for batch in (6, 64, 65, 256):
+        x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
+        y, _ = _run(wv, ob, x)
+        # two operands rounded to 11 bits, as derived beside the kernel
+        assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch
+
+
+@pytest.mark.parametrize("fmt", ["Q4_0", "Q4_K", "IQ3_S", "TernaryPacked", "IQ1_S"])
+def test_batched_non_finite_parameters(wv, fmt):
+    """A row whose scales are infinite or NaN comes out non-finite, as its dequantised weights are; its neighbours do not."""
+    rows, cols, batch = 130, 512, 9
+    w = np.random.default_rng(1).normal(0, 0.02, rows * cols).astype(np.float32)
+    ob = O.pack(fmt, w, rows, cols)
+    per_row = (len(ob.scales) if len(ob.scales) else len(ob.raw)) // rows
+    for r, bad in ((3, np.inf), (77, np.nan)):
+        if len(ob.scales):
+            ob.scales[r * per_row] = bad
+        else:
+            ob.raw[r * per_row:r * per_row + 4] = np.frombuffer(np.float32(bad).tobytes(), np.uint8)     # the first block's scale
+    x = np.random.default_rng(2).normal(0, 1, (batch, cols)).astype(np.float32)
+    y, _ = _run(wv, ob, x)
+    assert not np.any(np.isfinite(y[:, [3, 77]]))
+    assert np.all(np.isfinite(np.delete(y, [3, 77], axis=1)))

@@ -3,12 +3,23 @@
 //
 // The reference runs dense.Forward row by row over the batch (layers/dense/simd.go:557-614 per row,
 // gemv_parallel.go:12-391); its WebGPU shaders do the same per dispatch. Here the batch is the N dimension of a
-// tcgen05.mma: a CTA owns 128 rows of W (the MMA's M) and a range of the columns (split-K); per 32 columns its 512
-// producer threads dequantise a 128 x 32 slice of W to TF32 values in the canonical K-major 128-byte-swizzled
-// operand layout in shared memory and stage the matching slice of X (rounded to TF32) beside it, one elected thread
-// issues four tcgen05.mma (M 128, N = batch padded to 16, K 8) per slice into a TMEM accumulator, tcgen05.commit
-// hands the stage back, and at the end four warps read the accumulator with tcgen05.ld and store Y (or the split's
-// partial, which the last split of the row tile to finish adds up in split order).
+// tcgen05.mma: a CTA owns 128 rows of W (the MMA's M) and a range of the columns (split-K). A pipeline stage is a
+// 32-column slice. The 512 producer threads form four groups of 128 (a thread per row); each group owns a run of
+// consecutive columns and the groups' slices go through the pipeline in turn, so that a thread reads its row 128 bits to
+// 64 bytes at a time although every slice is one chunk wide (the order in which slices are summed is free as long as X
+// takes the same one). A thread dequantises a 32-weight chunk to TF32 values in the canonical K-major 128-byte-swizzled
+// operand layout; one thread copies the matching slice of X (rounded to TF32 by a kernel in front) beside it, one elected
+// thread issues four tcgen05.mma (M 128, N = batch padded to 16, K 8) per slice into a TMEM accumulator, and
+// tcgen05.commit hands the stage back. At the end all producer warps read the accumulator with tcgen05.ld; the splits of
+// a row tile are one thread-block cluster, which adds its accumulators up in split order through distributed shared
+// memory.
+//
+// Bound: up to some 64 rows the producers' instruction stream (five instructions per weight) together with the MMAs, which
+// take about 52 cycles each however few rows X has; at 256 rows the copies of X out of L2 (every row tile reads all of it) and
+// the tensor pipe. Measured against the version before (512 producers of 8 weights each, two slices a stage, issue loops run
+// by one lane, split sums through global memory), 16 / 64 / 256 rows: Q8_0 4096 x 4096 21.7 / 28.3 / 56.9 -> 15.9 / 18.2 /
+// 26.2 us, Q4_K 14336 x 4096 66.2 / 67.6 / 82.0 -> 36.6 / 41.9 / 55.2 us, Q4_0 1024 x 1024 12.0 / 18.2 / 42.6 -> 8.1 / 9.3 /
+// 15.4 us. With the loads and the conversion left out the 14336 x 4096 launch takes 15.5 us at 16 rows.
 //
 // Arithmetic: both operands are rounded to TF32 (round to nearest, 11 significant bits) by the producers, so the
 // hardware's truncation of the low mantissa bits drops zeros; products are exact in the FP32 accumulator. Each term
@@ -17,7 +28,7 @@
 //
 // Every wait is bounded: a wait that runs out records a code in the mapped error word, raises the CTA's abort flag,
 // and all roles fall through to the common exit, where the TMEM columns are released.
-#include "wv_common.cuh"
+#include "wv_gemv_common.cuh"
 #include "wv_tma_common.cuh"
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -25,101 +36,182 @@
 
 #define TCG_PRODUCERS 512
 #define TCG_THREADS (TCG_PRODUCERS + 64)     // + the MMA warp and the warp whose first lane issues the X copies
-#define TCG_MAX_STAGES 6
 #define TCG_M 128
-#define TCG_KB 2            // 32-column slices per pipeline stage
+#define TCG_GROUPS (TCG_PRODUCERS / TCG_M)
+#define TCG_MAX_STAGES (2 * TCG_GROUPS)
+#define TCG_MAX_SPLIT 8     // portable cluster size
 
-__constant__ float c_tcg_iq4nl[16] = WV_IQ4NL_GRID;
-
-// ------------------------------------------------------------------ dequantisation of a quarter chunk (8 weights)
-// The unpack kernel's arithmetic with the parameters of the 8 weights hoisted. The values are rounded to TF32 right
-// after, so the two places where the reference divides (k-quant scale / 255, min / 127) multiply by the reciprocal
-// here: the difference is one unit in the 24th bit, against the rounding to 11 bits that follows.
-struct TcgRaw { unsigned lo[2]; unsigned hi[2]; float p0, p1; unsigned km; };
-
-// q (0..3) names the 8 weights of chunk ch; the four threads that share a chunk are neighbouring lanes, so that a
-// warp's loads fall into whole 32-byte sectors (8 rows x 4 quarters per warp).
-template <int F>
-__device__ __forceinline__ void tcg_load_raw(TcgRaw& r, const WvDevBlob& b, long long ch, int q) {
-  constexpr WvFmtInfo fi = wv_fmt_info(F);
-  constexpr int BL = fi.bits_lo, BH = fi.bits_hi;
-  const int half = q >> 1;
-  if constexpr (BL == 8) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(b.lo + ch * 8) + q); r.lo[0] = v.x; r.lo[1] = v.y; }
-  else if constexpr (BL == 4) r.lo[0] = __ldg(b.lo + ch * 4 + q);
-  else if constexpr (BL == 2) r.lo[0] = __ldg(b.lo + ch * 2 + half) >> (16 * (q & 1));
-  else r.lo[0] = __ldg(b.lo + ch) >> (8 * q);
-  if constexpr (BH >= 1) r.hi[0] = __ldg(b.hi + ch * BH);
-  if constexpr (BH == 2) r.hi[1] = __ldg(b.hi + ch * BH + 1);
-  const long long i = ch * 32 + q * 8;   // flat index of the first weight
-  if constexpr (fi.kind == WK_CLASSIC) {
-    r.p0 = __ldg(b.p0 + ch);
-    if constexpr (fi.has_min) r.p1 = __ldg(b.p1 + ch);
-  } else if constexpr (fi.kind == WK_KQUANT) {
-    const float2 dd = __ldg(reinterpret_cast<const float2*>(b.p0) + (ch >> 3));
-    r.p0 = dd.x; r.p1 = dd.y;
-    if constexpr (fi.has_min) r.km = __ldg(b.km + ch);
-    else r.km = __ldg(reinterpret_cast<const unsigned short*>(b.km) + ch);
-  } else if constexpr (fi.kind == WK_IQ || fi.kind == WK_TERNARY) {
-    r.p0 = __ldg(b.p0 + (fi.pgroup == 16 ? ch * 2 + half : ch));
-  } else if constexpr (fi.kind == WK_BINARY) {
-    r.p0 = __ldg(b.p0 + i / b.group);
-  } else if constexpr (fi.kind == WK_AFFINE) {
-    r.p0 = __ldg(b.p0 + i / b.group);
-    r.p1 = __ldg(b.p1 + i / b.group);
-  }
-}
-
-template <int F>
-__device__ __forceinline__ void tcg_convert(const TcgRaw& r, int q, float (&w)[8]) {
-  constexpr WvFmtInfo fi = wv_fmt_info(F);
-  constexpr int BL = fi.bits_lo, BH = fi.bits_hi;
-  const int half = q >> 1;
-  float sc = r.p0, mn = 0.f;
-  if constexpr (fi.kind == WK_CLASSIC) { if constexpr (fi.has_min) mn = r.p1; }
-  if constexpr (fi.kind == WK_AFFINE) mn = r.p1;
-  if constexpr (fi.kind == WK_KQUANT) {
-    const unsigned su = (r.km >> (8 * half)) & 0xffu;
-    sc = r.p0 * (float)(su ? su : 1u) * (1.0f / 255.0f);    // a zero scale byte stands for d / 255 (quant/kquant.go:180-182)
-    if constexpr (fi.has_min) {
-      const unsigned mu = (r.km >> (16 + 8 * half)) & 0xffu;
-      mn = r.p1 * (float)(int)(signed char)mu * (1.0f / 127.0f);
-    }
-  }
-  // code -> float without an integer conversion: the code lands in the mantissa of 2^23, and subtracting
-  // 2^23 + mid leaves (code - mid) exactly
-  constexpr float magic = 8388608.0f + (float)((fi.kind == WK_CLASSIC || fi.kind == WK_KQUANT) && !fi.has_min ? fi.mid : 0);
+// ------------------------------------------------------------------ weight loads
+template <int N> __device__ __forceinline__ void tcg_words(unsigned (&d)[N], const void* p) {
+  if constexpr (N == 1) d[0] = __ldg(reinterpret_cast<const unsigned*>(p));
+  else if constexpr (N == 2) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(p)); d[0] = v.x; d[1] = v.y; }
+  else if constexpr (N == 4) { const uint4 v = __ldg(reinterpret_cast<const uint4*>(p)); d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w; }
+  else {
+    static_assert(N % 8 == 0, "whole 256-bit loads");
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    constexpr unsigned mask = (1u << BL) - 1u;
-    unsigned u = (r.lo[(j * BL) >> 5] >> ((j * BL) & 31)) & mask;
-    unsigned ubits = u | 0x4B000000u;
-    if constexpr (BL == 8 && BH == 0) ubits = __byte_perm(r.lo[j >> 2], 0x4B000000u, 0x7440u + (unsigned)(j & 3));   // one instruction: byte j under the exponent of 2^23
+    for (int i = 0; i < N; i += 8)
+      asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(d[i]), "=r"(d[i + 1]), "=r"(d[i + 2]), "=r"(d[i + 3]), "=r"(d[i + 4]), "=r"(d[i + 5]), "=r"(d[i + 6]), "=r"(d[i + 7])
+                   : "l"(reinterpret_cast<const char*>(p) + 4 * i));
+  }
+}
+// A thread's unit of loading: U consecutive chunks of its row, 64 bytes of the lo plane at most. The 32 lanes of a warp are 32
+// rows, so every load touches 32 different lines and the L1 tag stage is what limits them: few wide loads, not many narrow ones
+// (chunk by chunk the tag stage was busy for 17 of the 39 thousand cycles of a 4096 x 4096 Q8_0 launch).
+template <int F> struct TcgUnit { static constexpr int U = wv_fmt_info(F).bits_lo == 8 ? 2 : 4; };
+
+// VEC: the row's first chunk and the unit's are multiples of U chunks, so that every plane is read with one or two aligned
+// vector loads; otherwise chunk by chunk. cnt: chunks of the unit that exist (VEC reads all U: rows are whole units).
+template <int F, bool VEC>
+__device__ __forceinline__ void tcg_load(FragT<F> (&f)[TcgUnit<F>::U], const WvDevBlob& b, long long ch, int cnt) {
+  constexpr WvFmtInfo fi = wv_fmt_info(F);
+  constexpr int U = TcgUnit<F>::U, BL = fi.bits_lo, BH = fi.bits_hi;
+  if constexpr (!VEC) {
+#pragma unroll
+    for (int u = 0; u < U; u++) if (u < cnt) load_frag<F>(f[u], b, ch + u);
+  } else {
+    unsigned lo[U * BL];
+    tcg_words(lo, b.lo + ch * BL);
+#pragma unroll
+    for (int i = 0; i < U * BL; i++) f[i / BL].lo[i % BL] = lo[i];
     if constexpr (BH > 0) {
-      const int jj = q * 8 + j;
-      const int k = wv_k_of(BL, jj), m = wv_m_of(BL, jj);
-      const unsigned hw = (BH == 2 && wv_hi_word(BH, k)) ? r.hi[1] : r.hi[0];
-      u |= ((hw >> wv_hi_bit(BH, k, m)) & ((1u << BH) - 1u)) << BL;
+      unsigned hi[U * BH];
+      tcg_words(hi, b.hi + ch * BH);
+#pragma unroll
+      for (int i = 0; i < U * BH; i++) f[i / BH].hi[i % BH] = hi[i];
     }
-    if constexpr (BH > 0) ubits = u | 0x4B000000u;
-    const float uf = __uint_as_float(ubits) - magic;     // (code - mid) for the symmetric block formats, the code otherwise
-    float v;
-    if constexpr (fi.kind == WK_CLASSIC || fi.kind == WK_KQUANT) v = fi.has_min ? fmaf(uf, sc, mn) : uf * sc;
-    else if constexpr (fi.kind == WK_IQ) {
-      if constexpr (fi.table) v = sc * c_tcg_iq4nl[u & 15];
-      else if constexpr (fi.sign) v = (u & 1) ? sc : -sc;
-      else v = sc * (uf - ((float)fi.mid + 0.5f));
+    if constexpr (fi.kind == WK_KQUANT) {          // a unit lies inside one super-block of eight chunks
+      const float2 dd = __ldg(reinterpret_cast<const float2*>(b.p0) + (ch >> 3));
+      unsigned km[U];
+      if constexpr (fi.has_min) tcg_words(km, b.km + ch);
+      else {
+        unsigned k2[U / 2];
+        tcg_words(k2, reinterpret_cast<const unsigned short*>(b.km) + ch);
+#pragma unroll
+        for (int u = 0; u < U; u++) km[u] = (k2[u / 2] >> (16 * (u & 1))) & 0xffffu;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) { f[u].pr[0] = __float_as_uint(dd.x); f[u].pr[1] = __float_as_uint(dd.y); f[u].pr[2] = km[u]; }
+    } else if constexpr (fi.kind == WK_BINARY || fi.kind == WK_AFFINE) {
+      const unsigned cpg = (unsigned)b.group >> 5;   // whole chunks per group
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const unsigned gi = (unsigned)(ch + u) / cpg;
+        f[u].pr[0] = __float_as_uint(__ldg(b.p0 + gi));
+        if constexpr (fi.has_min) f[u].pr[1] = __float_as_uint(__ldg(b.p1 + gi));
+      }
+    } else {
+      constexpr int NG = fi.pgroup == 16 ? 2 : 1;
+      unsigned p0[U * NG];
+      tcg_words(p0, b.p0 + ch * NG);
+#pragma unroll
+      for (int i = 0; i < U * NG; i++) f[i / NG].pr[i % NG] = p0[i];
+      if constexpr (fi.has_min) {
+        unsigned p1[U];
+        tcg_words(p1, b.p1 + ch);
+#pragma unroll
+        for (int u = 0; u < U; u++) f[u].pr[1] = p1[u];
+      }
     }
-    else if constexpr (fi.kind == WK_TERNARY) v = u == 0 ? -sc : (u == 2 ? sc : 0.0f);
-    else if constexpr (fi.kind == WK_BINARY) v = (u & 1) ? sc : -sc;
-    else v = fmaf(sc, uf, mn);   // affine
-    w[j] = v;
   }
 }
 
+// ------------------------------------------------------------------ dequantisation of a chunk (32 weights)
 __device__ __forceinline__ float tcg_tf32(float v) {
   unsigned o;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(o) : "f"(v));
   return __uint_as_float(o);
+}
+// Round to nearest, ties away from zero, as cvt.rna.tf32 does (which costs several instructions here): half a unit of the
+// eleventh bit is added to the magnitude; the tensor core reads a TF32 operand's upper 19 bits and ignores the rest
+// (clearing them first changes no bit of any output). `half` is
+// zero for chunks whose parameters are not finite, so that a NaN's mantissa cannot run over (a finite value may round
+// up to infinity, as it does with cvt.rna).
+__device__ __forceinline__ float tcg_round(float v, unsigned half) { return __uint_as_float(__float_as_uint(v) + half); }
+__device__ __forceinline__ bool tcg_finite(unsigned bits) { return (bits & 0x7f800000u) != 0x7f800000u; }
+
+// The unpack kernel's arithmetic with the parameters hoisted. The two places where the reference divides (k-quant scale
+// / 255, min / 127) multiply by the reciprocal here: the difference is one unit in the 24th bit, against the rounding
+// to 11 bits that follows. piece(p, v): the weights 4 p .. 4 p + 3.
+template <int F, typename P>
+__device__ __forceinline__ void tcg_convert(const FragT<F>& f, const float* tbl, P piece) {
+  constexpr WvFmtInfo fi = wv_fmt_info(F);
+  constexpr int BL = fi.bits_lo, BH = fi.bits_hi, SPW = 8 / BL;
+  constexpr unsigned MASK = 0x01010101u * ((1u << BL) - 1u);
+  constexpr unsigned MASKH = BH ? (0x01010101u * ((1u << BH) - 1u)) << BL : 0u;
+  float sc[2], mn[2] = {0.f, 0.f};
+  bool fin = tcg_finite(f.pr[0]);
+  if constexpr (fi.kind == WK_KQUANT) {
+    const float d = __uint_as_float(f.pr[0]);
+    if constexpr (fi.has_min) fin = fin && tcg_finite(f.pr[1]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      // scale bytes of zero were stored as 1 at upload: both stand for d / 255 (quant/kquant.go:180-182)
+      sc[h] = d * (float)(unsigned char)(f.pr[2] >> (8 * h)) * (1.0f / 255.0f);
+      if constexpr (fi.has_min) mn[h] = __uint_as_float(f.pr[1]) * (float)(signed char)(f.pr[2] >> (16 + 8 * h)) * (1.0f / 127.0f);
+    }
+  } else {
+    sc[0] = sc[1] = __uint_as_float(f.pr[0]);
+    if constexpr (fi.pgroup == 16) { sc[1] = __uint_as_float(f.pr[1]); fin = fin && tcg_finite(f.pr[1]); }
+    if constexpr (fi.has_min) { mn[0] = mn[1] = __uint_as_float(f.pr[1]); fin = fin && tcg_finite(f.pr[1]); }
+  }
+  const unsigned half = fin ? 0x1000u : 0u;
+  if constexpr (fi.sign) {                           // +- scale: rounded once, the code is its sign
+    const unsigned r = __float_as_uint(tcg_round(sc[0], half));
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] = __uint_as_float(r ^ ((~f.lo[0] << (31 - (4 * p + q))) & 0x80000000u));
+      piece(p, v);
+    }
+    return;
+  }
+  // code -> float without an integer conversion: the code lands in the mantissa of 2^23, and subtracting 2^23 + mid
+  // leaves (code - mid) exactly. Groups of SPW words' worth of codes complete SPW pieces of four consecutive weights each.
+  constexpr float magic = 8388608.0f + (float)fi.mid;
+  float w[4 * SPW];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int s = k % SPW;
+    unsigned bytes = (f.lo[k / SPW] >> (BL * s)) & MASK;      // the codes of group k, one per byte
+    if constexpr (BH > 0) {
+      const int hw = (k * BH) >> 3, sh = (k * BH) & 7;
+      unsigned hv = f.hi[hw];
+      hv = sh >= BL ? (hv >> (sh - BL)) : (hv << (BL - sh));
+      bytes |= hv & MASKH;
+    }
+    const int h = k >> 2;                                    // groups 0-3 are the first 16 weights
+    float v[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      if constexpr (fi.table) v[m] = sc[h] * tbl[(bytes >> (8 * m)) & 0xffu];
+      else v[m] = __uint_as_float(__byte_perm(bytes, 0x4B000000u, 0x7650 + m));
+    }
+    if constexpr (!fi.table) {
+#pragma unroll
+      for (int m = 0; m < 4; m += 2) {
+        float2 q = __fadd2_rn(make_float2(v[m], v[m + 1]), make_float2(-magic, -magic));
+        if constexpr (fi.half_mid) q = __fadd2_rn(q, make_float2(-0.5f, -0.5f));
+        if constexpr (fi.has_min) q = __ffma2_rn(q, make_float2(sc[h], sc[h]), make_float2(mn[h], mn[h]));
+        else if constexpr (fi.kind == WK_TERNARY) {           // zero whatever the scale
+          q.x = q.x == 0.f ? 0.f : q.x * sc[h];
+          q.y = q.y == 0.f ? 0.f : q.y * sc[h];
+        } else q = __fmul2_rn(q, make_float2(sc[h], sc[h]));
+        v[m] = q.x; v[m + 1] = q.y;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; m++) w[m * SPW + s] = tcg_round(v[m], half);
+    if (s == SPW - 1) {
+      const int j0 = (k / SPW) * 4 * SPW;                     // first weight of these SPW groups
+#pragma unroll
+      for (int p = 0; p < SPW; p++) {
+        const float o[4] = {w[4 * p], w[4 * p + 1], w[4 * p + 2], w[4 * p + 3]};
+        piece(j0 / 4 + p, o);
+      }
+    }
+  }
 }
 
 // ------------------------------------------------------------------ tcgen05 plumbing
@@ -154,40 +246,83 @@ struct TcgGeom {
   int row_begin, row_end;     // rows of the blob this launch covers
   int cpr;                    // chunks (32 columns) per row
   int batch, npad;            // activation rows, and that padded to a multiple of 16 (the MMA's N)
-  int ksplit, cps;            // column splits and chunks per split
-  int nstage;
-  unsigned a_bytes, b_bytes, stage_bytes;   // one slice of A (128 rows x 128 bytes) and of B; a stage holds TCG_KB of each
+  int ksplit, cps;            // column splits (= cluster size) and chunks per split
+  int rounds;                 // rounds of TCG_GROUPS stages in the ring: 2, or 1 where the activations leave no room
+  unsigned b_bytes, stage_bytes;            // a stage: one slice of A (128 rows x 128 bytes), then one of B (npad x 128 bytes)
   unsigned tmem_cols;         // power of two >= max(32, npad)
   int y_stride;               // floats between consecutive activation rows' outputs
 };
 
-template <int F, int D>   // D: stages whose weight loads are in flight
+#define TCG_A_BYTES (TCG_M * 128u)
+
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster(unsigned saddr, int rank) {
+  unsigned a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// The column order of a CTA: its nk chunks are units of U; group q owns the chunks first .. first + n, the first groups one
+// unit more where they do not divide. Round i takes one chunk of every group that has an i-th one: those are always the
+// first active(i) groups.
+struct TcgOrder {
+  int first[TCG_GROUPS], n[TCG_GROUPS];      // in chunks
+  __device__ __forceinline__ TcgOrder(int nk, int U) {
+    const int nu = (nk + U - 1) / U, base = nu / TCG_GROUPS, rem = nu % TCG_GROUPS;
+#pragma unroll
+    for (int q = 0; q < TCG_GROUPS; q++) {
+      first[q] = (base * q + min(q, rem)) * U;
+      n[q] = max(0, min((base + (q < rem ? 1 : 0)) * U, nk - first[q]));
+    }
+  }
+  __device__ __forceinline__ int active(int i) const {
+    int a = 0;
+#pragma unroll
+    for (int q = 0; q < TCG_GROUPS; q++) a += i < n[q] ? 1 : 0;
+    return a;
+  }
+};
+
+// grid (row tiles, splits), cluster (1, splits)
+template <int F, bool VEC>
 __global__ void __launch_bounds__(TCG_THREADS, 1)
-gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap, float* __restrict__ y, float* __restrict__ part,
-                    unsigned* __restrict__ counters, const TcgGeom g, int* __restrict__ err) {
+gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap, float* __restrict__ y, const TcgGeom g, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char tcg_smem[];
   __shared__ __align__(8) unsigned long long s_bar[2 * TCG_MAX_STAGES + 1];
   __shared__ unsigned s_tmem;
   __shared__ int s_abort;
-  __shared__ unsigned s_last;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ float s_tbl[16];          // IQ4_NL's grid
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // one value per warp, and the compiler knows it
   const int mt = blockIdx.x, sp = blockIdx.y;
   const int m0 = g.row_begin + mt * TCG_M;
   const int kc0 = sp * g.cps, kc1 = min(g.cpr, kc0 + g.cps);
-  const int nk = max(0, kc1 - kc0);
-  const int nst = (nk + TCG_KB - 1) / TCG_KB;    // pipeline stages to work through
+  constexpr int U = TcgUnit<F>::U;
+  const int nst = max(0, kc1 - kc0);             // slices = pipeline stages to work through
+  const TcgOrder order(nst, U);
   // the dynamic segment is declared 1024-byte aligned; round up all the same (the swizzle pattern is relative to 1024 bytes)
   const unsigned sbase = (smem_u32(tcg_smem) + 1023u) & ~1023u;
+  // The ring: round i's slice of group q is stage (i mod rounds) * 4 + q, in its (i / rounds)-th use
   auto full_bar = [&](int s) { return smem_u32(&s_bar[s]); };
   auto empty_bar = [&](int s) { return smem_u32(&s_bar[TCG_MAX_STAGES + s]); };
   const unsigned done_bar = smem_u32(&s_bar[2 * TCG_MAX_STAGES]);
+  const int rsh = g.rounds - 1;                  // log2(rounds)
+  auto stage_of = [&](int i, int q) { return (i & rsh) * TCG_GROUPS + q; };
 
   if (tid == 0) {
     s_abort = 0;
-    for (int s = 0; s < g.nstage; s++) { mbar_init(full_bar(s), TCG_PRODUCERS / 32 + 1); mbar_init(empty_bar(s), 1); }
+    for (int s = 0; s < TCG_MAX_STAGES; s++) { mbar_init(full_bar(s), TCG_M / 32 + 1); mbar_init(empty_bar(s), 1); }
     mbar_init(done_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (wv_fmt_info(F).table && tid < 16) s_tbl[tid] = c_grid4nl[tid];
   if (warp == TCG_PRODUCERS / 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(g.tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -195,119 +330,113 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   tcg_fence_before();
   __syncthreads();
   tcg_fence_after();
-  const unsigned tmem = *(volatile unsigned*)&s_tmem;
+  const unsigned tmem = __shfl_sync(0xffffffffu, *(volatile unsigned*)&s_tmem, 0);
   // The weights do not depend on the preceding kernel: the producers start at once. Only the thread that copies X waits
   // for it (X was rounded by the kernel right before this one), and nothing is stored before X has arrived.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp < TCG_PRODUCERS / 32) {
     // ------------------------------------------------------------ producers
-    const int row_l = tid >> 2;
-    const int quarter = tid & 3;                                 // which 8 of a chunk's 32 weights
+    const int grp = warp / (TCG_M / 32);                         // owns a run of the CTA's columns
+    const int row_l = tid & (TCG_M - 1);
     const int row = min(m0 + row_l, g.row_end - 1);              // rows past the end repeat the last one and are not stored
-    const long long ch_row = (long long)row * g.cpr;
-    // this thread's part of the A slice: 32 bytes of row row_l, 16-byte pieces quarter*2, quarter*2+1, swizzled by the row
-    const unsigned a_off = (unsigned)(row_l >> 3) * 1024u + (unsigned)(row_l & 7) * 128u;
-    // A stage holds TCG_KB consecutive 32-column slices (the barrier traffic and the loop's bookkeeping are paid per
-    // stage, not per slice). Loads run D stages ahead of the conversion (they take about a microsecond to come back):
-    // D register sets, the stage loop unrolled by D so that they are indexed statically.
-    TcgRaw raw[D][TCG_KB];
-    auto load = [&](TcgRaw (&r)[TCG_KB], int it) {
-#pragma unroll
-      for (int kb = 0; kb < TCG_KB; kb++) {
-        const int kc = kc0 + it * TCG_KB + kb;
-        if (kc < kc1) tcg_load_raw<F>(r[kb], b, ch_row + kc, quarter);
-      }
-    };
-#pragma unroll
-    for (int d = 0; d < D; d++) if (d < nst) load(raw[d], d);
-    int s = 0;
-    unsigned epar = 1;     // parity of the "empty" phase to wait for once the ring has wrapped
-    bool wrapped = false;
+    const int mine = order.n[0] * (grp == 0) + order.n[1] * (grp == 1) + order.n[2] * (grp == 2) + order.n[3] * (grp == 3);
+    const long long ch0 = (long long)row * g.cpr + kc0 + order.first[0] * (grp == 0) + order.first[1] * (grp == 1) + order.first[2] * (grp == 2) + order.first[3] * (grp == 3);
+    // this thread's part of the A slice: row row_l, its 16-byte pieces swizzled by the row; eight lanes of a store phase
+    // have eight different rows mod 8 and so cover all banks
+    const unsigned a_off = (unsigned)(row_l >> 3) * 1024u + (unsigned)(row_l & 7) * (128u + 16u);
+    // one unit ahead: its loads travel while the current unit is converted
+    FragT<F> nxt[U];
+    if (mine > 0) tcg_load<F, VEC>(nxt, b, ch0, mine);
     bool dead = false;
-    for (int it0 = 0; it0 < nst && !dead; it0 += D) {
+    for (int i0 = 0; i0 < mine && !dead; i0 += U) {
+      FragT<F> cur[U];
 #pragma unroll
-      for (int d = 0; d < D; d++) {
-        const int it = it0 + d;
-        if (it >= nst || dead) break;
+      for (int u = 0; u < U; u++) cur[u] = nxt[u];
+      if (i0 + U < mine) tcg_load<F, VEC>(nxt, b, ch0 + i0 + U, mine - i0 - U);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u;
+        if (i >= mine || dead) break;
         bool bad = *(volatile int*)&s_abort != 0;
-        if (!bad && wrapped && !mbar_wait(empty_bar(s), epar)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
+        const int s = stage_of(i, grp), use = i >> rsh;
+        if (!bad && use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
         if (__any_sync(0xffffffffu, bad)) { dead = true; break; }     // the whole warp leaves together (it meets at __syncwarp below)
-        const unsigned st = sbase + (unsigned)s * g.stage_bytes;
-#pragma unroll
-        for (int kb = 0; kb < TCG_KB; kb++) {
-          if (kc0 + it * TCG_KB + kb >= kc1) break;    // past the split's last slice: the MMA thread skips it too
-          float w[8];
-          tcg_convert<F>(raw[d][kb], quarter, w);
-#pragma unroll
-          for (int p = 0; p < 2; p++) {
-            const unsigned piece = (unsigned)(quarter * 2 + p) ^ (unsigned)(row_l & 7);
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(st + kb * g.a_bytes + a_off + piece * 16u), "f"(tcg_tf32(w[4 * p])),
-                         "f"(tcg_tf32(w[4 * p + 1])), "f"(tcg_tf32(w[4 * p + 2])), "f"(tcg_tf32(w[4 * p + 3])) : "memory");
-          }
-        }
-        if (it + D < nst) load(raw[d], it + D);
+        const unsigned st = sbase + (unsigned)s * g.stage_bytes + a_off;
+        tcg_convert<F>(cur[u], s_tbl, [&](int p, const float (&v)[4]) {
+          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(st ^ (16u * p)), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+        });
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(full_bar(s));      // one arrival per warp
-        if (++s == g.nstage) { s = 0; wrapped = true; epar ^= 1u; }
       }
     }
   } else if (warp == TCG_PRODUCERS / 32 + 1) {
-    // ------------------------------------------------------------ X copies (one thread): a stage's slices of the rounded
-    // activations arrive by tensor-map copies with the 128-byte swizzle, i.e. already in the operand layout; rows past
-    // the batch are zero-filled by the copy engine
-    if (lane == 0) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      int s = 0;
-      unsigned epar = 1;
-      bool wrapped = false;
-      for (int it = 0; it < nst; it++) {
-        if (*(volatile int*)&s_abort) break;
-        if (wrapped && !mbar_wait(empty_bar(s), epar)) { atomicCAS_system(err, 0, 530 + s); *(volatile int*)&s_abort = 1; break; }
-        const int nkb = min(TCG_KB, nk - it * TCG_KB);
-        mbar_expect_tx(full_bar(s), (unsigned)nkb * g.b_bytes);
-        const unsigned st = sbase + (unsigned)s * g.stage_bytes + TCG_KB * g.a_bytes;
-        for (int kb = 0; kb < nkb; kb++) tma_load_2d(st + kb * g.b_bytes, &xmap, (kc0 + it * TCG_KB + kb) * 32, 0, full_bar(s));
-        if (++s == g.nstage) { s = 0; wrapped = true; epar ^= 1u; }
+    // ------------------------------------------------------------ X copies: a stage's slice of the rounded activations arrives
+    // by a tensor-map copy with the 128-byte swizzle, i.e. already in the operand layout; rows past the batch are zero-filled
+    // by the copy engine. Here and in the MMA warp the whole warp runs the loop and one elected lane issues: the operands
+    // of these instructions live in uniform registers, and from a loop that only lane 0 ran, which the compiler cannot know to be
+    // uniform, every stage cost some 450 cycles of issue: 64 us instead of 36 for 16 rows at 14336 x 4096 in Q4_K, whatever
+    // else the kernel did.
+    const bool leader = elect_one();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    bool run = true;
+    for (int i = 0; i < order.n[0] && run; i++) {
+      const int use = i >> rsh, na = order.active(i);
+#pragma unroll
+      for (int q = 0; q < TCG_GROUPS; q++) {
+        if (q >= na || !run) break;
+        const int s = stage_of(i, q);
+        if (use > 0 && __any_sync(0xffffffffu, !mbar_wait(empty_bar(s), (use - 1) & 1))) { atomicCAS_system(err, 0, 530 + s); *(volatile int*)&s_abort = 1; run = false; break; }
+        if (leader) {
+          mbar_expect_tx(full_bar(s), g.b_bytes);
+          tma_load_2d(sbase + (unsigned)s * g.stage_bytes + TCG_A_BYTES, &xmap, (kc0 + order.first[q] + i) * 32, 0, full_bar(s));
+        }
+        __syncwarp();
       }
     }
-  } else if (lane == 0) {
-    // ------------------------------------------------------------ MMA issuer (one thread)
+  } else {
+    // ------------------------------------------------------------ MMA issuer
+    const bool leader = elect_one();
     const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(g.npad >> 3) << 17) | ((unsigned)(TCG_M >> 4) << 24);
-    int s = 0;
-    unsigned fpar = 0;
-    for (int it = 0; it < nst; it++) {
-      if (*(volatile int*)&s_abort) break;
-      if (!mbar_wait(full_bar(s), fpar)) { atomicCAS_system(err, 0, 510 + s); *(volatile int*)&s_abort = 1; break; }
-      tcg_fence_after();
-      const unsigned st = sbase + (unsigned)s * g.stage_bytes;
+    bool run = true;
+    for (int i = 0; i < order.n[0] && run; i++) {
+      const int na = order.active(i);
 #pragma unroll
-      for (int kb = 0; kb < TCG_KB; kb++) {
-        if (it * TCG_KB + kb >= nk) break;       // the split's last stage may hold one slice only
-        const unsigned long long da = tcg_desc(st + kb * g.a_bytes), db = tcg_desc(st + TCG_KB * g.a_bytes + kb * g.b_bytes);
+      for (int q = 0; q < TCG_GROUPS; q++) {
+        if (q >= na || !run) break;
+        const int s = stage_of(i, q);
+        if (__any_sync(0xffffffffu, !mbar_wait(full_bar(s), (i >> rsh) & 1))) { atomicCAS_system(err, 0, 510 + s); *(volatile int*)&s_abort = 1; run = false; break; }
+        tcg_fence_after();
+        if (leader) {
+          const unsigned st = sbase + (unsigned)s * g.stage_bytes;
+          const unsigned long long da = tcg_desc(st), db = tcg_desc(st + TCG_A_BYTES);
 #pragma unroll
-        for (int k = 0; k < 4; k++)   // 8 TF32 values = 32 bytes further along K inside the swizzled row
-          tcg_mma_tf32(tmem, da + (unsigned long long)(2 * k), db + (unsigned long long)(2 * k), idesc, (it > 0 || kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < 4; k++)   // 8 TF32 values = 32 bytes further along K inside the swizzled row
+            tcg_mma_tf32(tmem, da + (unsigned long long)(2 * k), db + (unsigned long long)(2 * k), idesc, (i > 0 || q > 0 || k > 0) ? 1u : 0u);
+          tcg_commit(empty_bar(s));        // arrives when these MMAs have read the stage
+        }
+        __syncwarp();
       }
-      tcg_commit(empty_bar(s));        // arrives when these MMAs have read the stage
-      if (++s == g.nstage) { s = 0; fpar ^= 1u; }
     }
-    tcg_commit(done_bar);               // arrives when every MMA issued above has finished
+    if (leader) tcg_commit(done_bar);      // arrives when every MMA issued above has finished
+    __syncwarp();
   }
 
-  // ---------------------------------------------------------------- epilogue: warps 0-3 own TMEM lanes 32 w .. 32 w + 31
-  float* dst = g.ksplit == 1 ? y : part + ((size_t)mt * g.ksplit + sp) * (size_t)g.batch * TCG_M;
-  if (warp < 4) {
+  // ---------------------------------------------------------------- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (the
+  // quarter a warp may access), 16 columns out of every 64. A split's accumulator waits in the ring's memory, which nothing
+  // uses any more once every MMA has finished (each stage that was filled has been read by one).
+  float* acc = reinterpret_cast<float*>(tcg_smem + (sbase - smem_u32(tcg_smem)));    // [batch][128]
+  if (warp < TCG_PRODUCERS / 32) {
     bool ok = !*(volatile int*)&s_abort;
-    if (ok && nk > 0 && !mbar_wait(done_bar, 0)) { atomicCAS_system(err, 0, 520); *(volatile int*)&s_abort = 1; ok = false; }
+    if (ok && !mbar_wait(done_bar, 0)) { atomicCAS_system(err, 0, 520); *(volatile int*)&s_abort = 1; ok = false; }
     ok = __all_sync(0xffffffffu, ok);     // tcgen05.ld is warp-wide
     tcg_fence_after();
-    const int row_l = warp * 32 + lane;
+    const int row_l = (warp & 3) * 32 + lane;
     const bool row_ok = m0 + row_l < g.row_end;
-    for (int c0 = 0; c0 < g.npad; c0 += 16) {
+    for (int c0 = (warp >> 2) * 16; c0 < g.npad && ok; c0 += 64) {
       float v[16];
-      if (ok && nk > 0) tcg_ld16(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0, v);
+      if (nst > 0) tcg_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0, v);
       else {
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = 0.f;
@@ -316,43 +445,39 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
       for (int j = 0; j < 16; j++) {
         const int m = c0 + j;
         if (m < g.batch) {
-          if (g.ksplit == 1) { if (row_ok) dst[(size_t)m * g.y_stride + m0 + row_l] = v[j]; }
-          else dst[(size_t)m * TCG_M + row_l] = v[j];
+          if (g.ksplit == 1) { if (row_ok) y[(size_t)m * g.y_stride + m0 + row_l] = v[j]; }
+          else acc[m * TCG_M + row_l] = v[j];
         }
       }
     }
   }
   tcg_fence_before();
-  if (g.ksplit > 1) __threadfence();
   __syncthreads();
   if (warp == TCG_PRODUCERS / 32) {
     tcg_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(g.tmem_cols) : "memory");
   }
   if (g.ksplit == 1) return;
-  // ---------------------------------------------------------------- the last split of this row tile adds the partials up, in split order
-  if (tid == 0) {
-    const unsigned prev = atomicAdd(&counters[mt], 1u);
-    s_last = (prev == (unsigned)g.ksplit - 1u);
-    if (s_last) counters[mt] = 0u;   // ready for the next launch
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const float* base = part + (size_t)mt * g.ksplit * (size_t)g.batch * TCG_M;
-  const size_t per = (size_t)g.batch * TCG_M;
-  for (int e = tid; e < g.batch * TCG_M; e += TCG_THREADS) {
-    const int m = e / TCG_M, row_l = e - m * TCG_M;
-    float v[8];
+  // ---------------------------------------------------------------- the cluster adds its accumulators up in split order: CTA sp
+  // stores every ksplit-th activation row's 128 sums. Every thread of every CTA reaches both barriers on all paths.
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  const unsigned acc_s = smem_u32(acc);
+  for (int e = tid; ; e += TCG_THREADS) {
+    const int m = (e / TCG_M) * g.ksplit + sp, row_l = e & (TCG_M - 1);
+    if (m >= g.batch) break;
+    float v[TCG_MAX_SPLIT];
+#pragma unroll
+    for (int u = 0; u < TCG_MAX_SPLIT; u++) if (u < g.ksplit) v[u] = ld_cluster(acc_s + 4u * (unsigned)(m * TCG_M + row_l), u);
     float sum = 0.f;
-    for (int s0 = 0; s0 < g.ksplit; s0 += 8) {
 #pragma unroll
-      for (int u = 0; u < 8; u++) v[u] = s0 + u < g.ksplit ? __ldcg(base + (size_t)(s0 + u) * per + e) : 0.f;
-#pragma unroll
-      for (int u = 0; u < 8; u++) if (s0 + u < g.ksplit) sum += v[u];
-    }
+    for (int u = 0; u < TCG_MAX_SPLIT; u++) if (u < g.ksplit) sum += v[u];
     if (m0 + row_l < g.row_end) y[(size_t)m * g.y_stride + m0 + row_l] = sum;
   }
+  __syncwarp();
+  cluster_arrive();      // the other CTAs may still be reading this one's sums
+  cluster_wait();
 }
 
 // X rounded to TF32 (round to nearest), element for element.
@@ -381,16 +506,52 @@ static PFN_cuTensorMapEncodeTiled_v12000 tcg_encode_fn() {
   }
   return fn;
 }
-static float* g_tcg_part = nullptr;
-static size_t g_tcg_part_floats = 0;
-static unsigned* g_tcg_cnt = nullptr;
-static int g_tcg_cnt_n = 0;
 static std::mutex g_tcg_mu;
 
 int wv_sm_count();
 
-template <int F>
+// Column splits for `mtiles` row tiles of `cpr` chunks: the splits of a tile are one cluster, and how many clusters of each
+// size run at once is a property of the chip (a cluster lives inside one GPC). The estimate counts waves of clusters,
+// each costing its slices plus some 24 slices' worth of start-up and epilogue; equal costs go to the smaller split.
+static int tcg_cps(int cpr, int ks, int unit) { return ((cpr + ks - 1) / ks + unit - 1) / unit * unit; }    // chunks per split, whole units
+template <typename K>
+static int tcg_splits(K kern, int dev, int mtiles, int cpr, int unit) {
+  static int active[64][TCG_MAX_SPLIT + 1] = {};       // resident clusters of each size, per device (0: not asked yet)
+  if (dev < 0 || dev >= 64) return 1;
+  int best = 1;
+  long long cost = -1;
+  for (int ks = 1; ks <= TCG_MAX_SPLIT && (ks == 1 || cpr / ks >= 8); ks++) {      // at least 8 chunks (256 columns) per split
+    const int cps = tcg_cps(cpr, ks, unit);
+    if ((cpr + cps - 1) / cps != ks) continue;          // every split of a cluster has columns
+    if (!active[dev][ks]) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, ks); cfg.blockDim = dim3(TCG_THREADS); cfg.dynamicSmemBytes = 200 * 1024;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = ks; at[0].val.clusterDim.z = 1;
+      cfg.attrs = at; cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = -1; }
+      active[dev][ks] = n;
+    }
+    const int n = ks == 1 ? wv_sm_count() : active[dev][ks];
+    if (n < 1) continue;
+    const long long c = (long long)((mtiles + n - 1) / n) * (cps + 24);
+    if (cost < 0 || c < cost) { cost = c; best = ks; }
+  }
+  return best;
+}
+
+template <int F, bool VEC>
 static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
+  auto kern = gemm_tcgen05_kernel<F, VEC>;
+  static unsigned attr_mask = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(attr_mask & (1u << (dev & 31)))) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024) != cudaSuccess) { wv_set_error("batched matvec: cannot raise the shared-memory limit"); return WV_ECUDA; }
+    attr_mask |= 1u << (dev & 31);
+  }
   TcgGeom g{};
   g.row_begin = rb; g.row_end = re;
   g.cpr = b.cols >> 5;
@@ -399,47 +560,16 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
   g.y_stride = b.rows;
   const int rows = re - rb;
   const int mtiles = (rows + TCG_M - 1) / TCG_M;
-  // column splits: enough CTAs for the SMs, at least 8 chunks (256 columns) per split
-  int ks = wv_sm_count() / mtiles;
-  if (ks > g.cpr / 8) ks = g.cpr / 8;
-  if (ks < 1) ks = 1;
-  g.cps = (g.cpr + ks - 1) / ks;
-  g.ksplit = (g.cpr + g.cps - 1) / g.cps;
-  g.a_bytes = TCG_M * 128u;
+  const int unit = VEC ? TcgUnit<F>::U : 1;
+  const int ks = tcg_splits(kern, dev, mtiles, g.cpr, unit);
+  g.cps = tcg_cps(g.cpr, ks, unit);
+  g.ksplit = ks;
   g.b_bytes = (unsigned)g.npad * 128u;
-  g.stage_bytes = TCG_KB * (g.a_bytes + g.b_bytes);
-  int ns = (int)((200u * 1024u) / g.stage_bytes);
-  if (ns > TCG_MAX_STAGES) ns = TCG_MAX_STAGES;
-  if (ns < 2) return 1;
-  g.nstage = ns;
+  g.stage_bytes = TCG_A_BYTES + g.b_bytes;
+  g.rounds = TCG_MAX_STAGES * g.stage_bytes <= 200u * 1024u ? 2 : 1;      // two up to 64 rows; one round of 256 rows takes 192 KB
   g.tmem_cols = 32;
   while ((int)g.tmem_cols < g.npad) g.tmem_cols *= 2;
-  const size_t smem = (size_t)ns * g.stage_bytes + 1024;
-  float* part = nullptr;
-  unsigned* cnt = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_tcg_mu);
-    if (g.ksplit > 1) {
-      const size_t need = (size_t)mtiles * g.ksplit * batch * TCG_M;
-      if (need > g_tcg_part_floats) {       // grows when a larger shape arrives (set-up time: not capturable)
-        cudaStreamSynchronize(st);
-        if (g_tcg_part) cudaFree(g_tcg_part);
-        g_tcg_part = nullptr; g_tcg_part_floats = 0;
-        if (cudaMalloc(&g_tcg_part, need * 4) != cudaSuccess) { cudaGetLastError(); wv_set_error("batched matvec: %zu bytes of split scratch unavailable", need * 4); return WV_ENOMEM; }
-        g_tcg_part_floats = need;
-      }
-      if (mtiles > g_tcg_cnt_n) {
-        cudaStreamSynchronize(st);
-        if (g_tcg_cnt) cudaFree(g_tcg_cnt);
-        g_tcg_cnt = nullptr; g_tcg_cnt_n = 0;
-        const int n = mtiles < 4096 ? 4096 : mtiles;
-        if (cudaMalloc(&g_tcg_cnt, (size_t)n * 4) != cudaSuccess) { cudaGetLastError(); wv_set_error("batched matvec: counter allocation failed"); return WV_ENOMEM; }
-        cudaMemset(g_tcg_cnt, 0, (size_t)n * 4);
-        g_tcg_cnt_n = n;
-      }
-    }
-    part = g_tcg_part; cnt = g_tcg_cnt;
-  }
+  const size_t smem = (size_t)g.rounds * TCG_GROUPS * g.stage_bytes + 1024;
   // X rounded to TF32 once, by a small kernel in front (each of the row tiles would otherwise round it again), into a
   // buffer of the library; the main kernel fetches it through a tensor map encoded per call.
   float* xr = nullptr;
@@ -466,20 +596,14 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
     if (enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, xr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
   }
-  auto kern = gemm_tcgen05_kernel<F, 4>;
-  static unsigned attr_mask = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(attr_mask & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024) != cudaSuccess) { wv_set_error("batched matvec: cannot raise the shared-memory limit"); return WV_ECUDA; }
-    attr_mask |= 1u << (dev & 31);
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(mtiles, g.ksplit); cfg.blockDim = dim3(TCG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)g.ksplit; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = g.ksplit > 1 ? 2 : 1;
   int* err = wv_tma_err_ptr();
   {
     const size_t n4 = (size_t)batch * b.cols / 4;
@@ -492,7 +616,7 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
       wv_set_error("batched matvec (rounding) launch: %s", cudaGetErrorString(cudaGetLastError())); return WV_ECUDA;
     }
   }
-  if (cudaLaunchKernelEx(&cfg, kern, b, xmap, dy, part, cnt, g, err) != cudaSuccess) { wv_set_error("batched matvec launch: %s", cudaGetErrorString(cudaGetLastError())); return WV_ECUDA; }
+  if (cudaLaunchKernelEx(&cfg, kern, b, xmap, dy, g, err) != cudaSuccess) { wv_set_error("batched matvec launch: %s", cudaGetErrorString(cudaGetLastError())); return WV_ECUDA; }
   return WV_OK;
 }
 
@@ -502,7 +626,7 @@ int wv_launch_gemm_tcgen05(const WvDevBlob& b, const float* dx, float* dy, int b
   if (batch < 2 || batch > 256 || !b.fast || b.format == WV_NONE || (b.cols & 31) || row_end <= row_begin) return 1;
   if ((reinterpret_cast<uintptr_t>(dx) & 15) || !wv_tma_err_ptr()) return 1;
   switch (b.format) {
-#define WV_F(f) case f: return launch_tcg<f>(b, dx, dy, batch, row_begin, row_end, st);
+#define WV_F(f) case f: return (b.cols >> 5) % TcgUnit<f>::U ? launch_tcg<f, false>(b, dx, dy, batch, row_begin, row_end, st) : launch_tcg<f, true>(b, dx, dy, batch, row_begin, row_end, st);
   WV_F(WV_Q8_0) WV_F(WV_Q4_0) WV_F(WV_Q4_1) WV_F(WV_Q5_0) WV_F(WV_Q5_1)
   WV_F(WV_Q2_K) WV_F(WV_Q3_K) WV_F(WV_Q4_K) WV_F(WV_Q5_K) WV_F(WV_Q6_K)
   WV_F(WV_IQ1_S) WV_F(WV_IQ2_XXS) WV_F(WV_IQ2_XS) WV_F(WV_IQ3_XXS) WV_F(WV_IQ3_S) WV_F(WV_IQ4_NL) WV_F(WV_IQ4_XS)
