@@ -9,8 +9,9 @@ from conftest import CASES, case_id, case_ok, make_w, to_product_blob
 pytestmark = pytest.mark.gpu
 
 # one chunk or less, one more than a chunk, half-chunk boundaries, more chunks than lanes, more rows than warps in the
-# grid, and (49154) x read from global memory
-SHAPES = [(7, 5), (40, 33), (37, 48), (19, 1022), (9, 1070), (9001, 46), (3, 49154)]
+# grid, shared memory just below 48 KB (11500, before any wider row), above it and at its limit (49150), and (49154) x
+# read from global memory
+SHAPES = [(7, 5), (40, 33), (37, 48), (19, 1022), (9, 1070), (9001, 46), (4, 11500), (5, 20001), (3, 49150), (3, 49154)]
 
 
 @pytest.mark.parametrize("case", [c for c in CASES if c[1] == 0], ids=case_id)

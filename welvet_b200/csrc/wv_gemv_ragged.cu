@@ -193,7 +193,9 @@ static int rag_go(K kern, bool xs, const WvDevBlob& b, const float* dx, float* d
   const size_t smem = xs ? ((size_t)b.cols + 96 + (b.cols + 96) / 32 + 1) * 4 : 0;
   int dev = 0;
   cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && !(attr_mask & (1u << (dev & 31)))) {
+  // Whatever the size: the limit without the attribute is 48 KB for static and dynamic memory together, and IQ4_NL's
+  // table makes 2 KB of the static kind.
+  if (xs && !(attr_mask & (1u << (dev & 31)))) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) { wv_set_error("gemv (ragged): cannot raise the shared-memory limit"); return WV_ECUDA; }
     attr_mask |= 1u << (dev & 31);
   }
