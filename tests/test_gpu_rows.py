@@ -54,3 +54,19 @@ def test_rows_keep_their_own_infinities(wv):
     x[2, 700] = np.inf
     y, _ = _run(wv, ob, x)
     assert np.all(np.isnan(y[2])) and np.array_equal(y[[0, 1, 3]], clean[[0, 1, 3]])
+
+
+@pytest.mark.parametrize("fmt,cols", [("Q4_K", 2048), ("Q6_K", 2048), ("TernaryPacked", 2048), ("IQ3_S", 2048), ("Q4_0", 4608), ("Q5_0", 4608)])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf])
+def test_infinite_activations_give_nan(wv, fmt, cols, bad):
+    """An infinity among ordinary values, in the formats without a min (whose sums hold nothing that is NaN by itself) as
+    well: the rows kernel and the one-row kernel make the row's outputs NaN, never a number or an infinity of some sign."""
+    rows = 40
+    w, _ = make_w(9, rows, cols)
+    ob = O.pack(fmt, w, rows, cols)
+    x = np.random.default_rng(10).normal(0, 1, (4, cols)).astype(np.float32)
+    x[2, 700] = bad
+    y, _ = _run(wv, ob, x)
+    assert np.all(np.isnan(y[2])) and np.all(np.isfinite(y[[0, 1, 3]]))
+    one, _ = _run(wv, ob, x[2:3])
+    assert np.all(np.isnan(one))

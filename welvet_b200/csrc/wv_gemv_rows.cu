@@ -249,7 +249,8 @@ gemv_rows_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restri
     float ta = amax, ts = (as[0] + as[1]) + (as[2] + as[3]);
 #pragma unroll
     for (int o = 16; o; o >>= 1) { ta += __shfl_xor_sync(0xffffffffu, ta, o); ts += __shfl_xor_sync(0xffffffffu, ts, o); }
-    const bool wide = !(ta <= 0.25f * ts) || g.wide;      // NaN compares false: non-finite input takes 24 bits
+    // NaN compares false and an infinity fails the second test (ta and ts are both infinite then): non-finite input takes 24 bits
+    const bool wide = !(ta <= 0.25f * ts && ts <= 3.4e38f) || g.wide;
     if (lane == 0) s_wide[m][wc] = wide;
     if (wide) {
       XQRegs q;

@@ -554,7 +554,8 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     float ta = amax, ts = asum;
 #pragma unroll
     for (int o = 16; o; o >>= 1) { ta += __shfl_xor_sync(0xffffffffu, ta, o); ts += __shfl_xor_sync(0xffffffffu, ts, o); }
-    const bool wide = !(ta <= 0.25f * ts) || g.force3;   // NaN compares false: non-finite input takes the wide path
+    // NaN compares false and an infinity fails the second test (ta and ts are both infinite then): non-finite input takes the wide path
+    const bool wide = !(ta <= 0.25f * ts && ts <= 3.4e38f) || g.force3;
     if (!wide) {
       XQRegs2 xr;
       if (live) {
