@@ -181,3 +181,25 @@ def test_batched_non_finite_parameters(wv, fmt):
     y, _ = _run(wv, ob, x)
     assert not np.any(np.isfinite(y[:, [3, 77]]))
     assert np.all(np.isfinite(np.delete(y, [3, 77], axis=1)))
+
+
+@pytest.mark.parametrize("fmt,header,mid_code", [("Q6_K", 24, 32), ("Q4_K", 40, 0)])
+def test_batched_scale_that_overflows(wv, fmt, header, mid_code):
+    """A super-block whose d is finite and whose group scale d * byte is not: the group's weights of code zero are NaN, as
+    dequantisation defines them, and so is the row; the rows beside it keep their values."""
+    rows, cols, batch = 130, 512, 9
+    w = np.random.default_rng(3).normal(0, 0.02, rows * cols).astype(np.float32)
+    ob = O.pack(fmt, w, rows, cols)
+    bits = {32: 6, 0: 4}[mid_code]
+    per_row = len(ob.raw) // rows
+    blk = ob.raw[5 * per_row:5 * per_row + header + 32 * bits]
+    blk[:4] = np.frombuffer(np.float32(3e38).tobytes(), np.uint8)
+    blk[8:24] = 1                                    # every group d / 255 ...
+    blk[8] = 255                                     # ... but the first: infinite
+    code = np.array([mid_code >> (i % bits) & 1 for i in range(256 * bits)], np.uint8)
+    blk[header:] = np.packbits(code, bitorder="little")
+    wd = O.unpack(ob).reshape(rows, cols)
+    assert np.all(np.isnan(wd[5, :16])) and np.all(np.isfinite(wd[5, 16:]))
+    x = np.random.default_rng(4).normal(0, 1, (batch, cols)).astype(np.float32)
+    y, _ = _run(wv, ob, x)
+    assert np.all(np.isnan(y[:, 5])) and np.all(np.isfinite(np.delete(y, 5, axis=1)))

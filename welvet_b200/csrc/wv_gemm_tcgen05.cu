@@ -125,8 +125,9 @@ __device__ __forceinline__ float tcg_tf32(float v) {
 // Round to nearest, ties away from zero, as cvt.rna.tf32 does (which costs several instructions here): half a unit of the
 // eleventh bit is added to the magnitude; the tensor core reads a TF32 operand's upper 19 bits and ignores the rest
 // (clearing them first changes no bit of any output). `half` is
-// zero for chunks whose parameters are not finite, so that a NaN's mantissa cannot run over (a finite value may round
-// up to infinity, as it does with cvt.rna).
+// zero for chunks whose scales or mins are not finite, so that a NaN's mantissa cannot run over (a finite value may round
+// up to infinity, as it does with cvt.rna). The products with the scale bytes count, not the stored parameters: a finite d can
+// give an infinite scale, and that times a code of zero is a NaN.
 __device__ __forceinline__ float tcg_round(float v, unsigned half) { return __uint_as_float(__float_as_uint(v) + half); }
 __device__ __forceinline__ bool tcg_finite(unsigned bits) { return (bits & 0x7f800000u) != 0x7f800000u; }
 
@@ -140,10 +141,9 @@ __device__ __forceinline__ void tcg_convert(const FragT<F>& f, const float* tbl,
   constexpr unsigned MASK = 0x01010101u * ((1u << BL) - 1u);
   constexpr unsigned MASKH = BH ? (0x01010101u * ((1u << BH) - 1u)) << BL : 0u;
   float sc[2], mn[2] = {0.f, 0.f};
-  bool fin = tcg_finite(f.pr[0]);
+  bool fin = true;
   if constexpr (fi.kind == WK_KQUANT) {
     const float d = __uint_as_float(f.pr[0]);
-    if constexpr (fi.has_min) fin = fin && tcg_finite(f.pr[1]);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       // scale bytes of zero were stored as 1 at upload: both stand for d / 255 (quant/kquant.go:180-182)
@@ -152,9 +152,11 @@ __device__ __forceinline__ void tcg_convert(const FragT<F>& f, const float* tbl,
     }
   } else {
     sc[0] = sc[1] = __uint_as_float(f.pr[0]);
-    if constexpr (fi.pgroup == 16) { sc[1] = __uint_as_float(f.pr[1]); fin = fin && tcg_finite(f.pr[1]); }
-    if constexpr (fi.has_min) { mn[0] = mn[1] = __uint_as_float(f.pr[1]); fin = fin && tcg_finite(f.pr[1]); }
+    if constexpr (fi.pgroup == 16) sc[1] = __uint_as_float(f.pr[1]);
+    if constexpr (fi.has_min) mn[0] = mn[1] = __uint_as_float(f.pr[1]);
   }
+#pragma unroll
+  for (int h = 0; h < 2; h++) fin = fin && tcg_finite(__float_as_uint(sc[h])) && (!fi.has_min || tcg_finite(__float_as_uint(mn[h])));
   const unsigned half = fin ? 0x1000u : 0u;
   if constexpr (fi.sign) {                           // +- scale: rounded once, the code is its sign
     const unsigned r = __float_as_uint(tcg_round(sc[0], half));
