@@ -91,3 +91,13 @@ def test_pickers_at_the_cluster_edges(wv, n):
         for k in (2, 33, 1024):
             for u in (0.0, 0.4, 1.0):
                 assert wv.sampling.SampleTopKCUDA(d.data_ptr(), n, k, 0.9, False, u) == O.topk_sample(v, k, 0.9, False, u), (k, u)
+
+
+def test_argmax_of_the_largest_vector(wv):
+    """2^31 - 1 values, the most the entry's count can say, with the winner in the last place."""
+    n = 2 ** 31 - 1
+    d = torch.zeros(n, device="cuda")
+    d[-1] = 1.0
+    assert wv.sampling.ArgMaxCUDA(d.data_ptr(), n) == n - 1
+    d[n // 2] = 1.0
+    assert wv.sampling.ArgMaxCUDA(d.data_ptr(), n) == n // 2

@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(TOPK_THREADS, 1) topk_sample_kernel(const floa
   cg::cluster_group cluster = cg::this_cluster();
   const int ncta = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int i0 = min(n, rank * per), mine = min(n, i0 + per) - i0;
+  const int i0 = min(n, rank * per), mine = min(n - i0, per);
   if (tid == 0) { s_prefix = 0ull; s_need = (unsigned)k; s_done = 0u; s_count = 0u; }
   for (int i = tid; i < TOPK_BINS; i += TOPK_THREADS) s_hist[0][i] = 0u;
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -550,7 +550,7 @@ int wv_launch_topk_sample(const float* d_logits, int n, int k, float temperature
     if (dev < 64) attr_mask |= 1ull << dev;
   }
   const int ncta = n <= TOPK_SMALL ? 1 : TOPK_CLUSTER;
-  const int per = (n + ncta - 1) / ncta;
+  const int per = (n - 1) / ncta + 1;
   const int cached = (long long)per * 4 <= TOPK_CACHE_BYTES;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncta); cfg.blockDim = dim3(TOPK_THREADS); cfg.dynamicSmemBytes = cached ? (size_t)per * 4 : 0; cfg.stream = st;

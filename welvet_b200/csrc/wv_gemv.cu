@@ -553,13 +553,13 @@ __global__ void __launch_bounds__(1024, 1) argmax_kernel(const float* __restrict
   if (ncta > 1) cluster.barrier_arrive();      // waited for below: every CTA runs before anything is stored into CTA 0
   float best = first;
   int bi = 0;
-  const int i0 = min(n, rank * per), i1 = min(n, i0 + per);
-  for (int b = i0 + tid; b < i1; b += 8 * 1024) {
+  const int i0 = min(n, rank * per), mine = min(n - i0, per);     // positions count from i0: no sum passes n, whatever n is
+  for (int b = tid; b < mine; b += 8 * 1024) {
     float x[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) x[q] = b + q * 1024 < i1 ? v[b + q * 1024] : first;     // `first` never exceeds best
+    for (int q = 0; q < 8; q++) x[q] = b + q * 1024 < mine ? v[i0 + b + q * 1024] : first;     // `first` never exceeds best
 #pragma unroll
-    for (int q = 0; q < 8; q++) if (x[q] > best) { best = x[q]; bi = b + q * 1024; }    // indices rise within a thread: ties keep the earliest
+    for (int q = 0; q < 8; q++) if (x[q] > best) { best = x[q]; bi = i0 + b + q * 1024; }      // indices rise within a thread: ties keep the earliest
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -600,7 +600,7 @@ int wv_launch_argmax(const float* d_logits, int n, int* d_out, cudaStream_t st) 
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = (unsigned)ncta; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, argmax_kernel, d_logits, n, d_out, n > 0 ? (n + ncta - 1) / ncta : 0) == cudaSuccess ? WV_OK : WV_ECUDA;
+  return cudaLaunchKernelEx(&cfg, argmax_kernel, d_logits, n, d_out, n > 0 ? (n - 1) / ncta + 1 : 0) == cudaSuccess ? WV_OK : WV_ECUDA;
 }
 
 thread_local const WvPeers* wv_cur_peers = nullptr;
