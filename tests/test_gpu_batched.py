@@ -203,3 +203,69 @@ def test_batched_scale_that_overflows(wv, fmt, header, mid_code):
     x = np.random.default_rng(4).normal(0, 1, (batch, cols)).astype(np.float32)
     y, _ = _run(wv, ob, x)
     assert np.all(np.isnan(y[:, 5])) and np.all(np.isfinite(np.delete(y, 5, axis=1)))
+
+
+def _packed(wv, fmt, rows, cols, seed):
+    w = np.random.default_rng(seed).normal(0, 0.02, rows * cols).astype(np.float32)
+    blob = wv.quant.Pack(wv.quant.Format(O.FMT[fmt]), w, rows, cols)
+    return wv.quant.EnsureResident(blob), blob
+
+
+def test_batched_calls_on_many_streams(wv):
+    """Batched calls in flight on 20 streams at once (more than the library keeps buffers for), each with activations of its
+    own: every one gives the bits it gives alone."""
+    rows, cols, batch, n = 20000, 2048, 24, 20
+    L = wv._lib.lib()
+    key, _keep = _packed(wv, "Q8_0", rows, cols, 30)
+    x = torch.randn(n, batch, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(31))
+    alone, y = torch.zeros(n, batch, rows, device="cuda"), torch.zeros(n, batch, rows, device="cuda")
+    for i in range(n):
+        wv._lib.check(L.wv_matvec_dev(key, x[i].data_ptr(), alone[i].data_ptr(), batch, cols, rows, None))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    for _ in range(3):
+        y.zero_()
+        torch.cuda.synchronize()
+        for i, s in enumerate(streams):
+            wv._lib.check(L.wv_matvec_dev(key, x[i].data_ptr(), y[i].data_ptr(), batch, cols, rows, s.cuda_stream))
+        torch.cuda.synchronize()
+        assert torch.equal(alone, y)
+    assert L.wv_device_status() == 0
+
+
+def test_batched_calls_in_graphs(wv):
+    """Two captured batched calls replayed on two streams while the stream they were captured on makes larger calls: the
+    graphs' buffers are their own, and outlive the growth of the stream's."""
+    rows, cols = 20000, 2048
+    L = wv._lib.lib()
+    key, _keep = _packed(wv, "Q4_K", rows, cols, 32)
+    gen = torch.Generator("cuda").manual_seed(33)
+    side = torch.cuda.Stream()
+    jobs = []
+    for batch in (8, 20):
+        x, y = torch.randn(batch, cols, device="cuda", generator=gen), torch.zeros(batch, rows, device="cuda")
+        with torch.cuda.stream(side):
+            wv._lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, rows, side.cuda_stream))
+        torch.cuda.synchronize()
+        want = y.clone()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            wv._lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, rows, torch.cuda.current_stream().cuda_stream))
+        jobs.append((g, x, y, want))
+    xb, yb = torch.randn(256, cols, device="cuda", generator=gen), torch.zeros(256, rows, device="cuda")
+    wv._lib.check(L.wv_matvec_dev(key, xb.data_ptr(), yb.data_ptr(), 256, cols, rows, side.cuda_stream))
+    torch.cuda.synchronize()
+    wantb = yb.clone()
+    streams = [torch.cuda.Stream() for _ in jobs]
+    for _ in range(3):
+        yb.zero_()
+        for _, _, y, _ in jobs:
+            y.zero_()
+        torch.cuda.synchronize()
+        for (g, _, _, _), s in zip(jobs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        wv._lib.check(L.wv_matvec_dev(key, xb.data_ptr(), yb.data_ptr(), 256, cols, rows, side.cuda_stream))
+        torch.cuda.synchronize()
+        assert torch.equal(yb, wantb) and all(torch.equal(y, want) for _, _, y, want in jobs)
+    assert L.wv_device_status() == 0

@@ -32,7 +32,9 @@
 #include "wv_tma_common.cuh"
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <atomic>
 #include <mutex>
+#include <vector>
 
 #define TCG_PRODUCERS 512
 #define TCG_THREADS (TCG_PRODUCERS + 64)     // + the MMA warp and the warp whose first lane issues the X copies
@@ -493,22 +495,110 @@ __global__ void __launch_bounds__(256) tcg_round_x_kernel(const float4* __restri
 }
 
 // ------------------------------------------------------------------ host side
-static float* g_tcg_xr = nullptr;
-static size_t g_tcg_xr_floats = 0;
 static PFN_cuTensorMapEncodeTiled_v12000 tcg_encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {     // once, whichever thread is first
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    else cudaGetLastError();
-  }
+      return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    cudaGetLastError();
+    return nullptr;
+  }();
   return fn;
 }
-static std::mutex g_tcg_mu;
+
+// Buffers for the rounded activations. A call's buffer may not be written by another call before its GEMM has read it, and a
+// captured call's may not be freed or used by anything else while a graph holds it:
+//   * a stream has a buffer of its own, which grows with what it is asked for (set-up time); calls on one stream are ordered,
+//     and its lock is held over both launches, so that two threads on one stream do not interleave them;
+//   * there are TCG_STREAM_BUFS of those; further streams allocate and free in stream order, call by call;
+//   * a stream that is being captured gets a buffer for this capture. The graph keeps it (a user object), graphs instantiated
+//     from it too, and it comes back for later captures when the last of them is gone.
+#define TCG_STREAM_BUFS 16
+struct TcgBuf { float* p; size_t floats; unsigned long long stream, capture; TcgBuf* next; };
+struct TcgStreamBuf { std::mutex mu; unsigned long long stream = 0; float* p = nullptr; size_t floats = 0; };
+struct TcgBufs {
+  std::mutex mu;                                   // everything below but `returned`
+  TcgStreamBuf streams[TCG_STREAM_BUFS];
+  int nstreams = 0;
+  std::vector<TcgBuf*> captured, idle;             // held by a graph or by a capture in progress; free for the next capture
+  std::atomic<TcgBuf*> returned{nullptr};          // given back by graphs that went away: a lock-free list, as the driver calls back
+};
+static TcgBufs& tcg_bufs() { static TcgBufs* b = new TcgBufs; return *b; }     // outlives every graph
+static void CUDART_CB tcg_give_back(void* q) {
+  TcgBuf* b = static_cast<TcgBuf*>(q);
+  std::atomic<TcgBuf*>& head = tcg_bufs().returned;
+  b->next = head.load();
+  while (!head.compare_exchange_weak(b->next, b)) {}
+}
+// Allocation is legal for this thread whatever another one (or this one) is capturing.
+struct TcgRelaxed {
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  TcgRelaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+  ~TcgRelaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+};
+struct TcgLease { float* p = nullptr; bool free_after = false; std::unique_lock<std::mutex> lock; };
+
+static int tcg_lease(TcgLease& out, size_t floats, cudaStream_t st) {
+  auto fail = [&]() { cudaGetLastError(); wv_set_error("batched matvec: %zu bytes for the rounded activations unavailable", floats * 4); return WV_ENOMEM; };
+  TcgBufs& bufs = tcg_bufs();
+  unsigned long long id = 0, cap = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(st, &status, &cap, &graph) != cudaSuccess) { cudaGetLastError(); status = cudaStreamCaptureStatusNone; }
+  // a stream's number (a handle may be reused); it may not be asked for in a capture, whose own number tells handles apart
+  if (status != cudaStreamCaptureStatusNone || cudaStreamGetId(st, &id) != cudaSuccess) { cudaGetLastError(); id = reinterpret_cast<uintptr_t>(st); }
+  if (status == cudaStreamCaptureStatusActive) {
+    std::lock_guard<std::mutex> lk(bufs.mu);
+    for (TcgBuf* b = bufs.returned.exchange(nullptr); b;) {
+      TcgBuf* next = b->next;
+      for (size_t i = 0; i < bufs.captured.size(); i++) if (bufs.captured[i] == b) { bufs.captured[i] = bufs.captured.back(); bufs.captured.pop_back(); break; }
+      bufs.idle.push_back(b);
+      b = next;
+    }
+    for (TcgBuf* b : bufs.captured) if (b->capture == cap && b->stream == id && b->floats >= floats) { out.p = b->p; return WV_OK; }
+    TcgBuf* b = nullptr;
+    for (size_t i = 0; i < bufs.idle.size() && !b; i++) if (bufs.idle[i]->floats >= floats) { b = bufs.idle[i]; bufs.idle[i] = bufs.idle.back(); bufs.idle.pop_back(); }
+    TcgRelaxed relaxed;
+    if (!b) {
+      for (TcgBuf* q : bufs.idle) { cudaFree(q->p); delete q; }      // all too small
+      bufs.idle.clear();
+      float* p = nullptr;
+      if (cudaMalloc(&p, floats * 4) != cudaSuccess) return fail();
+      b = new TcgBuf{p, floats, 0, 0, nullptr};
+    }
+    b->stream = id; b->capture = cap;
+    cudaUserObject_t obj = nullptr;
+    if (cudaUserObjectCreate(&obj, b, tcg_give_back, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) { bufs.idle.push_back(b); return fail(); }
+    bufs.captured.push_back(b);
+    // if the graph does not take it, the buffer goes back through the release
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) { cudaUserObjectRelease(obj, 1); return fail(); }
+    out.p = b->p;
+    return WV_OK;
+  }
+  TcgStreamBuf* sb = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(bufs.mu);
+    for (int i = 0; i < bufs.nstreams && !sb; i++) if (bufs.streams[i].stream == id) sb = &bufs.streams[i];
+    if (!sb && bufs.nstreams < TCG_STREAM_BUFS) { sb = &bufs.streams[bufs.nstreams++]; sb->stream = id; }
+  }
+  if (!sb) {
+    if (cudaMallocAsync(&out.p, floats * 4, st) != cudaSuccess) return fail();
+    out.free_after = true;
+    return WV_OK;
+  }
+  out.lock = std::unique_lock<std::mutex>(sb->mu);
+  if (sb->floats < floats) {
+    TcgRelaxed relaxed;
+    cudaStreamSynchronize(st);            // nothing else has ever used this buffer
+    if (sb->p) cudaFree(sb->p);
+    sb->p = nullptr; sb->floats = 0;
+    if (cudaMalloc(&sb->p, floats * 4) != cudaSuccess) return fail();
+    sb->floats = floats;
+  }
+  out.p = sb->p;
+  return WV_OK;
+}
 
 int wv_sm_count();
 
@@ -547,6 +637,8 @@ static int tcg_splits(K kern, int dev, int mtiles, int cpr, int unit) {
 template <int F, bool VEC>
 static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
   auto kern = gemm_tcgen05_kernel<F, VEC>;
+  auto enc = tcg_encode_fn();
+  if (!enc) return 1;
   static unsigned attr_mask = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -574,21 +666,10 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
   const size_t smem = (size_t)g.rounds * TCG_GROUPS * g.stage_bytes + 1024;
   // X rounded to TF32 once, by a small kernel in front (each of the row tiles would otherwise round it again), into a
   // buffer of the library; the main kernel fetches it through a tensor map encoded per call.
-  float* xr = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_tcg_mu);
-    const size_t need = (size_t)batch * b.cols;
-    if (need > g_tcg_xr_floats) {
-      cudaStreamSynchronize(st);
-      if (g_tcg_xr) cudaFree(g_tcg_xr);
-      g_tcg_xr = nullptr; g_tcg_xr_floats = 0;
-      if (cudaMalloc(&g_tcg_xr, need * 4) != cudaSuccess) { cudaGetLastError(); wv_set_error("batched matvec: %zu bytes for the rounded activations unavailable", need * 4); return WV_ENOMEM; }
-      g_tcg_xr_floats = need;
-    }
-    xr = g_tcg_xr;
-  }
-  auto enc = tcg_encode_fn();
-  if (!enc) return 1;
+  TcgLease lease;
+  if (const int rc = tcg_lease(lease, (size_t)batch * b.cols, st)) return rc;
+  float* xr = lease.p;
+  struct FreeAfter { TcgLease& l; cudaStream_t st; ~FreeAfter() { if (l.free_after) cudaFreeAsync(l.p, st); } } free_after{lease, st};
   CUtensorMap xmap;
   {
     cuuint64_t dims[2] = {(cuuint64_t)b.cols, (cuuint64_t)batch};
