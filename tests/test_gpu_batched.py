@@ -269,3 +269,27 @@ def test_batched_calls_in_graphs(wv):
         torch.cuda.synchronize()
         assert torch.equal(yb, wantb) and all(torch.equal(y, want) for _, _, y, want in jobs)
     assert L.wv_device_status() == 0
+
+
+@pytest.mark.parametrize("slice_", [1, 2, 5])
+@pytest.mark.parametrize("batch", [9, 100])
+def test_batched_wait_that_runs_out(wv, hooks, slice_, batch):
+    """A producer warp that never hands its slice over: the waits of the others run out, the call ends with the time-out
+    status, copies and MMAs that were in flight are waited for, and the next call is as good as any."""
+    rows, cols = 300, 14336
+    key, _keep = _packed(wv, "Q4_0", rows, cols, 40)
+    x = torch.randn(batch, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(41))
+    y = [torch.zeros(batch, rows, device="cuda") for _ in range(3)]
+
+    def call(i):
+        wv._lib.check(hooks.wv_matvec_dev(key, x.data_ptr(), y[i].data_ptr(), batch, cols, rows, None))
+        torch.cuda.synchronize()
+        return hooks.wv_device_status()
+
+    assert call(0) == 0
+    hooks.wv_set_tcg_stall(slice_, 2000)
+    try:
+        assert call(1) != 0
+    finally:
+        hooks.wv_set_tcg_stall(0, 0)
+    assert call(2) == 0 and torch.equal(y[0], y[2])

@@ -14,6 +14,9 @@ void wv_set_tma_tuning(int rows_per_group, int stages);
 // Width of the activation records of the integer-dot kernels: 0 = chosen per launch from the input
 // vector (16-bit unless it has isolated outliers), 3 = always 24-bit.
 void wv_set_act_width(int limbs);
+// Batched kernel: the first producer warp stops short of its `slice`-th slice (1, 2, ...; 0 = off) and the waits give up after
+// `spin` polls (0 = built-in limit), so that a bounded wait runs out.
+void wv_set_tcg_stall(int slice, int spin);
 #ifdef __cplusplus
 }
 #endif

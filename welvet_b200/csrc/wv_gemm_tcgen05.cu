@@ -27,9 +27,11 @@
 // rounding. TF32 keeps FP32's exponent range, so no operand needs scaling.
 //
 // Every wait is bounded: a wait that runs out records a code in the mapped error word, raises the CTA's abort flag,
-// and all roles fall through to the common exit, where the TMEM columns are released.
+// and all roles fall through to the common exit. There the copies of X and the MMAs still in flight are waited for (bounded
+// again) before the TMEM columns and the shared memory are given back.
 #include "wv_gemv_common.cuh"
 #include "wv_tma_common.cuh"
+#include "wv_dev_hooks.h"
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <atomic>
@@ -255,7 +257,16 @@ struct TcgGeom {
   unsigned b_bytes, stage_bytes;            // a stage: one slice of A (128 rows x 128 bytes), then one of B (npad x 128 bytes)
   unsigned tmem_cols;         // power of two >= max(32, npad)
   int y_stride;               // floats between consecutive activation rows' outputs
+#ifdef WV_DEV_HOOKS
+  int stall;                  // > 0: the first producer warp stops short of this slice, so that a wait runs out
+  unsigned spin;              // limit of the waits
+#endif
 };
+#ifdef WV_DEV_HOOKS
+#define TCG_SPIN g.spin
+#else
+#define TCG_SPIN TMA_SPIN_LIMIT
+#endif
 
 #define TCG_A_BYTES (TCG_M * 128u)
 
@@ -303,6 +314,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   __shared__ __align__(8) unsigned long long s_bar[2 * TCG_MAX_STAGES + 1];
   __shared__ unsigned s_tmem;
   __shared__ int s_abort;
+  __shared__ int s_made[TCG_PRODUCERS / 32];      // slices each producer warp has arrived for
   __shared__ float s_tbl[16];          // IQ4_NL's grid
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // one value per warp, and the compiler knows it
   const int mt = blockIdx.x, sp = blockIdx.y;
@@ -339,6 +351,8 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   // for it (X was rounded by the kernel right before this one), and nothing is stored before X has arrived.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  int copied_i = 0, copied_q = 0;                // copying warp: the round it reached, and the groups it served in that round
+
   if (warp < TCG_PRODUCERS / 32) {
     // ------------------------------------------------------------ producers
     const int grp = warp / (TCG_M / 32);                         // owns a run of the CTA's columns
@@ -353,6 +367,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
     FragT<F> nxt[U];
     if (mine > 0) tcg_load<F, VEC>(nxt, b, ch0, mine);
     bool dead = false;
+    int made = 0;
     for (int i0 = 0; i0 < mine && !dead; i0 += U) {
       FragT<F> cur[U];
 #pragma unroll
@@ -362,9 +377,12 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
       for (int u = 0; u < U; u++) {
         const int i = i0 + u;
         if (i >= mine || dead) break;
+#ifdef WV_DEV_HOOKS
+        if (g.stall > 0 && warp == 0 && i + 1 >= g.stall) { dead = true; break; }
+#endif
         bool bad = *(volatile int*)&s_abort != 0;
         const int s = stage_of(i, grp), use = i >> rsh;
-        if (!bad && use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
+        if (!bad && use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1, TCG_SPIN)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
         if (__any_sync(0xffffffffu, bad)) { dead = true; break; }     // the whole warp leaves together (it meets at __syncwarp below)
         const unsigned st = sbase + (unsigned)s * g.stage_bytes + a_off;
         tcg_convert<F>(cur[u], s_tbl, [&](int p, const float (&v)[4]) {
@@ -373,8 +391,10 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(full_bar(s));      // one arrival per warp
+        made = i + 1;
       }
     }
+    if (lane == 0) s_made[warp] = made;
   } else if (warp == TCG_PRODUCERS / 32 + 1) {
     // ------------------------------------------------------------ X copies: a stage's slice of the rounded activations arrives
     // by a tensor-map copy with the 128-byte swizzle, i.e. already in the operand layout; rows past the batch are zero-filled
@@ -387,16 +407,18 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
     bool run = true;
     for (int i = 0; i < order.n[0] && run; i++) {
       const int use = i >> rsh, na = order.active(i);
+      copied_i = i; copied_q = 0;
 #pragma unroll
       for (int q = 0; q < TCG_GROUPS; q++) {
         if (q >= na || !run) break;
         const int s = stage_of(i, q);
-        if (use > 0 && __any_sync(0xffffffffu, !mbar_wait(empty_bar(s), (use - 1) & 1))) { atomicCAS_system(err, 0, 530 + s); *(volatile int*)&s_abort = 1; run = false; break; }
+        if (use > 0 && __any_sync(0xffffffffu, !mbar_wait(empty_bar(s), (use - 1) & 1, TCG_SPIN))) { atomicCAS_system(err, 0, 530 + s); *(volatile int*)&s_abort = 1; run = false; break; }
         if (leader) {
           mbar_expect_tx(full_bar(s), g.b_bytes);
           tma_load_2d(sbase + (unsigned)s * g.stage_bytes + TCG_A_BYTES, &xmap, (kc0 + order.first[q] + i) * 32, 0, full_bar(s));
         }
         __syncwarp();
+        copied_q = q + 1;
       }
     }
   } else {
@@ -410,7 +432,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
       for (int q = 0; q < TCG_GROUPS; q++) {
         if (q >= na || !run) break;
         const int s = stage_of(i, q);
-        if (__any_sync(0xffffffffu, !mbar_wait(full_bar(s), (i >> rsh) & 1))) { atomicCAS_system(err, 0, 510 + s); *(volatile int*)&s_abort = 1; run = false; break; }
+        if (__any_sync(0xffffffffu, !mbar_wait(full_bar(s), (i >> rsh) & 1, TCG_SPIN))) { atomicCAS_system(err, 0, 510 + s); *(volatile int*)&s_abort = 1; run = false; break; }
         tcg_fence_after();
         if (leader) {
           const unsigned st = sbase + (unsigned)s * g.stage_bytes;
@@ -433,7 +455,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   float* acc = reinterpret_cast<float*>(tcg_smem + (sbase - smem_u32(tcg_smem)));    // [batch][128]
   if (warp < TCG_PRODUCERS / 32) {
     bool ok = !*(volatile int*)&s_abort;
-    if (ok && !mbar_wait(done_bar, 0)) { atomicCAS_system(err, 0, 520); *(volatile int*)&s_abort = 1; ok = false; }
+    if (ok && !mbar_wait(done_bar, 0, TCG_SPIN)) { atomicCAS_system(err, 0, 520); *(volatile int*)&s_abort = 1; ok = false; }
     ok = __all_sync(0xffffffffu, ok);     // tcgen05.ld is warp-wide
     tcg_fence_after();
     const int row_l = (warp & 3) * 32 + lane;
@@ -457,6 +479,24 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   }
   tcg_fence_before();
   __syncthreads();
+  if (*(volatile int*)&s_abort) {      // the same for every thread: nobody raises it after the barrier
+    if (warp == TCG_PRODUCERS / 32) mbar_wait(done_bar, 0, TCG_SPIN);        // the MMAs issued before the abort
+    if (warp == TCG_PRODUCERS / 32 + 1) {
+      // A stage's barrier completes when its copy has landed and its group's four warps have arrived: the arrivals that will
+      // never come are made up for here, then the last uses of every stage are waited for (the earlier ones have been read).
+#pragma unroll
+      for (int q = 0; q < TCG_GROUPS; q++) {
+        const int issued = min(order.n[q], copied_i + (q < copied_q ? 1 : 0));
+        for (int i = max(0, issued - g.rounds); i < issued; i++) {
+          const int s = stage_of(i, q);
+          if (lane < TCG_M / 32 && s_made[q * (TCG_M / 32) + lane] <= i) mbar_arrive(full_bar(s));
+          __syncwarp();
+          mbar_wait(full_bar(s), (i >> rsh) & 1, TCG_SPIN);
+        }
+      }
+    }
+    __syncthreads();
+  }
   if (warp == TCG_PRODUCERS / 32) {
     tcg_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(g.tmem_cols) : "memory");
@@ -495,6 +535,11 @@ __global__ void __launch_bounds__(256) tcg_round_x_kernel(const float4* __restri
 }
 
 // ------------------------------------------------------------------ host side
+#ifdef WV_DEV_HOOKS
+static int g_tcg_stall = 0;
+static unsigned g_tcg_spin = TMA_SPIN_LIMIT;
+extern "C" void wv_set_tcg_stall(int slice, int spin) { g_tcg_stall = slice; g_tcg_spin = spin > 0 ? (unsigned)spin : TMA_SPIN_LIMIT; }
+#endif
 static PFN_cuTensorMapEncodeTiled_v12000 tcg_encode_fn() {
   static const PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {     // once, whichever thread is first
     void* p = nullptr;
@@ -661,6 +706,9 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
   g.b_bytes = (unsigned)g.npad * 128u;
   g.stage_bytes = TCG_A_BYTES + g.b_bytes;
   g.rounds = TCG_MAX_STAGES * g.stage_bytes <= 200u * 1024u ? 2 : 1;      // two up to 64 rows; one round of 256 rows takes 192 KB
+#ifdef WV_DEV_HOOKS
+  g.stall = g_tcg_stall; g.spin = g_tcg_spin;
+#endif
   g.tmem_cols = 32;
   while ((int)g.tmem_cols < g.npad) g.tmem_cols *= 2;
   const size_t smem = (size_t)g.rounds * TCG_GROUPS * g.stage_bytes + 1024;

@@ -16,8 +16,8 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // Bounded wait: returns false when the phase did not complete within the spin limit.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  for (unsigned i = 0; i < TMA_SPIN_LIMIT; i++) {
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned limit = TMA_SPIN_LIMIT) {
+  for (unsigned i = 0; i < limit; i++) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
