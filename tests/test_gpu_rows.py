@@ -70,3 +70,15 @@ def test_infinite_activations_give_nan(wv, fmt, cols, bad):
     assert np.all(np.isnan(y[2])) and np.all(np.isfinite(y[[0, 1, 3]]))
     one, _ = _run(wv, ob, x[2:3])
     assert np.all(np.isnan(one))
+
+
+@pytest.mark.parametrize("fmt,rows,cols,batch", [("Q4_K", 24, 4096, 4), ("Q6_K", 29, 1024, 5), ("IQ3_XXS", 74, 6144, 2), ("Q4_K", 64, 6144, 3), ("TernaryPacked", 42, 4096, 4)])
+def test_few_rows_of_w_run_row_by_row(wv, fmt, rows, cols, batch):
+    """Where all activation rows' CTAs fit on the chip side by side the batch is that many one-row launches in one: the same
+    bits as one at a time."""
+    w, _ = make_w(rows, rows, cols)
+    ob = O.pack(fmt, w, rows, cols)
+    x = np.random.default_rng(rows).normal(0, 1, (batch, cols)).astype(np.float32)
+    y, _ = _run(wv, ob, x)
+    one = np.concatenate([_run(wv, ob, x[m:m + 1])[0] for m in range(batch)])
+    assert np.array_equal(y, one)

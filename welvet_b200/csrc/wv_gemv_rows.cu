@@ -343,6 +343,13 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
   g.cpr = b.cols >> 5;
   g.nwc = (g.cpr + 31) / 32;
   if (g.nwc > TMA_CONSUMER_WARPS) return 1;
+  // So few rows of W that row by row the CTAs of all activation rows run side by side, or nearly: that takes 3.6 - 4.4 us as long
+  // as there is an SM for each and 6.9 - 7.9 us up to two for each, while this kernel spreads the rows of W alone over the chip
+  // and takes 2.4 - 3.2 us and 1.45 us for each of a CTA's activation rows (Q4_K, four rows: 24 x 4096 4.1 against 8.2 us,
+  // 64 x 6144 7.5 against 9.1; three rows, 64 x 4096: 7.6 against 6.9).
+  const int ny = (batch + ROWS_NB - 1) / ROWS_NB, nb = (batch + ny - 1) / ny;
+  const long long side = (long long)(re - rb_) * batch, sms = wv_sm_count();
+  if (side <= sms || (side <= 2 * sms && nb * g.nwc >= 16)) return 1;
   g.nrg = TMA_CONSUMER_WARPS / g.nwc;
   if (g.nrg > TMA_MAX_ROW_GROUPS) g.nrg = TMA_MAX_ROW_GROUPS;
   g.tr = g.nrg * ROWS_RT;
@@ -365,7 +372,6 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
   if (grid > re - rb_) grid = re - rb_;
   g.rows_base = (re - rb_) / grid;
   g.rows_rem = (re - rb_) % grid;
-  const int ny = (batch + ROWS_NB - 1) / ROWS_NB;
   g.m_base = batch / ny;
   g.m_rem = batch % ny;
   auto kern = gemv_rows_kernel<F>;
@@ -382,7 +388,7 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
 }
 
 // Returns 1 for what this kernel does not take: FormatNone, IQ4_NL (float table arithmetic), planes whose rows are no 16-byte
-// multiples, the formats and widths below, and rows so wide that four rows' records leave the ring no room for two tiles (beyond 6144 columns in Q4_K).
+// multiples, few rows of W (launch_rows), the formats and widths below, and rows so wide that four rows' records leave the ring no room for two tiles (beyond 6144 columns in Q4_K).
 int wv_launch_gemv_rows(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st) {
   if (batch < 2 || !b.fast || b.format == WV_NONE || row_end <= row_begin || !wv_tma_err_ptr()) return 1;
   // What runs as 24-bit records on the tensor pipe row by row (gemv_mma_kernel: Q8_0, and the formats with one parameter
