@@ -82,3 +82,13 @@ def test_few_rows_of_w_run_row_by_row(wv, fmt, rows, cols, batch):
     y, _ = _run(wv, ob, x)
     one = np.concatenate([_run(wv, ob, x[m:m + 1])[0] for m in range(batch)])
     assert np.array_equal(y, one)
+
+
+@pytest.mark.parametrize("fmt", ["TernaryPacked", "IQ1_S", "Q4_0"])
+def test_two_rows_of_wide_matrices_run_one_by_one(wv, fmt):
+    rows, cols = 300, 9216
+    w, _ = make_w(2, rows, cols)
+    ob = O.pack(fmt, w, rows, cols)
+    x = np.random.default_rng(3).normal(0, 1, (2, cols)).astype(np.float32)
+    y, _ = _run(wv, ob, x)
+    assert np.array_equal(y, np.concatenate([_run(wv, ob, x[m:m + 1])[0] for m in range(2)]))

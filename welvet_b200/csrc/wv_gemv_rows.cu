@@ -351,6 +351,10 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
   const long long side = (long long)(re - rb_) * batch, sms = wv_sm_count();
   if (side <= sms || (side <= 2 * sms && nb * g.nwc >= 16)) return 1;
   g.nrg = TMA_CONSUMER_WARPS / g.nwc;
+  // One row group (more than eight column warps) leaves up to seven warps idle: two activation rows are faster one by one in the
+  // formats that unpack cheaply (no hi plane; 4096 x 9216: IQ1_S 14.2 against 14.7 us, Ternary 14.3 against 15.2; IQ3_S, with one,
+  // 17.4 against 16.5), three are not (Ternary 21.2 against 19.6).
+  if (g.nrg == 1 && batch == 2 && wv_fmt_info(F).bits_hi == 0) return 1;
   if (g.nrg > TMA_MAX_ROW_GROUPS) g.nrg = TMA_MAX_ROW_GROUPS;
   g.tr = g.nrg * ROWS_RT;
   g.wide = wv_act_width() == 3;
