@@ -293,3 +293,18 @@ def test_batched_wait_that_runs_out(wv, hooks, slice_, batch):
     finally:
         hooks.wv_set_tcg_stall(0, 0)
     assert call(2) == 0 and torch.equal(y[0], y[2])
+
+
+@pytest.mark.parametrize("shape", [(40, 14336), (300, 14336), (70, 4352), (129, 8192)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("fmt", ["Q8_0", "Q4_K", "AffinePacked"])
+def test_batched_few_rows_many_columns(wv, fmt, shape):
+    """One to three row tiles whose columns are split over more CTAs than a portable cluster holds; the last split shorter than
+    the others, or not."""
+    rows, cols = shape
+    w = np.random.default_rng(cols).normal(0, 0.02, rows * cols).astype(np.float32)
+    ob = O.pack(fmt, w, rows, cols)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    for batch in (6, 33, 256):
+        x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
+        y, _ = _run(wv, ob, x)
+        assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch

@@ -43,7 +43,7 @@
 #define TCG_M 128
 #define TCG_GROUPS (TCG_PRODUCERS / TCG_M)
 #define TCG_MAX_STAGES (2 * TCG_GROUPS)
-#define TCG_MAX_SPLIT 8     // portable cluster size
+#define TCG_MAX_SPLIT 16    // cluster size (beyond 8 the kernel has to ask for it)
 
 // ------------------------------------------------------------------ weight loads
 template <int N> __device__ __forceinline__ void tcg_words(unsigned (&d)[N], const void* p) {
@@ -511,12 +511,17 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   for (int e = tid; ; e += TCG_THREADS) {
     const int m = (e / TCG_M) * g.ksplit + sp, row_l = e & (TCG_M - 1);
     if (m >= g.batch) break;
-    float v[TCG_MAX_SPLIT];
+    float v[8], sum = 0.f;
 #pragma unroll
-    for (int u = 0; u < TCG_MAX_SPLIT; u++) if (u < g.ksplit) v[u] = ld_cluster(acc_s + 4u * (unsigned)(m * TCG_M + row_l), u);
-    float sum = 0.f;
+    for (int u = 0; u < 8; u++) if (u < g.ksplit) v[u] = ld_cluster(acc_s + 4u * (unsigned)(m * TCG_M + row_l), u);
 #pragma unroll
-    for (int u = 0; u < TCG_MAX_SPLIT; u++) if (u < g.ksplit) sum += v[u];
+    for (int u = 0; u < 8; u++) if (u < g.ksplit) sum += v[u];
+    if (g.ksplit > 8) {
+#pragma unroll
+      for (int u = 0; u < 8; u++) if (8 + u < g.ksplit) v[u] = ld_cluster(acc_s + 4u * (unsigned)(m * TCG_M + row_l), 8 + u);
+#pragma unroll
+      for (int u = 0; u < 8; u++) if (8 + u < g.ksplit) sum += v[u];
+    }
     if (m0 + row_l < g.row_end) y[(size_t)m * g.y_stride + m0 + row_l] = sum;
   }
   __syncwarp();
@@ -689,6 +694,7 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
   cudaGetDevice(&dev);
   if (!(attr_mask & (1u << (dev & 31)))) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024) != cudaSuccess) { wv_set_error("batched matvec: cannot raise the shared-memory limit"); return WV_ECUDA; }
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { wv_set_error("batched matvec: cannot allow clusters of 16"); return WV_ECUDA; }
     attr_mask |= 1u << (dev & 31);
   }
   TcgGeom g{};
