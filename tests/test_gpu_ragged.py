@@ -45,3 +45,43 @@ def test_ragged_batch_and_neighbours(wv):
     ref, den = X @ wd.T, np.abs(X) @ np.abs(wd).T
     assert np.all(np.isfinite(pre[:, 1:])) and np.all(np.abs(pre[:, 1:] - ref) <= 50 * 2.0 ** -24 * den)
     assert not np.any(np.isfinite(pre[:, 0]))
+
+
+def _raw_rows(wv, ob, X):
+    st = wv.weights.FromBlob(to_product_blob(wv, ob))
+    pre, _ = wv.dense.Forward(wv.dense.Layer(ob.cols, ob.rows, wv.dense.ActivationLinear, st), X)
+    wd = O.unpack(ob).reshape(ob.rows, ob.cols).astype(np.float64)
+    return pre, wd
+
+
+@pytest.mark.parametrize("fmt", ["TernaryPacked", "Q4_1"])
+def test_ragged_neighbours_infinite_weights(wv, fmt):
+    """A group that two rows share, in which the neighbour's weights are infinite and this row's are not: a ternary group of
+    infinite scale where this row has zeros, and codes of 15 times a scale of 1e38 beside codes of 0."""
+    rows, cols = 4, 40                     # weights 32 - 39 are row 0's, 40 - 47 row 1's
+    w, _ = make_w(8, rows, cols)
+    X = np.random.default_rng(9).normal(0, 1, (2, cols)).astype(np.float32)
+    ob = O.pack(fmt, w, rows, cols)
+    if fmt == "TernaryPacked":
+        ob.scales[2] = np.inf
+        ob.raw[8:12] = [0x55, 0x55, 0xAA, 0xAA]
+    else:
+        ob.raw[24:28] = np.frombuffer(np.float32(1e38).tobytes(), np.uint8)
+        ob.raw[32:48] = [0] * 4 + [255] * 12
+    pre, wd = _raw_rows(wv, ob, X)
+    assert np.all(np.isfinite(wd[[0, 3]])) and np.any(np.isinf(wd[1]))
+    assert not np.any(np.isfinite(pre[:, 1]))
+    for r in (0, 3):
+        assert np.all(np.abs(pre[:, r] - X @ wd[r]) <= 100 * 2.0 ** -24 * (np.abs(X) @ np.abs(wd[r])))
+
+
+@pytest.mark.parametrize("fmt", ["Q8_0", "Q6_K", "IQ3_S", "IQ4_NL", "IQ4_XS", "TernaryPacked"])
+def test_ragged_large_activations(wv, fmt):
+    """Activations of 1e37: the products with the weights are far from float32's limit, those with the bare codes are not."""
+    rows, cols = 20, 1022
+    w, _ = make_w(11, rows, cols)
+    X = (1e37 * np.random.default_rng(12).normal(0, 1, (2, cols))).astype(np.float32)
+    pre, wd = _raw_rows(wv, O.pack(fmt, w, rows, cols), X)
+    ref, den = X.astype(np.float64) @ wd.T, np.abs(X.astype(np.float64)) @ np.abs(wd).T
+    assert den.max() < 3e38
+    assert np.all(np.isfinite(pre)) and np.all(np.abs(pre - ref) <= 100 * 2.0 ** -24 * den)

@@ -6,13 +6,16 @@
 // (chunk boundaries are aligned whatever the row length) and meets them with x shifted by start % 32. x sits in shared
 // memory with 32 zeros in front of it and behind it, which is what the neighbours' weights in a shared chunk are
 // multiplied with, and with one word of padding every 32, so that lanes 32 floats apart hit 32 different banks wherever
-// the row starts.
+// the row starts. A row whose sum comes out infinite or NaN is summed again over its own weights, one by one: zero times a
+// neighbour's infinity is no zero, and codes summed before they are scaled overflow for activations whose products with the
+// weights do not.
 //
 // Bound: launch and memory latency (a 2730 x 1022 matrix is 1 - 3 MB). A weight costs about 7 instructions; the
 // weight-by-weight kernel this replaces spent some 60 (64-bit index arithmetic, bit extraction from global memory
 // and, for the k-quants, two divisions). Measured back to back on a stream, Q8_0, Q4_0, Q4_K and IQ3_S at 2730 x 1022
 // and 1022 x 2730: 271 us before for the eight launches, 43 us now (5.4 us a launch, of which about 4 us is the
 // host's own cost of a call).
+#include "wv_dequant.cuh"
 #include "wv_gemv_common.cuh"
 #include "wv_tma_common.cuh"
 
@@ -29,10 +32,9 @@ __device__ __forceinline__ void rag_stage_x(float* xs, const float* __restrict__
   else if (threadIdx.x < 96) xs[rag_slot(cols + threadIdx.x)] = 0.f;    // positions cols + 32 .. cols + 95
 }
 
-// Dot of one chunk with the 32 activations xv(j). h0 / h1: the chunk's halves that hold weights of this row at all (a
-// half that is entirely the neighbour's may carry the neighbour's infinite or NaN scale).
+// Dot of one chunk with the 32 activations xv(j).
 template <int F, typename X>
-__device__ __forceinline__ float rag_chunk(const FragT<F>& f, X xv, const float* tbl, bool h0, bool h1) {
+__device__ __forceinline__ float rag_chunk(const FragT<F>& f, X xv, const float* tbl) {
   constexpr WvFmtInfo fi = wv_fmt_info(F);
   constexpr int BL = fi.bits_lo, BH = fi.bits_hi, SPW = 8 / BL;
   constexpr unsigned MASK = 0x01010101u * ((1u << BL) - 1u);
@@ -53,10 +55,6 @@ __device__ __forceinline__ float rag_chunk(const FragT<F>& f, X xv, const float*
     sc[0] = sc[1] = __uint_as_float(f.pr[0]);
     if constexpr (fi.pgroup == 16) sc[1] = __uint_as_float(f.pr[1]);
     if constexpr (fi.has_min) mn[0] = mn[1] = __uint_as_float(f.pr[1]);
-  }
-  if constexpr (fi.pgroup == 16) {
-    if (!h0) { sc[0] = 0.f; mn[0] = 0.f; }
-    if (!h1) { sc[1] = 0.f; mn[1] = 0.f; }
   }
   const float magic = 8388608.0f + (float)fi.mid;   // code under the exponent of 2^23, minus this: (code - mid) exactly
   float acc[4] = {0.f, 0.f, 0.f, 0.f}, tot = 0.f;
@@ -92,6 +90,15 @@ __device__ __forceinline__ float rag_chunk(const FragT<F>& f, X xv, const float*
   return tot;
 }
 
+// The products of every step-th weight of a row, from `first` on.
+template <int F>
+__device__ __forceinline__ float rag_row_own(const WvDevBlob& b, const float* __restrict__ xb, int row, int first, int step) {
+  constexpr WvFmtInfo fi = wv_fmt_info(F);
+  float acc = 0.f;
+  for (int c = first; c < b.cols; c += step) acc = fmaf(wv_dequant(b, fi, (long long)row * b.cols + c), __ldg(xb + c), acc);
+  return acc;
+}
+
 // XS: x in shared memory (otherwise read from global memory, with the zeros around it by comparison).
 template <int F, bool XS>
 __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_chunk_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
@@ -112,6 +119,7 @@ __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_chunk_kernel(const Wv
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (XS) rag_stage_x(rag_xs, xb, b.cols);
   __syncthreads();
+  bool odd = false;
   for (; row < row_end; row += nw) {
     start = (long long)row * b.cols;
     const int s = (int)(start & 31), nch = (s + b.cols + 31) >> 5;
@@ -122,17 +130,27 @@ __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_chunk_kernel(const Wv
       FragT<F> nxt = cur;
       if (c + 32 < nch) load_frag<F>(nxt, b, ch0 + c + 32);
       const int i0 = 32 + c * 32 - s;      // padded position of the chunk's first weight; columns i0 - 32 ...
-      const bool h0 = i0 + 16 > 32, h1 = i0 + 16 < 32 + b.cols;
       if constexpr (XS) {
         const float* p0 = rag_xs + rag_slot(i0);
         const int thr = s ? s : 32;         // from here on the next 32-float group: one word of padding further
-        acc += rag_chunk<F>(cur, [&](int j) { return (j < thr ? p0 : p0 + 1)[j]; }, s_tbl + lane, h0, h1);
+        acc += rag_chunk<F>(cur, [&](int j) { return (j < thr ? p0 : p0 + 1)[j]; }, s_tbl + lane);
       } else {
         acc += rag_chunk<F>(cur, [&](int j) { const int col = i0 - 32 + j; return (col >= 0 && col < b.cols) ? __ldg(xb + col) : 0.f; },
-                            s_tbl + lane, h0, h1);
+                            s_tbl + lane);
       }
       cur = nxt;
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) yb[row] = acc;
+    odd = odd || !(fabsf(acc) <= 3.402823466e38f);
+  }
+  // Behind the loop, which so keeps its registers: the rows whose sum was not finite, read back.
+  if (!odd) return;
+  __syncwarp();
+  for (row = row_begin + gw; row < row_end; row += nw) {
+    if (fabsf(yb[row]) <= 3.402823466e38f) continue;
+    float acc = rag_row_own<F>(b, xb, row, lane, 32);
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) yb[row] = acc;
