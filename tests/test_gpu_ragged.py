@@ -85,3 +85,22 @@ def test_ragged_large_activations(wv, fmt):
     ref, den = X.astype(np.float64) @ wd.T, np.abs(X.astype(np.float64)) @ np.abs(wd).T
     assert den.max() < 3e38
     assert np.all(np.isfinite(pre)) and np.all(np.abs(pre - ref) <= 100 * 2.0 ** -24 * den)
+
+
+# 8, 16 and 32 lanes per row: widths on both sides of 8 and 16 units (chunks: 225 / 226, 481 / 482; vectors of 4 elements: 29 / 30,
+# 61 / 62; of 8: 57 / 58, 121 / 122), and rows enough for fewer lanes than units; rows that leave a warp's last rows empty
+LANE_SHAPES = [(65, 29), (33, 30), (37, 57), (38, 58), (39, 61), (41, 62), (65, 121), (33, 122), (70, 225), (71, 226), (30, 481), (29, 482),
+               (1579, 1022), (3157, 514), (3159, 1030)]
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[1] == 0], ids=case_id)
+def test_ragged_lanes_per_row(wv, case):
+    f, bw, dt = case
+    for rows, cols in LANE_SHAPES:
+        if not case_ok(case, rows, cols):
+            continue
+        w, _ = make_w(rows + cols, rows, cols)
+        X = np.random.default_rng(cols).normal(0, 1, (3, cols)).astype(np.float32)
+        pre, wd = _raw_rows(wv, O.pack(f, w, rows, cols, bw, dt), X)
+        # float32: a lane adds at most cols / 32 + 8 products in a row, then 8 sums; a weight with a min has two more roundings
+        assert np.all(np.abs(pre - X @ wd.T) <= (cols / 32 + 30) * 2.0 ** -24 * (np.abs(X) @ np.abs(wd).T) + 1e-30), (rows, cols)

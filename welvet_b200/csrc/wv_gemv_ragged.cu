@@ -99,36 +99,40 @@ __device__ __forceinline__ float rag_row_own(const WvDevBlob& b, const float* __
   return acc;
 }
 
-// XS: x in shared memory (otherwise read from global memory, with the zeros around it by comparison).
-template <int F, bool XS>
-__global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_chunk_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
+// XS: x in shared memory (otherwise read from global memory, with the zeros around it by comparison). LPR: lanes per row; a
+// warp works on 32 / LPR rows.
+template <int F, bool XS, int LPR>
+__global__ void __launch_bounds__(RAG_THREADS, 4) gemv_ragged_chunk_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
                                                                         int row_begin, int row_end) {
   constexpr WvFmtInfo fi = wv_fmt_info(F);
+  constexpr int RPW = 32 / LPR;
   extern __shared__ float rag_xs[];
   __shared__ float s_tbl[fi.table ? 512 : 1];
-  const int lane = threadIdx.x & 31, gw = (int)((blockIdx.x * RAG_THREADS + threadIdx.x) >> 5), nw = (int)(gridDim.x * RAG_THREADS) >> 5;
+  const int lane = threadIdx.x & 31, sl = lane % LPR, gw = (int)((blockIdx.x * RAG_THREADS + threadIdx.x) >> 5), nw = (int)(gridDim.x * RAG_THREADS) >> 5;
   const float* xb = x + (size_t)blockIdx.y * b.cols;
   float* yb = y + (size_t)blockIdx.y * b.rows;
-  int row = row_begin + gw;
+  const int first = row_begin + gw * RPW;                 // the warp's first rows
+  int row = first + lane / LPR;
   long long start = (long long)row * b.cols;
   FragT<F> cur;
   // the first chunk's weights do not depend on the preceding kernel
-  if (row < row_end && lane < (int)(((start & 31) + b.cols + 31) >> 5)) load_frag<F>(cur, b, (start >> 5) + lane);
+  if (row < row_end && sl < (int)(((start & 31) + b.cols + 31) >> 5)) load_frag<F>(cur, b, (start >> 5) + sl);
   if constexpr (fi.table) for (int i = threadIdx.x; i < 512; i += RAG_THREADS) s_tbl[i] = c_grid4nl[i >> 5];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (XS) rag_stage_x(rag_xs, xb, b.cols);
   __syncthreads();
   bool odd = false;
-  for (; row < row_end; row += nw) {
+  for (int r0 = first; r0 < row_end; r0 += nw * RPW) {    // the same for the whole warp
+    row = r0 + lane / LPR;
     start = (long long)row * b.cols;
-    const int s = (int)(start & 31), nch = (s + b.cols + 31) >> 5;
+    const int s = (int)(start & 31), nch = row < row_end ? (s + b.cols + 31) >> 5 : 0;
     const long long ch0 = start >> 5;
-    if (row != row_begin + gw && lane < nch) load_frag<F>(cur, b, ch0 + lane);
+    if (r0 != first && sl < nch) load_frag<F>(cur, b, ch0 + sl);
     float acc = 0.f;
-    for (int c = lane; c < nch; c += 32) {
+    for (int c = sl; c < nch; c += LPR) {
       FragT<F> nxt = cur;
-      if (c + 32 < nch) load_frag<F>(nxt, b, ch0 + c + 32);
+      if (c + LPR < nch) load_frag<F>(nxt, b, ch0 + c + LPR);
       const int i0 = 32 + c * 32 - s;      // padded position of the chunk's first weight; columns i0 - 32 ...
       if constexpr (XS) {
         const float* p0 = rag_xs + rag_slot(i0);
@@ -141,30 +145,31 @@ __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_chunk_kernel(const Wv
       cur = nxt;
     }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) yb[row] = acc;
-    odd = odd || !(fabsf(acc) <= 3.402823466e38f);
+    for (int o = LPR / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (sl == 0 && row < row_end) yb[row] = acc;
+    odd = odd || !(fabsf(acc) <= 3.402823466e38f);          // a row past the end has a sum of zero
   }
   // Behind the loop, which so keeps its registers: the rows whose sum was not finite, read back.
-  if (!odd) return;
+  if (!__any_sync(0xffffffffu, odd)) return;
   __syncwarp();
-  for (row = row_begin + gw; row < row_end; row += nw) {
-    if (fabsf(yb[row]) <= 3.402823466e38f) continue;
-    float acc = rag_row_own<F>(b, xb, row, lane, 32);
+  for (int r0 = first; r0 < row_end; r0 += nw * RPW) {
+    row = r0 + lane / LPR;
+    const bool redo = row < row_end && !(fabsf(yb[row]) <= 3.402823466e38f);
+    float acc = redo ? rag_row_own<F>(b, xb, row, sl, LPR) : 0.f;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) yb[row] = acc;
+    for (int o = LPR / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (redo && sl == 0) yb[row] = acc;
   }
 }
 
 // FormatNone: a lane takes aligned 16-byte vectors of the flat element array; elements outside the row are skipped
-// (they are the neighbours' and may be anything).
-template <int DT, bool XS>
+// (they are the neighbours' and may be anything). Vectors inside the row, all but the first and the last, need no test.
+template <int DT, bool XS, int LPR>
 __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_plain_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y,
                                                                         int row_begin, int row_end) {
-  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8, RPW = 32 / LPR;
   extern __shared__ float rag_xs[];
-  const int lane = threadIdx.x & 31, gw = (int)((blockIdx.x * RAG_THREADS + threadIdx.x) >> 5), nw = (int)(gridDim.x * RAG_THREADS) >> 5;
+  const int lane = threadIdx.x & 31, sl = lane % LPR, gw = (int)((blockIdx.x * RAG_THREADS + threadIdx.x) >> 5), nw = (int)(gridDim.x * RAG_THREADS) >> 5;
   const float* xb = x + (size_t)blockIdx.y * b.cols;
   float* yb = y + (size_t)blockIdx.y * b.rows;
   const uint4* wp = reinterpret_cast<const uint4*>(b.lo);
@@ -172,42 +177,53 @@ __global__ void __launch_bounds__(RAG_THREADS) gemv_ragged_plain_kernel(const Wv
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (XS) rag_stage_x(rag_xs, xb, b.cols);
   __syncthreads();
-  for (int row = row_begin + gw; row < row_end; row += nw) {
+  for (int r0 = row_begin + gw * RPW; r0 < row_end; r0 += nw * RPW) {
+    const int row = r0 + lane / LPR;
     const long long start = (long long)row * b.cols;
-    const int s = (int)(start % EPV), nv = (s + b.cols + EPV - 1) / EPV;
+    const int s = (int)(start % EPV), nv = row < row_end ? (s + b.cols + EPV - 1) / EPV : 0;
     const uint4* rp = wp + start / EPV;
-    float acc = 0.f;
-    for (int v0 = lane; v0 < nv; v0 += 128) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};      // short chains of additions
+    for (int v0 = sl; v0 < nv; v0 += 4 * LPR) {
       uint4 q[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) q[u] = v0 + 32 * u < nv ? __ldg(rp + v0 + 32 * u) : make_uint4(0, 0, 0, 0);
+      for (int u = 0; u < 4; u++) q[u] = v0 + LPR * u < nv ? __ldg(rp + v0 + LPR * u) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        const int c0 = (v0 + 32 * u) * EPV - s;
+        if (XS && v0 + LPR * u >= nv) break;      // (from global memory the loads of x are better off without it)
+        const int c0 = (v0 + LPR * u) * EPV - s;
         const unsigned ws[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
-#pragma unroll
-        for (int e = 0; e < EPV; e++) {
-          float w;
-          if constexpr (DT == WV_DT_F32) w = __uint_as_float(ws[e]);
+        auto weight = [&](int e) {
+          if constexpr (DT == WV_DT_F32) return __uint_as_float(ws[e]);
           else {
             const unsigned hw = (e & 1) ? ws[e >> 1] >> 16 : ws[e >> 1] & 0xffffu;
-            if constexpr (DT == WV_DT_BF16) w = __uint_as_float(hw << 16);
-            else w = __half2float(__ushort_as_half((unsigned short)hw));
+            if constexpr (DT == WV_DT_BF16) return __uint_as_float(hw << 16);
+            else return __half2float(__ushort_as_half((unsigned short)hw));
           }
-          const int col = c0 + e;
-          if (col >= 0 && col < b.cols) acc = fmaf(w, XS ? rag_xs[rag_slot(col + 32)] : __ldg(xb + col), acc);
+        };
+        if (XS && c0 >= 0 && c0 + EPV <= b.cols) {
+          const float* p0 = rag_xs + rag_slot(c0 + 32);
+          const int thr = 32 - (c0 & 31);     // from here on the next 32-float group: one word of padding further
+#pragma unroll
+          for (int e = 0; e < EPV; e++) sum[u] = fmaf(weight(e), (e < thr ? p0 : p0 + 1)[e], sum[u]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < EPV; e++) {
+            const int col = c0 + e;
+            if (col >= 0 && col < b.cols) sum[u] = fmaf(weight(e), XS ? rag_xs[rag_slot(col + 32)] : __ldg(xb + col), sum[u]);
+          }
         }
       }
     }
+    float acc = (sum[0] + sum[1]) + (sum[2] + sum[3]);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) yb[row] = acc;
+    for (int o = LPR / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (sl == 0 && row < row_end) yb[row] = acc;
   }
 }
 
 // ------------------------------------------------------------------ host side
 template <typename K>
-static int rag_go(K kern, bool xs, const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st, unsigned& attr_mask) {
+static int rag_go(K kern, bool xs, int lpr, const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st, unsigned& attr_mask) {
   const size_t smem = xs ? ((size_t)b.cols + 96 + (b.cols + 96) / 32 + 1) * 4 : 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -217,28 +233,47 @@ static int rag_go(K kern, bool xs, const WvDevBlob& b, const float* dx, float* d
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) { wv_set_error("gemv (ragged): cannot raise the shared-memory limit"); return WV_ECUDA; }
     attr_mask |= 1u << (dev & 31);
   }
-  // a warp per row until the SMs hold no more CTAs side by side; then rows in turn, so that x is staged at most that often
+  // `lpr` lanes per row until the SMs hold no more CTAs side by side; then rows in turn, so that x is staged at most that often
   int per_sm = smem ? (int)((220 * 1024) / smem) : 8;
   per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
-  int grid = (re - rb + RAG_THREADS / 32 - 1) / (RAG_THREADS / 32);
+  const int rpc = RAG_THREADS / lpr;
+  int grid = (re - rb + rpc - 1) / rpc;
   if (grid > per_sm * wv_sm_count()) grid = per_sm * wv_sm_count();
   const cudaError_t e = launch_pdl(kern, dim3(grid, batch), dim3(RAG_THREADS), smem, st, b, dx, dy, rb, re);
   if (e != cudaSuccess) { wv_set_error("gemv (ragged) launch: %s", cudaGetErrorString(e)); return WV_ECUDA; }
   return WV_OK;
 }
+// Lanes per row. A row has `units` chunks or vectors at most: lanes beyond that idle (27 of 32 at 100 columns), and the last of a
+// row's steps fills its lanes only in part (33 chunks take two steps of 32 lanes or five of eight). So as few lanes as leave
+// 16 warps for every SM: with fewer warps the latency of a row's steps shows. A warp per row, whatever the shape, took 149 us
+// for 33 rows of Q8_0 at 9001 x 46 and 60 us for 33 of bf16 at 2730 x 1022; the weight-by-weight kernel takes 70 and 49, this
+// 34 and 45.
+static int rag_lanes(int units, int rows, int batch) {
+  int lpr = units <= 8 ? 8 : (units <= 16 ? 16 : 32);
+  while (lpr > 8 && units <= 6 * lpr && (long long)rows * batch * (lpr / 2) / 32 >= 16 * wv_sm_count()) lpr /= 2;
+  return lpr;
+}
 template <int F>
 static int rag_format(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
-  static unsigned attr[2] = {0, 0};
-  if (b.cols <= RAG_MAX_COLS) return rag_go(gemv_ragged_chunk_kernel<F, true>, true, b, dx, dy, batch, rb, re, st, attr[0]);
-  return rag_go(gemv_ragged_chunk_kernel<F, false>, false, b, dx, dy, batch, rb, re, st, attr[1]);
+  static unsigned attr[4] = {0, 0, 0, 0};
+  if (b.cols > RAG_MAX_COLS) return rag_go(gemv_ragged_chunk_kernel<F, false, 32>, false, 32, b, dx, dy, batch, rb, re, st, attr[3]);
+  switch (rag_lanes((b.cols + 62) >> 5, re - rb, batch)) {
+  case 8: return rag_go(gemv_ragged_chunk_kernel<F, true, 8>, true, 8, b, dx, dy, batch, rb, re, st, attr[0]);
+  case 16: return rag_go(gemv_ragged_chunk_kernel<F, true, 16>, true, 16, b, dx, dy, batch, rb, re, st, attr[1]);
+  }
+  return rag_go(gemv_ragged_chunk_kernel<F, true, 32>, true, 32, b, dx, dy, batch, rb, re, st, attr[2]);
 }
 template <int DT>
 static int rag_plain(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
-  static unsigned attr[2] = {0, 0};
-  if (b.cols <= RAG_MAX_COLS) return rag_go(gemv_ragged_plain_kernel<DT, true>, true, b, dx, dy, batch, rb, re, st, attr[0]);
-  return rag_go(gemv_ragged_plain_kernel<DT, false>, false, b, dx, dy, batch, rb, re, st, attr[1]);
+  static unsigned attr[4] = {0, 0, 0, 0};
+  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  if (b.cols > RAG_MAX_COLS) return rag_go(gemv_ragged_plain_kernel<DT, false, 32>, false, 32, b, dx, dy, batch, rb, re, st, attr[3]);
+  switch (rag_lanes((b.cols + 2 * EPV - 2) / EPV, re - rb, batch)) {
+  case 8: return rag_go(gemv_ragged_plain_kernel<DT, true, 8>, true, 8, b, dx, dy, batch, rb, re, st, attr[0]);
+  case 16: return rag_go(gemv_ragged_plain_kernel<DT, true, 16>, true, 16, b, dx, dy, batch, rb, re, st, attr[1]);
+  }
+  return rag_go(gemv_ragged_plain_kernel<DT, true, 32>, true, 32, b, dx, dy, batch, rb, re, st, attr[2]);
 }
-
 int wv_launch_gemv_flat(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st);   // wv_layout.cu
 
 int wv_launch_gemv_ragged(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st) {
