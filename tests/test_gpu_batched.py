@@ -308,3 +308,17 @@ def test_batched_few_rows_many_columns(wv, fmt, shape):
         x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
         y, _ = _run(wv, ob, x)
         assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch
+
+
+@pytest.mark.parametrize("group,cols", [(32, 1920), (96, 1920), (160, 1920), (256, 2048), (96, 1056)])
+def test_batched_affine_groups(wv, group, cols):
+    """Groups of one, three, five and eight chunks: inside a producer's load unit, across two units, and (1056 columns, 33 chunks)
+    chunk by chunk."""
+    rows = 200
+    w = np.random.default_rng(group).normal(0, 0.02, rows * cols).astype(np.float32)
+    ob = O.pack("AffinePacked", w, rows, cols, group)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    for batch in (6, 70):
+        x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
+        y, _ = _run(wv, ob, x)
+        assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch

@@ -97,12 +97,32 @@ __device__ __forceinline__ void tcg_load(FragT<F> (&f)[TcgUnit<F>::U], const WvD
 #pragma unroll
       for (int u = 0; u < U; u++) { f[u].pr[0] = __float_as_uint(dd.x); f[u].pr[1] = __float_as_uint(dd.y); f[u].pr[2] = km[u]; }
     } else if constexpr (fi.kind == WK_BINARY || fi.kind == WK_AFFINE) {
-      const unsigned cpg = (unsigned)b.group >> 5;   // whole chunks per group
+      // Whole chunks per group. Every load is 32 lines, so a group's parameters are loaded once for the chunks of it that are in the
+      // unit, and groups of one chunk like those of the other formats: a load per chunk made these formats slower at few rows of W
+      // than they had been (six rows, 1024 x 14336, groups of 64: 22.3 us once, 23.9 with a load per chunk, 21.2 now).
+      const unsigned cpg = (unsigned)b.group >> 5;
+      if (cpg == 1) {
+        unsigned p0[U], p1[U];
+        tcg_words(p0, b.p0 + ch);
+        if constexpr (fi.has_min) tcg_words(p1, b.p1 + ch);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          f[u].pr[0] = p0[u];
+          if constexpr (fi.has_min) f[u].pr[1] = p1[u];
+        }
+        return;
+      }
+      unsigned gi = (unsigned)ch / cpg, in = (unsigned)ch - gi * cpg;      // `in` is the same for every row: a row is whole groups
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        const unsigned gi = (unsigned)(ch + u) / cpg;
-        f[u].pr[0] = __float_as_uint(__ldg(b.p0 + gi));
-        if constexpr (fi.has_min) f[u].pr[1] = __float_as_uint(__ldg(b.p1 + gi));
+        if (u == 0 || in == 0) {
+          f[u].pr[0] = __float_as_uint(__ldg(b.p0 + gi));
+          if constexpr (fi.has_min) f[u].pr[1] = __float_as_uint(__ldg(b.p1 + gi));
+        } else {
+          f[u].pr[0] = f[u > 0 ? u - 1 : 0].pr[0];
+          if constexpr (fi.has_min) f[u].pr[1] = f[u > 0 ? u - 1 : 0].pr[1];
+        }
+        if (++in == cpg) { in = 0; gi++; }
       }
     } else {
       constexpr int NG = fi.pgroup == 16 ? 2 : 1;
