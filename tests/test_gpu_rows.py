@@ -86,9 +86,24 @@ def test_few_rows_of_w_run_row_by_row(wv, fmt, rows, cols, batch):
 
 @pytest.mark.parametrize("fmt", ["TernaryPacked", "IQ1_S", "Q4_0"])
 def test_two_rows_of_wide_matrices_run_one_by_one(wv, fmt):
-    rows, cols = 300, 9216
+    rows, cols = 1200, 9216
     w, _ = make_w(2, rows, cols)
     ob = O.pack(fmt, w, rows, cols)
     x = np.random.default_rng(3).normal(0, 1, (2, cols)).astype(np.float32)
     y, _ = _run(wv, ob, x)
     assert np.array_equal(y, np.concatenate([_run(wv, ob, x[m:m + 1])[0] for m in range(2)]))
+
+
+@pytest.mark.parametrize("fmt", ["TernaryPacked", "Q4_K"])
+def test_two_rows_of_a_streamed_wide_matrix_keep_their_precision(wv, fmt):
+    """More than 64 MB of codes at 9216 columns: two rows stay on the integer-dot kernel, whose error the tensor cores' TF32
+    (2.9e-4 of the result's norm) exceeds."""
+    n, block, cols = {"TernaryPacked": 112, "Q4_K": 56}[fmt], 256, 9216
+    w = np.random.default_rng(5).normal(0, 0.02, block * cols).astype(np.float32)
+    ob = O.pack(fmt, w, block, cols)          # rows are whole groups: a block of them, repeated
+    big = O.Blob(ob.format, n * block, cols, np.tile(ob.raw, n), np.tile(ob.scales, n), np.tile(ob.mins, n), ob.block_weights, ob.dtype)
+    x = np.random.default_rng(6).normal(0, 1, (2, cols)).astype(np.float32)
+    y, _ = _run(wv, big, x)
+    ref = np.tile(x.astype(np.float64) @ O.unpack(ob).reshape(block, cols).astype(np.float64).T, n)
+    # 16-bit records: an activation is off by amax / 65024 of its chunk at most, some 5e-5 of its size on the average
+    assert np.linalg.norm(y - ref) <= 1e-4 * np.linalg.norm(ref)

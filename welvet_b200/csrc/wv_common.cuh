@@ -99,6 +99,12 @@ struct WvDevBlob {
   const uint32_t* km;   // k-quants: per-chunk scale/min bytes
 };
 
+// A matrix whose codes alone take more than 64 MB: row by row it would be streamed from HBM once per activation row.
+__host__ inline bool wv_beyond_l2(const WvDevBlob& b) {
+  const WvFmtInfo fi = wv_fmt_info(b.format);
+  return (double)b.n * (fi.bits_lo + fi.bits_hi) / 8.0 > 64e6;
+}
+
 // ---- chunk-internal addressing -------------------------------------------------------
 template <int B> struct WvLane {
   static constexpr int CPW = 32 / B;   // codes per lo word

@@ -759,9 +759,7 @@ int wv_launch_gemv(const WvDevBlob& b, const float* dx, float* dy, int batch, in
   }
   // What that kernel does not take of a matrix that does not fit L2 would be streamed from HBM once per row, so there the
   // tensor-core kernel takes every batch.
-  const WvFmtInfo bfi = wv_fmt_info(b.format);
-  const bool big = (double)b.n * (bfi.bits_lo + bfi.bits_hi) / 8.0 > 64e6;
-  if (batched && (batch >= batch_min() || big)) {
+  if (batched && (batch >= batch_min() || wv_beyond_l2(b))) {
     // Several activation rows: the tensor-core kernel streams and dequantises the matrix once for up to 256 of
     // them. What it does not take (FormatNone, ragged rows) runs row by row below.
     int rc = wv_launch_gemm_tcgen05(b, dx, dy, batch < 256 ? batch : 256, row_begin, row_end, st);

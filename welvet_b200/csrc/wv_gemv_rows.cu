@@ -346,15 +346,16 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
   // So few rows of W that row by row the CTAs of all activation rows run side by side, or nearly: that takes 3.6 - 4.4 us as long
   // as there is an SM for each and 6.9 - 7.9 us up to two for each, while this kernel spreads the rows of W alone over the chip
   // and takes 2.4 - 3.2 us and 1.45 us for each of a CTA's activation rows (Q4_K, four rows: 24 x 4096 4.1 against 8.2 us,
-  // 64 x 6144 7.5 against 9.1; three rows, 64 x 4096: 7.6 against 6.9).
+  // 64 x 6144 7.5 against 9.1; three rows, 64 x 4096: 7.6 against 6.9; two rows, 128 x 9216: 7.5 against 6.9).
   const int ny = (batch + ROWS_NB - 1) / ROWS_NB, nb = (batch + ny - 1) / ny;
   const long long side = (long long)(re - rb_) * batch, sms = wv_sm_count();
-  if (side <= sms || (side <= 2 * sms && nb * g.nwc >= 16)) return 1;
+  if (side <= sms || (side <= 2 * sms && nb >= 3 && nb * g.nwc >= 16)) return 1;
   g.nrg = TMA_CONSUMER_WARPS / g.nwc;
   // One row group (more than eight column warps) leaves up to seven warps idle: two activation rows are faster one by one in the
   // formats that unpack cheaply (no hi plane; 4096 x 9216: IQ1_S 14.2 against 14.7 us, Ternary 14.3 against 15.2; IQ3_S, with one,
-  // 17.4 against 16.5), three are not (Ternary 21.2 against 19.6).
-  if (g.nrg == 1 && batch == 2 && wv_fmt_info(F).bits_hi == 0) return 1;
+  // 17.4 against 16.5), three are not (Ternary 21.2 against 19.6), nor are two rows of a matrix of few rows (128 x 9216, Ternary: 7.1
+  // against 6.9) or of one that is streamed from HBM and would go to the tensor-core kernel (40960 x 9216, Ternary: 199 against 101).
+  if (g.nrg == 1 && batch == 2 && wv_fmt_info(F).bits_hi == 0 && re - rb_ >= 8 * sms && !wv_beyond_l2(b)) return 1;
   if (g.nrg > TMA_MAX_ROW_GROUPS) g.nrg = TMA_MAX_ROW_GROUPS;
   g.tr = g.nrg * ROWS_RT;
   g.wide = wv_act_width() == 3;
