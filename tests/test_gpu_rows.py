@@ -11,7 +11,7 @@ from test_gpu_batched import _run
 pytestmark = pytest.mark.gpu
 
 # rows x cols: fewer rows than SMs, a partial last tile, one column warp, a partial last column warp (1280 = 40 chunks),
-# 4608 (formats that the tensor pipe takes up to 4096), 6144 (the widest in most formats), 14336 (row by row)
+# 4608 (formats that the tensor pipe takes up to 4096), 6144, 14336 (row by row); the smallest run row by row in most batches
 SHAPES = [(5, 512), (300, 1024), (149, 1280), (450, 4096), (40, 4608), (64, 6144), (40, 14336)]
 
 
@@ -107,3 +107,28 @@ def test_two_rows_of_a_streamed_wide_matrix_keep_their_precision(wv, fmt):
     ref = np.tile(x.astype(np.float64) @ O.unpack(ob).reshape(block, cols).astype(np.float64).T, n)
     # 16-bit records: an activation is off by amax / 65024 of its chunk at most, some 5e-5 of its size on the average
     assert np.linalg.norm(y - ref) <= 1e-4 * np.linalg.norm(ref)
+
+
+# a band of one row in some CTAs, widths with two row groups (2048 to 8192, where 4-bit formats have no room for their ring)
+# and with one (8704)
+WIDE_SHAPES = [(100, 2048), (100, 7168), (100, 8192), (100, 8704)]
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[0] != "none"], ids=case_id)
+@pytest.mark.parametrize("shape", WIDE_SHAPES, ids=lambda s: f"{s[0]}x{s[1]}")
+def test_rows_four_to_a_cta(wv, case, shape):
+    """Four activation rows: all of a CTA's record slots in use, each against float64."""
+    rows, cols = shape
+    if not case_ok(case, rows, cols):
+        pytest.skip("layout needs aligned cols")
+    f, bw, dt = case
+    w, _ = make_w(rows + cols, rows, cols)
+    ob = O.pack(f, w, rows, cols, bw, dt)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    x = np.random.default_rng(cols).normal(0, 1, (4, cols)).astype(np.float32)
+    x[3] *= 1e3
+    x[1, ::97] *= 1e4             # outliers: 24-bit records for this row only
+    y, _ = _run(wv, ob, x)
+    for m in range(4):
+        err = np.abs(y[m] - wd @ x[m].astype(np.float64))
+        assert np.all(err <= 2 * _bound(ob, x[m])), (m, float(np.max(err / _bound(ob, x[m]))))
