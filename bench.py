@@ -522,7 +522,8 @@ def small_batch_gemm(torch, L, _lib, stream, O):
             us = _timed_graph(torch, stream, None, run) / n_l * 1e3
             row = {"format": name, "M": M, "us": round(us, 2), "gbs_packed_weights": round(nbytes / us / 1e3, 1),
                    "tflops": round(2.0 * M * rows * cols / us / 1e6, 2),
-                   "kernel": "tcgen05 (TF32 operands, W dequantised once)" if M >= 6 else "batch-1 integer-dot kernel, one launch per row"}
+                   "kernel": "tcgen05 (TF32 operands, W dequantised once)" if M >= 6 else
+                   "integer-dot rows kernel, up to four rows per pass over W" if M > 1 and name != "Q8_0" else "batch-1 integer-dot kernel, a launch row per activation row"}
             if ob is not None:
                 got = y.cpu().numpy()
                 worst = 0.0

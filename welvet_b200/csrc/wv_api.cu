@@ -785,8 +785,8 @@ static int grow(float** p, size_t* cap, size_t n, bool pinned) {
 // goroutines, layers/dense/cpu.go forwardTiledMC) overlap instead of queueing on one lock. x is copied into mapped pinned
 // memory and brought to the device by a one-CTA kernel (a copy-engine transfer of a few kilobytes costs more in start-up
 // than in transfer); the GEMV behind it is launched with programmatic stream serialisation, so its prologue overlaps
-// that kernel; y is stored by the GEMV straight into mapped pinned memory. Calls with a batch share slot 0: the
-// batched kernel's buffer of rounded activations belongs to the library and takes one launch at a time.
+// that kernel; y is stored by the GEMV straight into mapped pinned memory. Calls with a batch share slot 0, the
+// only one whose buffers grow to a batch's size.
 // A slot also keeps one instantiated CUDA graph per matrix it has served (copy-in kernel + GEMV with the slot's fixed
 // buffers): launches from several host threads are serialised by the driver, so a call that costs one graph launch instead
 // of two kernel launches leaves more of the GPU to the other callers. A graph is built on the second call for a matrix

@@ -14,15 +14,17 @@
 // a row tile are one thread-block cluster, which adds its accumulators up in split order through distributed shared
 // memory.
 //
-// Bound: up to some 64 rows the producers' instruction stream (five instructions per weight) together with the MMAs, which
-// take about 52 cycles each however few rows X has; at 256 rows the copies of X out of L2 (every row tile reads all of it) and
-// the tensor pipe. Measured against the version before (512 producers of 8 weights each, two slices a stage, issue loops run
-// by one lane, split sums through global memory), 16 / 64 / 256 rows: Q8_0 4096 x 4096 21.7 / 28.3 / 56.9 -> 15.9 / 18.2 /
-// 26.2 us, Q4_K 14336 x 4096 66.2 / 67.6 / 82.0 -> 36.6 / 41.9 / 55.2 us, Q4_0 1024 x 1024 12.0 / 18.2 / 42.6 -> 8.1 / 9.3 /
-// 15.4 us. With the loads and the conversion left out the 14336 x 4096 launch takes 15.5 us at 16 rows.
+// Bound: up to some 64 rows the latency of the producers' loads and instructions (eight executed per weight, all roles together)
+// and of the MMAs, which take about 52 cycles each however few rows X has; at 256 rows the tensor pipe (70 % of active cycles) and
+// the copies of X out of L2 (every row tile reads all of it). Measured against the version before (512 producers of 8 weights
+// each, two slices a stage, issue loops run by one lane, split sums through global memory), 16 / 64 / 256 rows, six matrices in
+// turn and one Y: Q8_0 4096 x 4096 21.7 / 28.3 / 56.9 -> 15.7 / 17.9 / 25.9 us, Q4_K 14336 x 4096 66.2 / 67.6 / 82.0 -> 36.6 /
+// 41.1 / 54.0 us (256 rows with a Y of 14.7 MB for each of four matrices: 83 -> 60.5), Q4_0 1024 x 1024 12.0 / 18.2 / 42.6 ->
+// 8.2 / 9.5 / 16.1 us. With the loads and the conversion left out the 14336 x 4096 launch takes 15.5 us at 16 rows.
 //
-// Arithmetic: both operands are rounded to TF32 (round to nearest, 11 significant bits) by the producers, so the
-// hardware's truncation of the low mantissa bits drops zeros; products are exact in the FP32 accumulator. Each term
+// Arithmetic: X is rounded to TF32 (round to nearest, 11 significant bits) with its low bits cleared, a weight by adding half a
+// unit of the eleventh bit to it, the rest being the tensor core's truncation, which reads an operand's upper 19 bits only;
+// products are exact in the FP32 accumulator. Each term
 // is off by at most 2^-11 + 2^-11 + 2^-22 of |w x|, i.e. |y - y_ref| <= 9.8e-4 * sum |w x| before accumulation
 // rounding. TF32 keeps FP32's exponent range, so no operand needs scaling.
 //

@@ -751,8 +751,11 @@ int wv_launch_gemv(const WvDevBlob& b, const float* dx, float* dy, int batch, in
   if (pp && batch != 1) return WV_ESHAPE;
   const bool batched = batch >= 2 && !pp && !wv_cur_fuse && !g_tune_r && !wv_tma_tuning_rt() && !batch_loop_forced();   // a kernel forced by a tuning code keeps the batch on it
   // A few rows: up to four per pass over W on the integer-dot kernel, which is more precise than the tensor cores' TF32.
-  // At 4096 x 4096 in Q4_K four rows take 11.1 us there, 22.8 on the tensor-core kernel, 18.8 row by row; from six rows
-  // (two passes, 18.9) the tensor-core kernel's time, which hardly depends on the batch, is the better one.
+  // Up to five rows that precision decides: in time the lines cross between four and five rows at 4096 x 4096 (Q4_K 11.3 us for
+  // four rows, 16.6 for five, the tensor-core kernel 15.3 whatever the batch; Q8_0, row by row, 13.6 and 16.7 against 15.6) and
+  // between five and six at 14336 x 4096 (Q4_K 35.9 and 40.4 against 36.3, Q8_0 36.5 and 42.6 against 38.7). At six the
+  // tensor-core kernel is the faster one, but for small matrices (1024 x 4096 in Q8_0 and Q4_0: 8.6 row by row, 10.8 and 10.3 there;
+  // level at eight rows).
   if (batched && batch < batch_min()) {
     const int rc = wv_launch_gemv_rows(b, dx, dy, batch, row_begin, row_end, st);
     if (rc != 1) return rc;

@@ -10,10 +10,11 @@
 // neighbour's infinity is no zero, and codes summed before they are scaled overflow for activations whose products with the
 // weights do not.
 //
-// Bound: launch and memory latency (a 2730 x 1022 matrix is 1 - 3 MB). A weight costs about 7 instructions; the
-// weight-by-weight kernel this replaces spent some 60 (64-bit index arithmetic, bit extraction from global memory
+// Bound: launch and memory latency for one activation row (a 2730 x 1022 matrix is 1 - 3 MB), instructions from some eight rows
+// on (33 rows of Q4_0 at 9001 x 100: 78 % of the issue slots). A weight of a lane's
+// chunk costs some 14 instructions there, all included; the weight-by-weight kernel this replaces spent some 60 (64-bit index arithmetic, bit extraction from global memory
 // and, for the k-quants, two divisions). Measured back to back on a stream, Q8_0, Q4_0, Q4_K and IQ3_S at 2730 x 1022
-// and 1022 x 2730: 271 us before for the eight launches, 43 us now (5.4 us a launch, of which about 4 us is the
+// and 1022 x 2730: 271 us before for the eight launches, 41.6 us now (3.7 to 6.1 us a launch, of which about 4 us is the
 // host's own cost of a call).
 #include "wv_dequant.cuh"
 #include "wv_gemv_common.cuh"

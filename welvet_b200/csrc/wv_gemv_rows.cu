@@ -393,12 +393,15 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
 }
 
 // Returns 1 for what this kernel does not take: FormatNone, IQ4_NL (float table arithmetic), planes whose rows are no 16-byte
-// multiples, few rows of W (launch_rows), the formats and widths below, and rows so wide that four rows' records leave the ring no room for two tiles (beyond 6144 columns in Q4_K).
+// multiples, few rows of W (launch_rows), the formats and widths below, and rows so wide that four rows' records leave the ring
+// no room for two tiles: beyond 6144 columns in Q5_1 and Q6_K, 6656 in Q5_K, 7168 in the other 4-bit formats and IQ3_S, 7680 in Q3_K,
+// 8192 in Q2_K, 9216 to 11264 in the other 1- and 2-bit formats. A tile halves beyond 8192 columns (one row group instead of two),
+// so that all but Q5_1 and Q6_K are taken again from there to 8704 - 9216 (Q2_K 10240).
 int wv_launch_gemv_rows(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st) {
   if (batch < 2 || !b.fast || b.format == WV_NONE || row_end <= row_begin || !wv_tma_err_ptr()) return 1;
   // What runs as 24-bit records on the tensor pipe row by row (gemv_mma_kernel: Q8_0, and the formats with one parameter
-  // group per chunk up to 4096 columns) stays there: three limbs instead of two make this kernel slower than that one (Q8_0
-  // at 4096 x 4096, four rows: 17.9 against 13.6 us), and two would be less precise.
+  // group per chunk up to 4096 columns) stays there whatever the shape, since two limbs would be less precise. Three would make
+  // this kernel the slower one where it was tried (Q8_0 at 4096 x 4096, four rows: 17.9 against 13.6 us).
   const WvFmtInfo fi = wv_fmt_info(b.format);
   if (b.format == WV_Q8_0 || (b.cols <= 4096 && b.format != WV_IQ3_XXS && fi.kind != WK_KQUANT && fi.pgroup != 16)) return 1;
   switch (b.format) {
