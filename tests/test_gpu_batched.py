@@ -322,3 +322,31 @@ def test_batched_affine_groups(wv, group, cols):
         x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
         y, _ = _run(wv, ob, x)
         assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch
+
+
+def test_batched_graphs_come_and_go(wv):
+    """Graphs captured and dropped one after another, each with more rows than the last, so that no buffer given back is large
+    enough for the next; then one with few rows, which reuses one, and a larger call outside a capture, which frees the rest."""
+    rows, cols = 1024, 2048
+    L = wv._lib.lib()
+    key, _keep = _packed(wv, "Q8_0", rows, cols, 34)
+    side = torch.cuda.Stream()
+    gen = torch.Generator("cuda").manual_seed(35)
+    x, y = torch.zeros(6, cols, device="cuda"), torch.zeros(6, rows, device="cuda")
+    wv._lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), 6, cols, rows, side.cuda_stream))      # the kernel is loaded before any capture
+    for batch in (8, 40, 120, 16, 250):
+        x, y = torch.randn(batch, cols, device="cuda", generator=gen), torch.zeros(batch, rows, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            wv._lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, rows, torch.cuda.current_stream().cuda_stream))
+        g.replay()
+        torch.cuda.synchronize()
+        got = y.clone()
+        g.reset()
+        del g
+        y.zero_()
+        wv._lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, rows, side.cuda_stream))
+        torch.cuda.synchronize()
+        assert torch.equal(got, y), batch
+    assert L.wv_device_status() == 0

@@ -598,6 +598,14 @@ struct TcgBufs {
   int nstreams = 0;
   std::vector<TcgBuf*> captured, idle;             // held by a graph or by a capture in progress; free for the next capture
   std::atomic<TcgBuf*> returned{nullptr};          // given back by graphs that went away: a lock-free list, as the driver calls back
+  void collect() {                                 // under mu
+    for (TcgBuf* b = returned.exchange(nullptr); b;) {
+      TcgBuf* next = b->next;
+      for (size_t i = 0; i < captured.size(); i++) if (captured[i] == b) { captured[i] = captured.back(); captured.pop_back(); break; }
+      idle.push_back(b);
+      b = next;
+    }
+  }
 };
 static TcgBufs& tcg_bufs() { static TcgBufs* b = new TcgBufs; return *b; }     // outlives every graph
 static void CUDART_CB tcg_give_back(void* q) {
@@ -625,19 +633,12 @@ static int tcg_lease(TcgLease& out, size_t floats, cudaStream_t st) {
   if (status != cudaStreamCaptureStatusNone || cudaStreamGetId(st, &id) != cudaSuccess) { cudaGetLastError(); id = reinterpret_cast<uintptr_t>(st); }
   if (status == cudaStreamCaptureStatusActive) {
     std::lock_guard<std::mutex> lk(bufs.mu);
-    for (TcgBuf* b = bufs.returned.exchange(nullptr); b;) {
-      TcgBuf* next = b->next;
-      for (size_t i = 0; i < bufs.captured.size(); i++) if (bufs.captured[i] == b) { bufs.captured[i] = bufs.captured.back(); bufs.captured.pop_back(); break; }
-      bufs.idle.push_back(b);
-      b = next;
-    }
+    bufs.collect();
     for (TcgBuf* b : bufs.captured) if (b->capture == cap && b->stream == id && b->floats >= floats) { out.p = b->p; return WV_OK; }
     TcgBuf* b = nullptr;
     for (size_t i = 0; i < bufs.idle.size() && !b; i++) if (bufs.idle[i]->floats >= floats) { b = bufs.idle[i]; bufs.idle[i] = bufs.idle.back(); bufs.idle.pop_back(); }
     TcgRelaxed relaxed;
-    if (!b) {
-      for (TcgBuf* q : bufs.idle) { cudaFree(q->p); delete q; }      // all too small
-      bufs.idle.clear();
+    if (!b) {        // those that are too small stay for now: freeing waits for the device, which a capture forbids
       float* p = nullptr;
       if (cudaMalloc(&p, floats * 4) != cudaSuccess) return fail();
       b = new TcgBuf{p, floats, 0, 0, nullptr};
@@ -668,6 +669,12 @@ static int tcg_lease(TcgLease& out, size_t floats, cudaStream_t st) {
     cudaStreamSynchronize(st);            // nothing else has ever used this buffer
     if (sb->p) cudaFree(sb->p);
     sb->p = nullptr; sb->floats = 0;
+    {
+      std::lock_guard<std::mutex> lk(bufs.mu);      // set-up time: what captures left behind goes as well
+      bufs.collect();
+      for (TcgBuf* q : bufs.idle) { cudaFree(q->p); delete q; }
+      bufs.idle.clear();
+    }
     if (cudaMalloc(&sb->p, floats * 4) != cudaSuccess) return fail();
     sb->floats = floats;
   }
