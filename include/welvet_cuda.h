@@ -79,6 +79,12 @@ int wv_blob_info(uint64_t key, int* rows, int* cols, uint64_t* wire_bytes, uint6
  * Host pointers, synchronous, like the reference's device path (affine_cache.go:370-445).
  * Checks in == cols and out == rows (dense.dims, layers/dense/dense.go:129-143). */
 int wv_matvec(uint64_t key, const float* x, float* y, int batch, int in, int out);
+/* dense.Forward's two results for float32 (applyBiasAct, layers/dense/dense.go:145-167): pre = W x + bias and
+ * post = act(pre), each [batch, out] on the host. The bias is added in float64 to the first nbias columns of a row (all of
+ * them when nbias >= out; bias may be NULL when nbias == 0), pre is that sum rounded to float32, and the activation (a
+ * core.ActivationType value, core/layer.go:91-98) is evaluated in float64 on the rounded sum. Synchronous, like wv_matvec. */
+int wv_matvec_bias_act(uint64_t key, const float* x, const double* bias, int nbias, int act, float* pre, float* post,
+                       int batch, int in, int out);
 /* Device pointers, asynchronous on `stream` (a cudaStream_t; NULL = default stream). For
  * chained decode and for benchmarking with inputs resident in HBM. */
 int wv_matvec_dev(uint64_t key, const float* dx, float* dy, int batch, int in, int out, void* stream);

@@ -109,6 +109,29 @@ def test_dense_forward_batched(wv):
         assert np.allclose(post[m], pm / (1 + np.exp(-pm)), rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("rows,cols,batch,nbias", [(333, 512, 1, 333), (512, 1024, 8, 600), (130, 254, 5, 7), (257, 512, 3, 0)])
+def test_dense_forward_bias_and_activations(wv, rows, cols, batch, nbias):
+    """Bias and activation behind the GEMV against the float64 passes of dense.Activate: biases shorter and longer than a row, every
+    activation. The sum is the same bits; the activation may round to the neighbouring float32 (float64 functions of a few
+    units in the last place each; 1 + tanh(v) loses its leading digits for negative v, hence the term in |v|)."""
+    d = wv.dense
+    rng = np.random.default_rng(rows)
+    layer = d.NewConfigured(cols, rows, d.ActivationLinear, wv.quant.DTypeFloat32, wv.quant.Format.FormatQ5_0, rng.normal(0, 0.1, rows * cols).astype(np.float32))
+    x = rng.normal(0, 1, (batch, cols)).astype(np.float32)
+    y = d.Forward(layer, x)[0].astype(np.float64)
+    if nbias:
+        layer.Weights.Bias = rng.normal(0, 1, nbias)
+        y[:, :nbias] += layer.Weights.Bias[:rows]
+    for act in d._ACTIVATIONS:
+        layer.Activation = act
+        pre, post = d.Forward(layer, x)
+        assert pre.dtype == post.dtype == np.float32 and (pre is post) == (act == d.ActivationLinear and not nbias)
+        np.testing.assert_array_equal(pre, y.astype(np.float32))
+        p = pre.astype(np.float64)
+        ref = d.Activate(p, act)
+        assert np.all(np.abs(post - ref) <= 2.0 ** -23 * np.abs(ref) + 2.0 ** -49 * np.abs(p) + 1e-45), act
+
+
 def test_host_pointer_calls_from_threads(wv):
     """wv_matvec (host pointers in and out) from six threads at once, as goroutines call Dense in the reference: the
     staging slots keep the calls apart, every result equals the single-threaded one bit for bit."""

@@ -17,7 +17,7 @@ SYMBOLS = [
     "wv_init", "wv_available", "wv_device_count", "wv_last_error",
     "wv_blob_upload", "wv_blob_upload_wire", "wv_blob_upload_shard", "wv_shard_range",
     "wv_blob_has", "wv_blob_evict", "wv_cache_clear", "wv_cache_bytes", "wv_cache_set_limit",
-    "wv_blob_info", "wv_matvec", "wv_matvec_dev", "wv_unpack", "wv_unpack_dev",
+    "wv_blob_info", "wv_matvec", "wv_matvec_bias_act", "wv_matvec_dev", "wv_unpack", "wv_unpack_dev",
     "wv_pack_sizes", "wv_pack", "wv_pack_upload_dev", "wv_device_status", "wv_matvec_dev_static",
     "wv_argmax_dev", "wv_argmax", "wv_matvec_dev_multi", "wv_matvec_dev_gather", "wv_gather_alloc", "wv_gather_open", "wv_gather_close", "wv_gather_free", "wv_gather_read", "wv_gather_signal", "wv_gather_wait", "wv_gather_sync",
     "wv_matvec_dev_swiglu", "wv_matvec_dev_add", "wv_matvec_dev_group_gather", "wv_matvec_dev_fused", "wv_rmsnorm_dev", "wv_rope_cache_dev",
@@ -84,6 +84,7 @@ def lib() -> C.CDLL:
         L.wv_blob_evict.argtypes = [u64]
         L.wv_blob_info.argtypes = [u64, C.POINTER(i), C.POINTER(i), C.POINTER(u64), C.POINTER(u64), C.POINTER(i)]
         L.wv_matvec.argtypes = [u64, vp, vp, i, i, i]
+        L.wv_matvec_bias_act.argtypes = [u64, vp, vp, i, i, vp, vp, i, i, i]
         L.wv_matvec_dev.argtypes = [u64, vp, vp, i, i, i, vp]
         L.wv_matvec_dev_static.argtypes = [u64, vp, vp, i, i, vp]
         L.wv_argmax_dev.argtypes = [vp, i, vp, vp]

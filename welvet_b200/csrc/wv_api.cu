@@ -798,6 +798,8 @@ struct StageSlot {
   cudaStream_t st = nullptr;
   float *hx = nullptr, *hx_dev = nullptr, *dx = nullptr, *hy = nullptr, *hy_dev = nullptr;
   size_t hx_n = 0, dx_n = 0, hy_n = 0;
+  float *ax = nullptr, *ax_dev = nullptr, *da = nullptr, *ay = nullptr, *ay_dev = nullptr;   // wv_matvec_bias_act: its inputs, device side, results
+  size_t ax_n = 0, da_n = 0, ay_n = 0;
   std::unordered_map<uint64_t, SlotGraph> graphs;
   void drop_graphs() {
     for (auto& kv : graphs) if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -825,14 +827,8 @@ static int grow_mapped(float** h, float** d, size_t* cap, size_t n) {
   return WV_OK;
 }
 
-extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int in, int out) {
-  int rc = ensure_init();
-  if (rc) return rc;
-  if (!x || !y) { wv_set_error("wv_matvec: null pointer"); return WV_EARG; }
-  Entry e;
-  if ((rc = lookup(key, &e))) return rc;
-  if ((rc = check_dims(e, batch, in, out))) return rc;
-  const size_t nx = (size_t)batch * in, ny = (size_t)batch * out;
+// A locked slot for a call, with its stream.
+static int take_slot(int batch, StageSlot** out) {
   StageSlot* slot = nullptr;
   if (batch == 1) {
     // a caller thread keeps coming back to the slot it took first, so that slot's buffers and launch graphs serve it again
@@ -848,11 +844,30 @@ extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int 
     slot = &g_slots[0];
     slot->mu.lock();
   }
-  std::lock_guard<std::mutex> lk(slot->mu, std::adopt_lock);
   if (!slot->st) {
     if (slot == &g_slots[0]) slot->st = g_stream;
-    else CUDA_TRY(cudaStreamCreateWithFlags(&slot->st, cudaStreamNonBlocking));
+    else if (cudaStreamCreateWithFlags(&slot->st, cudaStreamNonBlocking) != cudaSuccess) {
+      slot->st = nullptr;
+      slot->mu.unlock();
+      wv_set_error("no stream for a staging slot: %s", cudaGetErrorString(cudaGetLastError()));
+      return WV_ECUDA;
+    }
   }
+  *out = slot;
+  return WV_OK;
+}
+
+extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int in, int out) {
+  int rc = ensure_init();
+  if (rc) return rc;
+  if (!x || !y) { wv_set_error("wv_matvec: null pointer"); return WV_EARG; }
+  Entry e;
+  if ((rc = lookup(key, &e))) return rc;
+  if ((rc = check_dims(e, batch, in, out))) return rc;
+  const size_t nx = (size_t)batch * in, ny = (size_t)batch * out;
+  StageSlot* slot = nullptr;
+  if ((rc = take_slot(batch, &slot))) return rc;
+  std::lock_guard<std::mutex> lk(slot->mu, std::adopt_lock);
   if (slot->hx_n < nx || slot->dx_n < nx || slot->hy_n < ny) slot->drop_graphs();   // the buffers are about to move
   if ((rc = grow_mapped(&slot->hx, &slot->hx_dev, &slot->hx_n, nx)) || (rc = grow(&slot->dx, &slot->dx_n, nx, false)) ||
       (rc = grow_mapped(&slot->hy, &slot->hy_dev, &slot->hy_n, ny))) return rc;
@@ -896,6 +911,69 @@ extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int 
   CUDA_TRY(cudaStreamSynchronize(slot->st));
   if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
   memcpy(y, slot->hy, ny * 4);
+  return WV_OK;
+}
+
+// ---------------------------------------------------------------- bias and activation behind the GEMV
+// core.ActivationType values (core/layer.go:91-98) and core.Activate (core/activate.go:6-38), in float64.
+enum WvActivation : int { WV_ACT_LINEAR = -1, WV_ACT_RELU = 0, WV_ACT_SILU, WV_ACT_GELU, WV_ACT_TANH, WV_ACT_SIGMOID, WV_ACT_LEAKY_RELU, WV_ACT_RELU2 };
+__device__ __forceinline__ double activate(double v, int act) {
+  switch (act) {
+  case WV_ACT_RELU: return v < 0.0 ? 0.0 : v;
+  case WV_ACT_RELU2: return v < 0.0 ? 0.0 : v * v;
+  case WV_ACT_LEAKY_RELU: return v < 0.0 ? 0.01 * v : v;
+  case WV_ACT_SILU: return v / (1.0 + exp(-v));
+  case WV_ACT_GELU: return 0.5 * v * (1.0 + tanh(0.79788456080286535588 * (v + 0.044715 * v * v * v)));      // sqrt(2 / pi)
+  case WV_ACT_TANH: return tanh(v);
+  case WV_ACT_SIGMOID: return 1.0 / (1.0 + exp(-v));
+  }
+  return v;
+}
+// A thread per output, bias[out] from device memory; both results go straight to mapped host memory. Bound by those stores: 0.9 MB
+// over a 50 GB/s host link are 18 us at 8 rows of 14336 outputs. On the host the same float64 passes took 0.45 of the call's 0.55 ms.
+__global__ void __launch_bounds__(256) bias_act_kernel(const float* __restrict__ y, const double* __restrict__ bias, int nbias, int act, float* __restrict__ pre,
+                                                       float* __restrict__ post, int out) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= out) return;
+  const size_t i = (size_t)blockIdx.y * out + c;
+  float p = y[i];
+  if (c < nbias) p = (float)((double)p + bias[c]);
+  pre[i] = p;
+  post[i] = (float)activate((double)p, act);
+}
+
+extern "C" int wv_matvec_bias_act(uint64_t key, const float* x, const double* bias, int nbias, int act, float* pre, float* post, int batch,
+                                  int in, int out) {
+  int rc = ensure_init();
+  if (rc) return rc;
+  if (!x || !pre || !post || nbias < 0 || (nbias && !bias)) { wv_set_error("wv_matvec_bias_act: bad argument"); return WV_EARG; }
+  if (act < WV_ACT_LINEAR || act > WV_ACT_RELU2) { wv_set_error("wv_matvec_bias_act: unknown activation %d", act); return WV_EARG; }
+  Entry e;
+  if ((rc = lookup(key, &e))) return rc;
+  if ((rc = check_dims(e, batch, in, out))) return rc;
+  if (nbias > out) nbias = out;
+  StageSlot* slot = nullptr;
+  if ((rc = take_slot(batch, &slot))) return rc;
+  std::lock_guard<std::mutex> lk(slot->mu, std::adopt_lock);
+  // x and the bias behind it in one pinned buffer, brought over together; W x stays on the device
+  const size_t nx = (size_t)batch * in, ny = (size_t)batch * out, xpad = (nx + 3) & ~(size_t)3, nin = xpad + 2 * (size_t)nbias;
+  const size_t npad = (nin + 3) & ~(size_t)3;
+  if ((rc = grow_mapped(&slot->ax, &slot->ax_dev, &slot->ax_n, npad)) || (rc = grow(&slot->da, &slot->da_n, npad + ny, false)) ||
+      (rc = grow_mapped(&slot->ay, &slot->ay_dev, &slot->ay_n, 2 * ny))) return rc;
+  memcpy(slot->ax, x, nx * 4);
+  if (nbias) memcpy(slot->ax + xpad, bias, (size_t)nbias * 8);
+  const int n4 = (int)(npad / 4);
+  const int blocks = n4 < 256 ? 1 : (n4 / 256 < 64 ? n4 / 256 : 64);
+  stage_in_kernel<<<blocks, 256, 0, slot->st>>>(reinterpret_cast<const float4*>(slot->ax_dev), reinterpret_cast<float4*>(slot->da), n4, nullptr, nullptr, 0);
+  rc = cudaGetLastError() == cudaSuccess ? wv_launch_gemv(e.blob, slot->da, slot->da + npad, batch, 0, e.blob.rows, slot->st) : WV_ECUDA;
+  if (!rc && launch_pdl(bias_act_kernel, dim3((out + 255) / 256, batch), dim3(256), 0, slot->st, slot->da + npad,
+                        reinterpret_cast<const double*>(slot->da + xpad), nbias, act, slot->ay_dev, slot->ay_dev + ny, out) != cudaSuccess) rc = WV_ECUDA;
+  if (rc) { wv_set_error("wv_matvec_bias_act: launch failed (%d): %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
+  CUDA_TRY(cudaStreamSynchronize(slot->st));
+  if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec_bias_act: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
+  memcpy(pre, slot->ay, ny * 4);
+  memcpy(post, slot->ay + ny, ny * 4);
   return WV_OK;
 }
 

@@ -113,12 +113,26 @@ def ForwardCUDA(l: Layer, input: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
     batch, in_, out = _dims(l, input)
     if l.Activation not in _ACTIVATIONS:
         raise WelvetError(_lib.WV_EARG, f"dense: unknown activation {l.Activation}")
+    bias = l.Weights.Bias
+    plain = l.Activation == ActivationLinear and (bias is None or len(bias) == 0)
     pre = np.empty((batch, out), input.dtype)
+    if input.dtype == np.float32 and l.Weights.Packed is not None and (plain or bias is None or np.ndim(bias) == 1):
+        # float32 in, float32 out: the results come straight into the arrays that are returned, bias and activation from the device
+        # (as passes over the batch here they took 0.45 of the 0.55 ms of 8 rows against 14336 x 4096)
+        key = quant.EnsureResident(l.Weights.Packed)
+        xs = np.ascontiguousarray(input.reshape(-1)[: batch * in_], np.float32)
+        if plain:
+            check(lib().wv_matvec(key, xs.ctypes.data, pre.ctypes.data, batch, in_, out))
+            return pre, pre
+        post = np.empty((batch, out), np.float32)
+        b = np.ascontiguousarray(bias, np.float64).reshape(-1) if bias is not None and len(bias) else None
+        check(lib().wv_matvec_bias_act(key, xs.ctypes.data, None if b is None else b.ctypes.data, 0 if b is None else b.size, l.Activation,
+                                       pre.ctypes.data, post.ctypes.data, batch, in_, out))
+        return pre, post
     y = np.empty(batch * out, np.float32)
     MatVecCUDA(l.Weights, np.asarray(input, np.float32), y, batch, in_, out)
     pre[...] = y.reshape(batch, out)
-    bias = l.Weights.Bias
-    if l.Activation == ActivationLinear and (bias is None or len(bias) == 0):
+    if plain:
         return pre, pre
     v = pre.astype(np.float64)
     if bias is not None and len(bias):
