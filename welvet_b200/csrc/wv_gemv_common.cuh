@@ -343,55 +343,54 @@ __device__ __forceinline__ float idot_chunk(const FragT<F>& f, const XQRegs& x) 
   return fmaf(mt.x, v, extra);
 }
 
-// ------------------------------------------------------------------ two-limb activations (16-bit)
-// The default arithmetic of the bulk-copy kernel: per 32-column chunk X_j = rint(x_j * 32512 / amax),
-// |X_j| <= 32512, split as X = L0 + 256 L1 with an unsigned low byte and a signed high byte, so a group
-// of four codes needs two dp4a instead of three and the limb sums always recombine in 32-bit integers
-// (255 * 32 * 32512 < 2^31). Per element |x_j - X_j sf| <= amax / 65024, sf = amax / 32512. A chunk
+// ------------------------------------------------------------------ 16-bit activations
+// The default arithmetic of the bulk-copy kernels: per 32-column chunk X_j = rint(x_j * 32512 / amax),
+// |X_j| <= 32512, two to a word, so a group of four codes needs two dp2a (16-bit times byte) and the sums
+// are whole in one accumulator (255 * 32 * 32512 < 2^31; as two byte limbs with dp4a they took a shift-add
+// more per sum). Per element |x_j - X_j sf| <= amax / 65024, sf = amax / 32512. A chunk
 // whose large values sit next to much smaller ones loses the small ones' low bits; the kernel decides
 // per launch, from the whole vector, whether that can matter (see gemv_tma_kernel) and takes the
 // three-limb path of quantize_chunk / idot_chunk when it can.
+__device__ __forceinline__ int dp2a_lo(unsigned x, unsigned codes, int c) {      // two signed 16-bit by the codes' bytes 0 and 1
+  int d;
+  asm("dp2a.lo.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(codes), "r"(c));
+  return d;
+}
+__device__ __forceinline__ int dp2a_hi(unsigned x, unsigned codes, int c) {      // by bytes 2 and 3
+  int d;
+  asm("dp2a.hi.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(codes), "r"(c));
+  return d;
+}
 struct XQRegs2 {
-  unsigned xw[16];   // word limb*8 + k
+  unsigned xw[16];   // word k: the activations of group k's codes 0 and 1, word 8 + k: of codes 2 and 3
   float4 mt;         // {sf, sf*SX(all), sf*SX(first 16), sf*SX(second 16)}
-  int iv[4];         // -mid*sum(limb l, half h) at l*2+h (halves pre-added for 32-wide groups)
+  int iv[2];         // -mid*SX of half h (the whole chunk's in iv[0] for 32-wide groups)
 };
 
-// xv: the chunk's 32 activations (already in registers), amax: their largest magnitude, bad: inf / NaN seen.
+// xv: the chunk's 32 activations (already in registers), amax: their largest magnitude, finite.
 template <int F>
-__device__ __forceinline__ void quantize_chunk2(XQRegs2& x, const float (&xv)[32], float amax, bool bad) {
+__device__ __forceinline__ void quantize_chunk2(XQRegs2& x, const float (&xv)[32], float amax) {
   constexpr WvFmtInfo fi = wv_fmt_info(F);
   constexpr int BL = fi.bits_lo;
   float sf = 0.f, inv = 0.f;
-  if (bad) sf = __uint_as_float(0x7fc00000u);          // inf / NaN in x: results become NaN
-  else if (amax >= 1.0e-30f) { sf = amax * (1.0f / 32512.0f); inv = 32512.0f / amax; }   // |x inv| <= 32512 (1 + 2^-23)
-  int sl[2][2] = {{0, 0}, {0, 0}};
+  if (amax >= 1.0e-30f) { sf = amax * (1.0f / 32512.0f); inv = 32512.0f / amax; }   // |x inv| <= 32512 (1 + 2^-23)
+  int sx[2] = {0, 0};
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     unsigned X[4];
-    // the low 23 bits of 1.5*2^23 + rint(v) hold rint(v) in two's complement (|v| < 2^22): bytes 0 and 1
-    // are the two limbs as they are, no subtraction needed
+    // the low 16 bits of 1.5*2^23 + rint(v) are rint(v) in two's complement
 #pragma unroll
     for (int m = 0; m < 4; m++) X[m] = __float_as_uint(fmaf(xv[WvLane<BL>::j_of(k, m)], inv, 12582912.0f));
-    const unsigned a01 = __byte_perm(X[0], X[1], 0x5140), a23 = __byte_perm(X[2], X[3], 0x5140);   // {b0,b0',b1,b1'}
-    const unsigned w0 = __byte_perm(a01, a23, 0x5410), w1 = __byte_perm(a01, a23, 0x7632);
-    x.xw[k] = w0; x.xw[8 + k] = w1;
+    x.xw[k] = __byte_perm(X[0], X[1], 0x5410);
+    x.xw[8 + k] = __byte_perm(X[2], X[3], 0x5410);
     const int hh = (BL == 1 || k < 4) ? 0 : 1;   // 1-bit planes split the halves by byte lane: everything in half 0
-    sl[0][hh] = dp4a_uu(w0, 0x01010101u, sl[0][hh]);
-    sl[1][hh] = dp4a_su(w1, 0x01010101u, sl[1][hh]);
+    sx[hh] = dp2a_lo(x.xw[k], 0x01010101u, dp2a_lo(x.xw[8 + k], 0x01010101u, sx[hh]));
   }
-  const int sx0 = sl[0][0] + (sl[1][0] << 8), sx1 = sl[0][1] + (sl[1][1] << 8);
-  x.mt = make_float4(sf, sf * (float)(sx0 + sx1), sf * (float)sx0, sf * (float)sx1);
-#pragma unroll
-  for (int i = 0; i < 4; i++) x.iv[i] = 0;
+  x.mt = make_float4(sf, sf * (float)(sx[0] + sx[1]), sf * (float)sx[0], sf * (float)sx[1]);
+  x.iv[0] = x.iv[1] = 0;
   if constexpr (QCfg<F>::INT_MID) {
-    if constexpr (QCfg<F>::HALVES) {
-#pragma unroll
-      for (int l = 0; l < 2; l++) { x.iv[l * 2] = -fi.mid * sl[l][0]; x.iv[l * 2 + 1] = -fi.mid * sl[l][1]; }
-    } else {
-#pragma unroll
-      for (int l = 0; l < 2; l++) x.iv[l * 2] = -fi.mid * (sl[l][0] + sl[l][1]);
-    }
+    if constexpr (QCfg<F>::HALVES) { x.iv[0] = -fi.mid * sx[0]; x.iv[1] = -fi.mid * sx[1]; }
+    else x.iv[0] = -fi.mid * (sx[0] + sx[1]);
   }
 }
 
@@ -404,9 +403,7 @@ __device__ __forceinline__ void idot_sums2(const FragT<F>& f, const XQRegs2& x, 
   constexpr unsigned MASKH = BH ? (0x01010101u * ((1u << BH) - 1u)) << BL : 0u;
   constexpr bool HALVES = QCfg<F>::HALVES;
   constexpr int NH = QCfg<F>::NH;
-  int I[2][2];
-#pragma unroll
-  for (int l = 0; l < 2; l++) { I[l][0] = x.iv[l * 2]; I[l][1] = HALVES ? x.iv[l * 2 + 1] : 0; }
+  int I[2] = {x.iv[0], HALVES ? x.iv[1] : 0};
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const int w = k / SPW, sh = k % SPW;
@@ -418,11 +415,11 @@ __device__ __forceinline__ void idot_sums2(const FragT<F>& f, const XQRegs2& x, 
       bytes |= hv & MASKH;
     }
     const int h = (HALVES && k >= 4) ? 1 : 0;
-    I[0][h] = dp4a_uu(bytes, x.xw[k], I[0][h]);
-    I[1][h] = dp4a_us(bytes, x.xw[8 + k], I[1][h]);
+    I[h] = dp2a_lo(x.xw[k], bytes, I[h]);
+    I[h] = dp2a_hi(x.xw[8 + k], bytes, I[h]);
   }
 #pragma unroll
-  for (int h = 0; h < NH; h++) val[h] = (float)(I[0][h] + (I[1][h] << 8));
+  for (int h = 0; h < NH; h++) val[h] = (float)I[h];
 }
 
 // Scale / min arithmetic shared by the two- and three-limb paths: val[h] = sum over half h of
@@ -467,9 +464,6 @@ __device__ __forceinline__ float idot_chunk2(const FragT<F>& f, const XQRegs2& x
   idot_sums2<F>(f, x, val);
   return idot_finish<F>(f, val, x.mt);
 }
-// One name for both activation widths (the kernel's main loop is instantiated once per width).
-template <int F> __device__ __forceinline__ float idot_any(const FragT<F>& f, const XQRegs& x) { return idot_chunk<F>(f, x); }
-template <int F> __device__ __forceinline__ float idot_any(const FragT<F>& f, const XQRegs2& x) { return idot_chunk2<F>(f, x); }
 
 // Launch with programmatic dependent launch allowed: the kernel may start while its
 // predecessor drains and must execute griddepcontrol.wait before touching dependent data.

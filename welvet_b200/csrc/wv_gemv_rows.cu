@@ -90,13 +90,15 @@ __device__ __forceinline__ void rows_prepare(RowsPrep<F>& p, const FragT<F>& f) 
   }
 }
 
-// The ROWS_RT chunk-rows' shares for one activation row, whose record r holds L limbs of 8 words, then {sf, sums}, then start values.
+// The ROWS_RT chunk-rows' shares for one activation row, whose record r holds L times 8 words, then {sf, sums}, then start values:
+// three byte limbs (L = 3), or 16-bit activations two to a word, whose sums need one accumulator (L = 2).
 template <int F, int L>
 __device__ __forceinline__ void rows_dot(const RowsPrep<F> (&p)[ROWS_RT], const uint4* r, int XS, float (&v)[ROWS_RT]) {
   constexpr WvFmtInfo fi = wv_fmt_info(F);
   constexpr bool HALVES = QCfg<F>::HALVES;
   constexpr int NH = QCfg<F>::NH;
-  int I[ROWS_RT][L][NH];
+  constexpr int NA = L == 3 ? 3 : 1;
+  int I[ROWS_RT][NA][NH];
   if constexpr (QCfg<F>::INT_MID) {           // -mid * sum of the limb, per half
     const uint4 i0 = r[(2 * L + 1) * XS];
     int iv[6] = {(int)i0.x, (int)i0.y, (int)i0.z, (int)i0.w, 0, 0};
@@ -104,14 +106,14 @@ __device__ __forceinline__ void rows_dot(const RowsPrep<F> (&p)[ROWS_RT], const 
 #pragma unroll
     for (int rr = 0; rr < ROWS_RT; rr++)
 #pragma unroll
-      for (int l = 0; l < L; l++)
+      for (int l = 0; l < NA; l++)
 #pragma unroll
         for (int h = 0; h < NH; h++) I[rr][l][h] = iv[l * 2 + h];
   } else {
 #pragma unroll
     for (int rr = 0; rr < ROWS_RT; rr++)
 #pragma unroll
-      for (int l = 0; l < L; l++)
+      for (int l = 0; l < NA; l++)
 #pragma unroll
         for (int h = 0; h < NH; h++) I[rr][l][h] = 0;
   }
@@ -126,7 +128,8 @@ __device__ __forceinline__ void rows_dot(const RowsPrep<F> (&p)[ROWS_RT], const 
       for (int k = 0; k < 4; k++)
 #pragma unroll
         for (int rr = 0; rr < ROWS_RT; rr++)
-          I[rr][l][h] = l == L - 1 ? dp4a_us(p[rr].by[4 * q + k], xw[k], I[rr][l][h]) : dp4a_uu(p[rr].by[4 * q + k], xw[k], I[rr][l][h]);
+          if constexpr (L == 2) I[rr][0][h] = l == 0 ? dp2a_lo(xw[k], p[rr].by[4 * q + k], I[rr][0][h]) : dp2a_hi(xw[k], p[rr].by[4 * q + k], I[rr][0][h]);
+          else I[rr][l][h] = l == L - 1 ? dp4a_us(p[rr].by[4 * q + k], xw[k], I[rr][l][h]) : dp4a_uu(p[rr].by[4 * q + k], xw[k], I[rr][l][h]);
     }
   const float4 mt = u4f(r[2 * L * XS]);       // {sf, sf SX, sf SX(first 16), sf SX(second 16)}
 #pragma unroll
@@ -135,8 +138,8 @@ __device__ __forceinline__ void rows_dot(const RowsPrep<F> (&p)[ROWS_RT], const 
 #pragma unroll
     for (int h = 0; h < NH; h++) {
       float val;
-      // two limbs, and three with codes of at most four bits, stay below 2^31
-      if constexpr (L == 2) val = (float)(I[rr][0][h] + (I[rr][1][h] << 8));
+      // 16-bit activations, and three limbs with codes of at most four bits, stay below 2^31
+      if constexpr (L == 2) val = (float)I[rr][0][h];
       else if constexpr (fi.bits_lo + fi.bits_hi <= 4) val = (float)(I[rr][0][h] + (I[rr][1][h] << 8) + (I[rr][2][h] << 16));
       else val = fmaf(65536.0f, (float)I[rr][2][h], (float)(I[rr][0][h] + (I[rr][1][h] << 8)));
       t = fmaf(p[rr].S[h], val, t);
@@ -265,14 +268,14 @@ gemv_rows_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restri
       r[8 * XS] = make_uint4((unsigned)q.iv[4], (unsigned)q.iv[5], 0u, 0u);
     } else {
       XQRegs2 q;
-      quantize_chunk2<F>(q, xv, amax, false);
+      quantize_chunk2<F>(q, xv, amax);
 #pragma unroll
       for (int l = 0; l < 2; l++) {
         r[(2 * l) * XS] = make_uint4(q.xw[8 * l], q.xw[8 * l + 1], q.xw[8 * l + 2], q.xw[8 * l + 3]);
         r[(2 * l + 1) * XS] = make_uint4(q.xw[8 * l + 4], q.xw[8 * l + 5], q.xw[8 * l + 6], q.xw[8 * l + 7]);
       }
       r[4 * XS] = f4u(q.mt);
-      r[5 * XS] = make_uint4((unsigned)q.iv[0], (unsigned)q.iv[1], (unsigned)q.iv[2], (unsigned)q.iv[3]);
+      r[5 * XS] = make_uint4((unsigned)q.iv[0], (unsigned)q.iv[1], 0u, 0u);
     }
   }
   // row groups without an activation row of their own load none

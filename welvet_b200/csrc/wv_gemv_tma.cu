@@ -24,6 +24,7 @@
 #include <mutex>
 #include <tuple>
 
+#define TMA_XPITCH 36   // floats per staged chunk of x: the 16-byte accesses of eight neighbouring chunks fall into different banks
 struct TmaGeom {
   int cpr;           // chunks per row
   int nwc;           // column warps per row (ceil(cpr/32))
@@ -36,7 +37,7 @@ struct TmaGeom {
   int rows_base, rows_rem;  // single matrix: CTA b owns rows_base (+1 if b < rows_rem) consecutive rows
   int lead;          // tiles issued before the producer waits for the activation loads to be on their way
   int force3;        // development switch: always use the 24-bit activation records
-  unsigned x_off;    // staged activations: 33 floats per chunk (32 + one of padding)
+  unsigned x_off;    // staged activations: TMA_XPITCH floats per chunk
   unsigned red_off;  // float red[2][nrg][nwc][32]
   unsigned gate_off; // gate | up launches: the gate's row sums of this CTA's band (TMA_GATE_ROWS floats)
   unsigned bar_off;  // full[nstage], empty[nstage]
@@ -257,9 +258,8 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
   __shared__ double s_norm[NORM ? TMA_CONSUMER_WARPS : 1];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // All consumer warps copy x into shared memory with coalesced loads; each chunk of 32
-  // floats gets a 33-float slot so that lanes reading their own chunks element by element
-  // hit 32 different banks. Every CTA starts its copy at a different place of x: all SMs
+  // All consumer warps copy x into shared memory with coalesced loads; a lane then reads its own chunk with 16-byte loads
+  // (element by element from 33-float slots the prologue issued some 70 instructions more per thread). Every CTA starts its copy at a different place of x: all SMs
   // asking for the same lines in the same order would queue up at one L2 slice after the other.
   // With column passes, pass cp brings in its own slice of x (after every warp is done with the previous one).
   const int npass = MP ? g.ncp : 1;
@@ -302,14 +302,14 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
         const int i0 = tid + u * TMA_CONSUMER_WARPS * 32;
         int i = i0 + rot;
         if (i >= nv) i -= nv;
-        if (i0 < nv) { float* d = xs + (i >> 3) * 33 + (i & 7) * 4; d[0] = v[u].x; d[1] = v[u].y; d[2] = v[u].z; d[3] = v[u].w; }
+        if (i0 < nv) *reinterpret_cast<float4*>(xs + (i >> 3) * TMA_XPITCH + (i & 7) * 4) = v[u];
       }
     } else {
       if (lane == 0) asm volatile("red.relaxed.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(&s_xissued)) : "memory");
       double ss = 0.0;
       for (int i = tid; i < g.cpr * 32; i += TMA_CONSUMER_WARPS * 32) {
         const float xv1 = __ldg(xrow + i);
-        xs[(i >> 5) * 33 + (i & 31)] = xv1;
+        xs[(i >> 5) * TMA_XPITCH + (i & 31)] = xv1;
         if constexpr (NORM) ss += (double)xv1 * (double)xv1;
       }
       if constexpr (NORM) {
@@ -389,7 +389,7 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
   int fs = 0;
   unsigned fpar = 0;
   auto wait_tile = [&](bool block) -> bool {
-    if (dead || *(volatile int*)&s_abort) { dead = true; return true; }
+    if (dead) return true;
     if (!block) {
       unsigned ok;
       asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -494,7 +494,11 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     }
   };
 
-  const float* xc = reinterpret_cast<const float*>(smem + g.x_off) + (size_t)(live ? c : 0) * 33;
+  float4* xc = reinterpret_cast<float4*>(smem + g.x_off) + (size_t)(live ? c : 0) * (TMA_XPITCH / 4);
+  auto chunk_x = [&](float (&xv)[32]) {      // this lane's chunk
+#pragma unroll
+    for (int q = 0; q < 8; q++) { const float4 t = xc[q]; xv[4 * q] = t.x; xv[4 * q + 1] = t.y; xv[4 * q + 2] = t.z; xv[4 * q + 3] = t.w; }
+  };
   for (cp = 0; cp < npass; cp++) {
   copy_x();
   if constexpr (NORM) {
@@ -505,12 +509,11 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     // every chunk is normalised in place by the one lane of row group 0 that owns it; the other row groups' warps
     // read it after the barrier (all warps that have a row group take part; the others have left)
     if (rg == 0 && live) {
-      float* xw = reinterpret_cast<float*>(smem + g.x_off) + (size_t)c * 33;
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        const float gq[4] = {gam[k].x, gam[k].y, gam[k].z, gam[k].w};
-#pragma unroll
-        for (int m = 0; m < 4; m++) xw[4 * k + m] = (xw[4 * k + m] * inv) * gq[m];
+        float4 t = xc[k];
+        t.x = (t.x * inv) * gam[k].x; t.y = (t.y * inv) * gam[k].y; t.z = (t.z * inv) * gam[k].z; t.w = (t.w * inv) * gam[k].w;
+        xc[k] = t;
       }
     }
     asm volatile("bar.sync 14, %0;" ::"r"(nactive * 32) : "memory");
@@ -523,12 +526,14 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
 #pragma unroll
     for (int k = 0; k < 8; k++) xfr[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (live) {
+      float xv[32];
+      chunk_x(xv);
 #pragma unroll
       for (int w = 0; w < 4; w++)
 #pragma unroll
         for (int h = 0; h < 2; h++)
-          xfr[2 * w + h] = make_float4(xc[WvLane<BL>::j_of(2 * w, 2 * h)], xc[WvLane<BL>::j_of(2 * w + 1, 2 * h)],
-                                       xc[WvLane<BL>::j_of(2 * w, 2 * h + 1)], xc[WvLane<BL>::j_of(2 * w + 1, 2 * h + 1)]);
+          xfr[2 * w + h] = make_float4(xv[WvLane<BL>::j_of(2 * w, 2 * h)], xv[WvLane<BL>::j_of(2 * w + 1, 2 * h)],
+                                       xv[WvLane<BL>::j_of(2 * w, 2 * h + 1)], xv[WvLane<BL>::j_of(2 * w + 1, 2 * h + 1)]);
     }
     const unsigned lane4 = (unsigned)lane * 8u;
     main_loop([&](const FragT<F>& f) { return chunk_value_tbl<F>(f, xfr, tbl, lane4); });
@@ -543,8 +548,7 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     // records, whose error is 2^-9 of that. Weights that sit exactly on the small elements of outlier chunks can
     // exceed either bound: no criterion on x alone excludes that.
     float xv[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) xv[j] = xc[j];
+    chunk_x(xv);
     float am[4] = {0.f, 0.f, 0.f, 0.f}, as[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < 32; j++) { const float a = fabsf(xv[j]); am[j & 3] = fmaxf(am[j & 3], a); as[j & 3] += a; }
@@ -559,7 +563,7 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     if (!wide) {
       XQRegs2 xr;
       if (live) {
-        quantize_chunk2<F>(xr, xv, amax, false);
+        quantize_chunk2<F>(xr, xv, amax);
         if constexpr (BL == 8) {
           const bool sw = lane & 4;
 #pragma unroll
@@ -576,14 +580,13 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
 #pragma unroll
         for (int t = 0; t < 16; t++) xr.xw[t] = 0u;
         xr.mt = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 4; i++) xr.iv[i] = 0;
+        xr.iv[0] = xr.iv[1] = 0;
       }
       main_loop([&](const FragT<F>& f) { return idot_chunk2<F>(f, xr); });
     } else {
       XQRegs xr;
       if (live) {
-        quantize_chunk<F>(xr, xc);
+        quantize_chunk<F>(xr, xv);
         if constexpr (BL == 8) {
           const bool sw = lane & 4;
 #pragma unroll
@@ -691,7 +694,7 @@ static int launch_tma(const WvDevBlob* bl, int nb, const float* dx, float* const
   unsigned off = 0;
   for (int i = 0; i < 5; i++) { g.off[i] = off; off = align128(off + g.rb[i] * g.tr); }
   g.stage_bytes = off;
-  const unsigned xbytes = align128((unsigned)g.cpr * 132u);
+  const unsigned xbytes = align128((unsigned)g.cpr * TMA_XPITCH * 4u);
   const WvFuse* fuse = wv_cur_fuse;
   const bool gated = fuse && fuse->mode == 1;
   const unsigned gate_bytes = gated ? TMA_GATE_ROWS * 4u : 0u;
