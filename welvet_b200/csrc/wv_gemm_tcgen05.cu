@@ -7,20 +7,19 @@
 // 32-column slice. The 512 producer threads form four groups of 128 (a thread per row); each group owns a run of
 // consecutive columns and the groups' slices go through the pipeline in turn, so that a thread reads its row 128 bits to
 // 64 bytes at a time although every slice is one chunk wide (the order in which slices are summed is free as long as X
-// takes the same one). A thread dequantises a 32-weight chunk to TF32 values in the canonical K-major 128-byte-swizzled
-// operand layout; one thread copies the matching slice of X (rounded to TF32 by a kernel in front) beside it, one elected
-// thread issues four tcgen05.mma (M 128, N = batch padded to 16, K 8) per slice into a TMEM accumulator, and
-// tcgen05.commit hands the stage back. At the end all producer warps read the accumulator with tcgen05.ld; the splits of
-// a row tile are one thread-block cluster, which adds its accumulators up in split order through distributed shared
-// memory.
+// takes the same one). A thread dequantises a 32-weight chunk to TF32 values and stores them to tensor memory, where a row is
+// a lane and a value a column (the MMA's A operand); one thread copies the matching slice of X (rounded to TF32 by a kernel in
+// front) to shared memory, one elected thread issues four tcgen05.mma (M 128, N = batch padded to 16, K 8) per slice into a
+// TMEM accumulator, and tcgen05.commit hands the stage back. At the end all producer warps read the accumulator with
+// tcgen05.ld; the splits of a row tile are one thread-block cluster, which adds its accumulators up in split order through
+// distributed shared memory.
 //
-// Bound: up to some 64 rows the latency of the producers' loads and instructions (eight executed per weight, all roles together)
-// and of the MMAs, which take about 52 cycles each however few rows X has; at 256 rows the tensor pipe (70 % of active cycles) and
-// the copies of X out of L2 (every row tile reads all of it). Measured against the version before (512 producers of 8 weights
-// each, two slices a stage, issue loops run by one lane, split sums through global memory), 16 / 64 / 256 rows, six matrices in
-// turn and one Y: Q8_0 4096 x 4096 21.7 / 28.3 / 56.9 -> 15.7 / 17.9 / 25.9 us, Q4_K 14336 x 4096 66.2 / 67.6 / 82.0 -> 36.6 /
-// 41.1 / 54.0 us (256 rows with a Y of 14.7 MB for each of four matrices: 83 -> 60.5), Q4_0 1024 x 1024 12.0 / 18.2 / 42.6 ->
-// 8.2 / 9.5 / 16.1 us. With the loads and the conversion left out the 14336 x 4096 launch takes 15.5 us at 16 rows.
+// Bound: the latency and the instructions of the producers (0.7 to 1 us for the four groups' slices of a round), at 256 rows the
+// tensor pipe as well. With W's slices in tensor memory instead of shared memory a chunk takes two stores instead of eight and no
+// proxy fence, and shared memory holds X alone: the rest is L1, where the second half of every 128-byte line of W waits for the
+// next unit (forcing the whole carve-out on the same code: Q8_0, 33 rows, 4096 x 4096 13.8 -> 17.2 us). us per launch, slices of
+// W in shared memory and sums of one row of W at a time / now: Q8_0 4096 x 4096, 33 rows 16.7 / 13.7; Q8_0 14336 x 4096, 8 rows
+// 39.1 / 30.4; Q4_K 4096 x 4096, 128 and 256 rows 18.7 / 16.0 and 24.7 / 22.1; Q4_K 14336 x 4096, 256 rows 55.6 / 47.9.
 //
 // Arithmetic: X is rounded to TF32 (round to nearest, 11 significant bits) with its low bits cleared, a weight by adding half a
 // unit of the eleventh bit to it, the rest being the tensor core's truncation, which reads an operand's upper 19 bits only;
@@ -249,11 +248,18 @@ __device__ __forceinline__ void tcg_fence_after() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ unsigned long long tcg_desc(unsigned saddr) {
   return (unsigned long long)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((unsigned long long)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void tcg_mma_tf32(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned accumulate) {
+// A in tensor memory (lane = row, a column per TF32 value), B in shared memory.
+__device__ __forceinline__ void tcg_mma_tf32(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc, unsigned accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tcg_st16(unsigned taddr, const float (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]),
+        "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
 }
 __device__ __forceinline__ void tcg_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -276,8 +282,7 @@ struct TcgGeom {
   int batch, npad;            // activation rows, and that padded to a multiple of 16 (the MMA's N)
   int ksplit, cps;            // column splits (= cluster size) and chunks per split
   int rounds;                 // rounds of TCG_GROUPS stages in the ring: 2, or 1 where the activations leave no room
-  unsigned b_bytes, stage_bytes;            // a stage: one slice of A (128 rows x 128 bytes), then one of B (npad x 128 bytes)
-  unsigned tmem_cols;         // power of two >= max(32, npad)
+  unsigned b_bytes;           // a stage in shared memory: a slice of X, npad x 128 bytes
   int y_stride;               // floats between consecutive activation rows' outputs
 #ifdef WV_DEV_HOOKS
   int stall;                  // > 0: the first producer warp stops short of this slice, so that a wait runs out
@@ -290,7 +295,10 @@ struct TcgGeom {
 #define TCG_SPIN TMA_SPIN_LIMIT
 #endif
 
-#define TCG_A_BYTES (TCG_M * 128u)
+// Tensor memory: all 512 columns, the accumulator in the first 256, then a stage's slice of A in 32 columns each.
+#define TCG_TMEM 512
+#define TCG_TMEM_A 256
+static_assert(TCG_TMEM_A + 32 * TCG_MAX_STAGES <= TCG_TMEM, "stages of A");
 
 __device__ __forceinline__ bool elect_one() {
   unsigned p;
@@ -299,11 +307,11 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ld_cluster(unsigned saddr, int rank) {
+__device__ __forceinline__ float4 ld_cluster4(unsigned saddr, int rank) {
   unsigned a;
-  float v;
+  float4 v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
 
@@ -328,20 +336,29 @@ struct TcgOrder {
   }
 };
 
-// The sums of the activation rows that CTA sp of the cluster stores, over the splits' accumulators in split order. One loop for up
-// to eight splits and one for more: a loop that looks after both took 8 % longer at 64 x 512 with 256 rows (two splits).
+// The sums of the activation rows that CTA sp of the cluster stores, over the splits' accumulators in split order: four rows of W a
+// thread, the loads from all CTAs in flight together. It is bound by their latency (some 0.5 us a turn of the loop): one row of
+// W at a time, 256 rows took 7.2 of the 27 us of a 4096 x 4096 launch in Q4_K. One loop for up to eight splits and one for more.
 template <int N>
 __device__ __forceinline__ void tcg_add_splits(const TcgGeom& g, unsigned acc_s, float* __restrict__ y, int sp, int m0) {
   for (int e = threadIdx.x; ; e += TCG_THREADS) {
-    const int m = (e / TCG_M) * g.ksplit + sp, row_l = e & (TCG_M - 1);
+    const int m = (e / (TCG_M / 4)) * g.ksplit + sp, row_l = (e & (TCG_M / 4 - 1)) * 4;
     if (m >= g.batch) break;
-    float v[N];
+    float4 v[N];
 #pragma unroll
-    for (int u = 0; u < N; u++) if (u < g.ksplit) v[u] = ld_cluster(acc_s + 4u * (unsigned)(m * TCG_M + row_l), u);
-    float sum = 0.f;
+    for (int u = 0; u < N; u++) if (u < g.ksplit) v[u] = ld_cluster4(acc_s + 4u * (unsigned)(m * TCG_M + row_l), u);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < N; u++) if (u < g.ksplit) sum += v[u];
-    if (m0 + row_l < g.row_end) y[(size_t)m * g.y_stride + m0 + row_l] = sum;
+    for (int u = 0; u < N; u++) if (u < g.ksplit) { sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w; }
+    float* o = y + (size_t)m * g.y_stride + m0 + row_l;
+    const int left = g.row_end - m0 - row_l;
+    if (left >= 4 && (reinterpret_cast<uintptr_t>(o) & 15) == 0) *reinterpret_cast<float4*>(o) = sum;
+    else {
+      if (left > 0) o[0] = sum.x;
+      if (left > 1) o[1] = sum.y;
+      if (left > 2) o[2] = sum.z;
+      if (left > 3) o[3] = sum.w;
+    }
   }
 }
 
@@ -379,7 +396,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   }
   if (wv_fmt_info(F).table && tid < 16) s_tbl[tid] = c_grid4nl[tid];
   if (warp == TCG_PRODUCERS / 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(g.tmem_cols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "n"(TCG_TMEM) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcg_fence_before();
@@ -399,9 +416,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
     const int row = min(m0 + row_l, g.row_end - 1);              // rows past the end repeat the last one and are not stored
     const int mine = order.n[0] * (grp == 0) + order.n[1] * (grp == 1) + order.n[2] * (grp == 2) + order.n[3] * (grp == 3);
     const long long ch0 = (long long)row * g.cpr + kc0 + order.first[0] * (grp == 0) + order.first[1] * (grp == 1) + order.first[2] * (grp == 2) + order.first[3] * (grp == 3);
-    // this thread's part of the A slice: row row_l, its 16-byte pieces swizzled by the row; eight lanes of a store phase
-    // have eight different rows mod 8 and so cover all banks
-    const unsigned a_off = (unsigned)(row_l >> 3) * 1024u + (unsigned)(row_l & 7) * (128u + 16u);
+    const unsigned a_t = tmem + ((unsigned)((warp & 3) * 32) << 16) + TCG_TMEM_A;      // this warp's rows of the A slices
     // one unit ahead: its loads travel while the current unit is converted
     FragT<F> nxt[U];
     if (mine > 0) tcg_load<F, VEC>(nxt, b, ch0, mine);
@@ -423,12 +438,15 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         const int s = stage_of(i, grp), use = i >> rsh;
         if (!bad && use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1, TCG_SPIN)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
         if (__any_sync(0xffffffffu, bad)) { dead = true; break; }     // the whole warp leaves together (it meets at __syncwarp below)
-        const unsigned st = sbase + (unsigned)s * g.stage_bytes + a_off;
-        tcg_convert<F>(cur[u], s_tbl, [&](int p, const float (&v)[4]) {
-          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(st ^ (16u * p)), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+        tcg_fence_after();                    // the MMAs that read this stage before have been waited for
+        float a[16];
+        tcg_convert<F>(cur[u], s_tbl, [&](int p, const float (&v)[4]) {      // pieces come in rising order
+#pragma unroll
+          for (int e = 0; e < 4; e++) a[4 * (p & 3) + e] = v[e];
+          if ((p & 3) == 3) tcg_st16(a_t + (unsigned)(s * 32 + (p >> 2) * 16), a);
         });
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tcg_fence_before();
         if (lane == 0) mbar_arrive(full_bar(s));      // one arrival per warp
         made = i + 1;
       }
@@ -454,7 +472,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         if (use > 0 && __any_sync(0xffffffffu, !mbar_wait(empty_bar(s), (use - 1) & 1, TCG_SPIN))) { atomicCAS_system(err, 0, 530 + s); *(volatile int*)&s_abort = 1; run = false; break; }
         if (leader) {
           mbar_expect_tx(full_bar(s), g.b_bytes);
-          tma_load_2d(sbase + (unsigned)s * g.stage_bytes + TCG_A_BYTES, &xmap, (kc0 + order.first[q] + i) * 32, 0, full_bar(s));
+          tma_load_2d(sbase + (unsigned)s * g.b_bytes, &xmap, (kc0 + order.first[q] + i) * 32, 0, full_bar(s));
         }
         __syncwarp();
         copied_q = q + 1;
@@ -474,11 +492,10 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         if (__any_sync(0xffffffffu, !mbar_wait(full_bar(s), (i >> rsh) & 1, TCG_SPIN))) { atomicCAS_system(err, 0, 510 + s); *(volatile int*)&s_abort = 1; run = false; break; }
         tcg_fence_after();
         if (leader) {
-          const unsigned st = sbase + (unsigned)s * g.stage_bytes;
-          const unsigned long long da = tcg_desc(st), db = tcg_desc(st + TCG_A_BYTES);
+          const unsigned long long db = tcg_desc(sbase + (unsigned)s * g.b_bytes);
 #pragma unroll
-          for (int k = 0; k < 4; k++)   // 8 TF32 values = 32 bytes further along K inside the swizzled row
-            tcg_mma_tf32(tmem, da + (unsigned long long)(2 * k), db + (unsigned long long)(2 * k), idesc, (i > 0 || q > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < 4; k++)   // 8 TF32 values = 8 columns of A, 32 bytes further along K inside X's swizzled row
+            tcg_mma_tf32(tmem, tmem + (unsigned)(TCG_TMEM_A + 32 * s + 8 * k), db + (unsigned long long)(2 * k), idesc, (i > 0 || q > 0 || k > 0) ? 1u : 0u);
           tcg_commit(empty_bar(s));        // arrives when these MMAs have read the stage
         }
         __syncwarp();
@@ -506,12 +523,18 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = 0.f;
       }
+      if (g.ksplit > 1) {                          // rows past the batch as well: the ring has npad * 512 bytes and more
 #pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const int m = c0 + j;
-        if (m < g.batch) {
-          if (g.ksplit == 1) { if (row_ok) y[(size_t)m * g.y_stride + m0 + row_l] = v[j]; }
-          else acc[m * TCG_M + row_l] = v[j];
+        for (int j = 0; j < 16; j++) acc[(c0 + j) * TCG_M + row_l] = v[j];
+      } else if (row_ok) {
+        float* o = y + (size_t)c0 * g.y_stride + m0 + row_l;
+        const int left = g.batch - c0;
+        if (left >= 16) {                          // whole: no test per row
+#pragma unroll
+          for (int j = 0; j < 16; j++) o[(size_t)j * g.y_stride] = v[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; j++) if (j < left) o[(size_t)j * g.y_stride] = v[j];
         }
       }
     }
@@ -538,7 +561,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   }
   if (warp == TCG_PRODUCERS / 32) {
     tcg_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(g.tmem_cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TCG_TMEM) : "memory");
   }
   if (g.ksplit == 1) return;
   // ---------------------------------------------------------------- the cluster adds its accumulators up in split order: CTA sp
@@ -742,14 +765,11 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
   g.cps = tcg_cps(g.cpr, ks, unit);
   g.ksplit = ks;
   g.b_bytes = (unsigned)g.npad * 128u;
-  g.stage_bytes = TCG_A_BYTES + g.b_bytes;
-  g.rounds = TCG_MAX_STAGES * g.stage_bytes <= 200u * 1024u ? 2 : 1;      // two up to 64 rows; one round of 256 rows takes 192 KB
+  g.rounds = TCG_MAX_STAGES * g.b_bytes <= 200u * 1024u ? 2 : 1;      // two up to 192 rows
 #ifdef WV_DEV_HOOKS
   g.stall = g_tcg_stall; g.spin = g_tcg_spin;
 #endif
-  g.tmem_cols = 32;
-  while ((int)g.tmem_cols < g.npad) g.tmem_cols *= 2;
-  const size_t smem = (size_t)g.rounds * TCG_GROUPS * g.stage_bytes + 1024;
+  const size_t smem = (size_t)g.rounds * TCG_GROUPS * g.b_bytes + 1024;
   // X rounded to TF32 once, by a small kernel in front (each of the row tiles would otherwise round it again), into a
   // buffer of the library; the main kernel fetches it through a tensor map encoded per call.
   TcgLease lease;
