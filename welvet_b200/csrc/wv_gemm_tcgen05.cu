@@ -403,8 +403,8 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   __syncthreads();
   tcg_fence_after();
   const unsigned tmem = __shfl_sync(0xffffffffu, *(volatile unsigned*)&s_tmem, 0);
-  // The weights do not depend on the preceding kernel: the producers start at once. Only the thread that copies X waits
-  // for it (X was rounded by the kernel right before this one), and nothing is stored before X has arrived.
+  // The weights do not depend on the preceding kernel: the producers start at once, up to a full ring. Only then do they, and from
+  // the start the warps that copy X and issue the MMAs, wait for it (X was rounded by the kernel right before this one).
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   int copied_i = 0, copied_q = 0;                // copying warp: the round it reached, and the groups it served in that round
@@ -431,6 +431,8 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
       for (int u = 0; u < U; u++) {
         const int i = i0 + u;
         if (i >= mine || dead) break;
+        // From here on a stage is free only after X has come; however long the kernels before take, that is not a time-out.
+        if (i == g.rounds) asm volatile("griddepcontrol.wait;" ::: "memory");
 #ifdef WV_DEV_HOOKS
         if (g.stall > 0 && warp == 0 && i + 1 >= g.stall) { dead = true; break; }
 #endif
@@ -452,6 +454,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
       }
     }
     if (lane == 0) s_made[warp] = made;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
   } else if (warp == TCG_PRODUCERS / 32 + 1) {
     // ------------------------------------------------------------ X copies: a stage's slice of the rounded activations arrives
     // by a tensor-map copy with the 128-byte swizzle, i.e. already in the operand layout; rows past the batch are zero-filled
@@ -483,6 +486,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
     const bool leader = elect_one();
     const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(g.npad >> 3) << 17) | ((unsigned)(TCG_M >> 4) << 24);
     bool run = true;
+    asm volatile("griddepcontrol.wait;" ::: "memory");           // X comes after it
     for (int i = 0; i < order.n[0] && run; i++) {
       const int na = order.active(i);
 #pragma unroll
@@ -577,10 +581,13 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
   cluster_wait();
 }
 
-// X rounded to TF32 (round to nearest), element for element.
+// X rounded to TF32 (round to nearest), element for element. The kernel behind it may start as soon as this one has (it waits for
+// this one's end before it reads X): its set-up and its first slices of W then run beside the preceding kernel's end and this one.
+// us per launch, started after this kernel's own wait / before it: Q8_0 4096 x 4096, 33 rows 13.7 / 12.5; Q5_1 1024 x 1024, 64 rows
+// 8.1 / 7.0; Q8_0 14336 x 4096, 8 rows 30.4 / 28.6; at 256 rows the copy itself counts (22.1 / 21.8, with more blocks 21.6).
 __global__ void __launch_bounds__(256) tcg_round_x_kernel(const float4* __restrict__ x, float4* __restrict__ xr, size_t n4) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
     const float4 v = x[i];
     xr[i] = make_float4(tcg_tf32(v.x), tcg_tf32(v.y), tcg_tf32(v.z), tcg_tf32(v.w));
@@ -798,7 +805,11 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
     const size_t n4 = (size_t)batch * b.cols / 4;
     cudaLaunchConfig_t rc_ = {};
     int blocks = (int)((n4 + 255) / 256);
-    if (blocks > 2 * 148) blocks = 2 * 148;
+    // Two blocks fit beside a CTA of the kernel before. Up to three turns of those they are all resident early; beyond, the copy is
+    // what counts (100 rows of 6400 columns 16.0 us a call with 296 blocks, 16.2 with all; 256 of 4096 21.8 and 21.6).
+    const int beside = 2 * 148, all = 8 * 148;
+    if (blocks > 3 * beside) { if (blocks > all) blocks = all; }
+    else if (blocks > beside) blocks = beside;
     rc_.gridDim = dim3(blocks); rc_.blockDim = dim3(256); rc_.stream = st;
     rc_.attrs = at; rc_.numAttrs = 1;
     if (cudaLaunchKernelEx(&rc_, tcg_round_x_kernel, reinterpret_cast<const float4*>(dx), reinterpret_cast<float4*>(xr), n4) != cudaSuccess) {

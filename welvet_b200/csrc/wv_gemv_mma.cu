@@ -206,9 +206,11 @@ gemv_mma_kernel(const WvDevBlob b, const float* __restrict__ xf, float* __restri
     const CUtensorMap* tm[4] = {&tm_lo, &tm_hi, &tm_p0, &tm_p1};
     int ps = 0, issued = 0;
     unsigned ppar = 1;
-    bool wrapped = false, dead = false;
+    bool wrapped = false, dead = false, gated = false;
     auto issue_tile = [&](int mt, int seg) {   // lane 0 only
       if (wrapped) {
+        // a full ring: the consumers wait for the preceding kernel, which is no time-out however long it takes
+        if (!gated) { asm volatile("griddepcontrol.wait;" ::: "memory"); gated = true; }
         if (*(volatile int*)&s_abort || !mbar_wait(empty_bar(ps), ppar)) {
           if (!*(volatile int*)&s_abort) { atomicCAS_system(err, 0, 400 + ps); *(volatile int*)&s_abort = 1; }
           dead = true;

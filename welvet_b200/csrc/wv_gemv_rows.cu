@@ -192,6 +192,7 @@ gemv_rows_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restri
         if (t == 1) for (unsigned i = 0; i < TMA_SPIN_LIMIT; i++) if (*(volatile unsigned*)&s_xissued >= (unsigned)nactive) break;
         if (t >= g.nstage) {
           if (*(volatile int*)&s_abort) break;
+          if (t == g.nstage) asm volatile("griddepcontrol.wait;" ::: "memory");      // the consumers do: no time-out however long it takes
           if (!mbar_wait(empty_bar(s), par)) { atomicCAS_system(err, 0, 600 + s); *(volatile int*)&s_abort = 1; break; }
         }
         const int r0 = t * g.tr, nr = min(g.tr, band - r0);

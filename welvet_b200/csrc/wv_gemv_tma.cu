@@ -134,12 +134,14 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     int issued = 0;        // tiles issued so far, over all matrices
     int ps = 0;            // stage of the tile being issued
     unsigned ppar = 1;     // parity of the "empty" phase to wait for once the ring has wrapped
-    bool wrapped = false;
+    bool wrapped = false, gated = false;
     int bi = 0;            // matrix being streamed
     int pcp = 0;           // column pass being streamed
     auto issue_tile = [&](int t) {
       const int s = ps;
       if (wrapped) {
+        // a full ring: the consumers wait for the preceding kernel, which is no time-out however long it takes
+        if (!gated) { asm volatile("griddepcontrol.wait;" ::: "memory"); gated = true; }
         if (*(volatile int*)&s_abort || !mbar_wait(empty_bar(s), ppar)) {
           if (!*(volatile int*)&s_abort) { atomicCAS_system(err, 0, 100 + s); *(volatile int*)&s_abort = 1; }
           dead = true;
@@ -183,6 +185,7 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
                 if (*(volatile unsigned*)&s_xissued >= TMA_CONSUMER_WARPS) break;
               }
             }
+            if (wrapped && !gated) { asm volatile("griddepcontrol.wait;" ::: "memory"); gated = true; }
             if (wrapped && (*(volatile int*)&s_abort || !mbar_wait(empty_bar(s), ppar))) {
               if (!*(volatile int*)&s_abort) { atomicCAS_system(err, 0, 100 + s); *(volatile int*)&s_abort = 1; }
               ok = 0;
