@@ -221,3 +221,35 @@ def test_concurrent_host_callers(wv):
     for j in range(len(jobs)):
         for k in range(20):
             assert np.array_equal(out[j][k].view(np.uint32), want[j].view(np.uint32))
+
+
+@pytest.mark.parametrize("dt,rows,cols,batch", [(1, 1, 1024, 1), (1, 149, 1032, 1), (1, 296, 5000, 1), (1, 700, 8192, 2), (1, 2400, 1024, 1), (1, 33, 8200, 1), (1, 9, 1016, 1),
+                                                (2, 7, 2048, 1), (2, 148, 2056, 3), (2, 2368, 4104, 1), (2, 2369, 2048, 1), (2, 1500, 2048, 2), (3, 301, 8192, 1), (3, 60, 5000, 5)])
+def test_plain_rows_at_the_limits_of_the_ring_kernel(wv, dt, rows, cols, batch):
+    """FormatNone rows at the edges of the ring kernel's range (row bytes, columns, slices that do not divide the row, rows of W above
+    and below its limit, several rows of x, x that is not 16-byte aligned) against float64: float32 products and sums, so at most
+    cols + 8 roundings of 2^-24 of sum |w x|, of which random signs leave a fraction; the bound is 64 of them."""
+    import torch
+    from welvet_b200 import _lib
+    L, key = _lib.lib(), 0x7000 + rows * 16 + dt
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    w = torch.randn(rows * cols, device="cuda", generator=gen) * 0.02
+    torch.cuda.synchronize()
+    _lib.check(L.wv_pack_upload_dev(key, 0, dt, 0, w.data_ptr(), rows, cols, None))
+    d = torch.zeros(rows, cols, device="cuda")
+    _lib.check(L.wv_unpack_dev(key, d.data_ptr(), None))
+    buf = torch.randn(batch * cols + 1, device="cuda", generator=gen)
+    torch.cuda.synchronize()
+    try:
+        for off in (0, 1):
+            x = buf[off : off + batch * cols]
+            y = torch.full((batch, rows), float("nan"), device="cuda")
+            torch.cuda.synchronize()
+            _lib.check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, rows, None))
+            torch.cuda.synchronize()
+            xd = x.reshape(batch, cols).double()
+            err = (y.double() - xd @ d.double().T).abs()
+            assert bool((err <= 64 * 2.0 ** -24 * (xd.abs() @ d.double().abs().T)).all())
+        assert L.wv_device_status() == 0
+    finally:
+        L.wv_blob_evict(key)

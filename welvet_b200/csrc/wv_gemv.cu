@@ -14,6 +14,7 @@
 //     reference's own factorisation sc*sum(q*x) + mn*sum(x) (simd/dot_k.go:44-53);
 //   * warp-shuffle reduction, one store per row.
 #include "wv_gemv_common.cuh"
+#include "wv_tma_common.cuh"
 #include "wv_dev_hooks.h"
 #include <cooperative_groups.h>
 #include <stdlib.h>
@@ -395,6 +396,111 @@ gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restr
   }
 }
 
+// ------------------------------------------------------------------ FormatNone through a shared-memory ring
+// The same product for few rows of 4 to 32 KB. Bound: latency. The kernel above gives a warp whole rows, with two steps of 2 KB in
+// flight, so that few rows leave most of its warps without work. Here S of a CTA's sixteen warps share a row: a warp's slice of
+// the columns is fixed, so its part of x stays in registers, and a ring of its own brings in the slice of one row after the
+// other (lane 0 requests, before the wait for the preceding kernel what the ring holds; the warp reads: nothing to wait for but
+// its own copies; slices of some 2 KB, since a copy costs about 45 ns whatever its size). The slices' sums of a band meet in
+// shared memory at the end. Two CTAs fill an SM: with one for each SM, two of them went to the SMs that the preceding kernel left
+// first and others stayed empty (a 4096 x 4096 f32 launch behind one of Q4_K: 30 us instead of 13).
+// us per launch, the kernel above / this one: f32 512 x 8192 11.5 / 4.0, 2368 x 2048 6.1 / 4.7; f16 1000 x 8192 8.3 / 4.7, 1500 x 3000
+// 4.8 / 3.8, 2000 x 2048 3.7 / 3.6.
+#define RING_WARPS 16
+#define RING_SLOTS 16
+struct RingGeom { int vpr, vw, s, nslot; unsigned slot_bytes, red_off; int rows_base, rows_rem; };      // vectors per row and slice, slices per row, slots per warp
+template <int DT, int NV>      // NV: 16-byte vectors of a slice per lane at most
+__global__ void __launch_bounds__(RING_WARPS * 32, 2)
+gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float* __restrict__ y, int rows, int cols, int row_begin, const RingGeom g, int* __restrict__ err) {
+  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  extern __shared__ __align__(128) unsigned char ring_smem[];
+  __shared__ __align__(8) unsigned long long s_full[RING_WARPS][RING_SLOTS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bid = blockIdx.x, band = g.rows_base + (bid < g.rows_rem ? 1 : 0), c_lo = row_begin + bid * g.rows_base + min(bid, g.rows_rem);
+  const int sl = warp % g.s, grp = warp / g.s, ngrp = RING_WARPS / g.s;
+  const int v0 = sl * g.vw, nv = max(0, min(g.vw, g.vpr - v0));      // this warp's vectors of a row
+  const int n = nv > 0 && band > grp ? (band - grp + ngrp - 1) / ngrp : 0;      // and its rows: grp, grp + ngrp, ..
+  unsigned char* ring = ring_smem + (size_t)warp * g.nslot * g.slot_bytes;
+  const unsigned ring_s = smem_u32(ring);
+  const unsigned char* src = static_cast<const unsigned char*>(w) + ((size_t)(c_lo + grp) * g.vpr + v0) * 16;
+  const size_t step = (size_t)ngrp * g.vpr * 16;
+  auto request = [&](int i, int slot) {      // lane 0
+    const unsigned bar = smem_u32(&s_full[warp][slot]);
+    mbar_expect_tx(bar, (unsigned)nv * 16u);
+    bulk_g2s(ring_s + (unsigned)slot * g.slot_bytes, src + (size_t)i * step, (unsigned)nv * 16u, bar);
+  };
+  if (lane == 0) {
+    for (int q = 0; q < g.nslot; q++) mbar_init(smem_u32(&s_full[warp][q]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < min(n, g.nslot); i++) request(i, i);      // weights do not depend on the previous kernel
+  }
+  __syncwarp();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const float* xb = x + (size_t)blockIdx.y * cols;
+  float xr[NV * EPV];
+#pragma unroll
+  for (int u = 0; u < NV; u++) {
+    const int v = u * 32 + lane;
+    const bool on = v < nv;
+    const float* xp = xb + (size_t)(v0 + (on ? v : 0)) * EPV;
+#pragma unroll
+    for (int e = 0; e < EPV; e += 4) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (on) {
+        if ((reinterpret_cast<uintptr_t>(xb) & 15) == 0) t = __ldg(reinterpret_cast<const float4*>(xp + e));
+        else t = make_float4(__ldg(xp + e), __ldg(xp + e + 1), __ldg(xp + e + 2), __ldg(xp + e + 3));
+      }
+      xr[u * EPV + e] = t.x; xr[u * EPV + e + 1] = t.y; xr[u * EPV + e + 2] = t.z; xr[u * EPV + e + 3] = t.w;
+    }
+  }
+  float* red = reinterpret_cast<float*>(ring_smem + g.red_off);      // [band][s]
+  int slot = 0;
+  unsigned par = 0;
+  bool dead = false;
+  int i = 0;
+  for (; i < n; i++) {
+    if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&s_full[warp][slot]), par))) { atomicCAS_system(err, 0, 900 + slot); dead = true; break; }
+    const uint4* p = reinterpret_cast<const uint4*>(ring + (size_t)slot * g.slot_bytes);
+    float acc[2] = {0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < NV; u++) {
+      const int v = u * 32 + lane;
+      if (v >= nv) continue;      // what lies behind the slice in the slot may be anything
+      const uint4 q = p[v];
+      const unsigned ws[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        if constexpr (DT == WV_DT_F32) acc[e & 1] = fmaf(__uint_as_float(ws[e]), xr[u * EPV + e], acc[e & 1]);
+        else {
+          float f0, f1;
+          if constexpr (DT == WV_DT_BF16) { f0 = __uint_as_float(ws[e] << 16); f1 = __uint_as_float(ws[e] & 0xffff0000u); }
+          else { const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&ws[e])); f0 = hf.x; f1 = hf.y; }
+          acc[0] = fmaf(f0, xr[u * EPV + 2 * e], acc[0]);
+          acc[1] = fmaf(f1, xr[u * EPV + 2 * e + 1], acc[1]);
+        }
+      }
+    }
+    __syncwarp();                                                  // every lane has read the slot
+    if (lane == 0 && i + g.nslot < n) request(i + g.nslot, slot);
+    float a = acc[0] + acc[1];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) red[(grp + i * ngrp) * g.s + sl] = a;
+    if (++slot == g.nslot) { slot = 0; par ^= 1u; }
+  }
+  if (dead && lane == 0)      // the copies still in flight
+    for (int j = i; j < min(n, i + g.nslot); j++) mbar_wait(smem_u32(&s_full[warp][j % g.nslot]), (unsigned)(j / g.nslot) & 1u);
+  if (nv == 0 && lane == 0) for (int r = grp; r < band; r += ngrp) red[r * g.s + sl] = 0.f;
+  __syncthreads();
+  float* yb = y + (size_t)blockIdx.y * rows + c_lo;
+  for (int r = tid; r < band; r += RING_WARPS * 32) {
+    float a = red[r * g.s];
+    for (int q = 1; q < g.s; q++) a += red[r * g.s + q];
+    yb[r] = a;
+  }
+}
+
 // ------------------------------------------------------------------ dispatch
 int wv_launch_gemv_ragged(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st);
 
@@ -507,8 +613,60 @@ static int launch_format(const WvDevBlob& b, const float* dx, float* dy, int bat
   return launch_chunked<F, 2, 1, 2>(b, dx, dy, batch, rb, re, st);
 }
 
+int* wv_tma_err_ptr();
+template <int DT, int NV>
+static int launch_ring_nv(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, const RingGeom& g, size_t smem, int grid, cudaStream_t st) {
+  auto kern = gemv_ring_kernel<DT, NV>;
+  static unsigned attr_mask = 0;
+  int dev = 0; cudaGetDevice(&dev);
+  if (!(attr_mask & (1u << (dev & 31)))) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return WV_ECUDA;
+    attr_mask |= 1u << (dev & 31);
+  }
+  const cudaError_t e = launch_pdl(kern, dim3(grid, batch), dim3(RING_WARPS * 32), smem, st, (const void*)b.lo, dx, dy, b.rows, b.cols, rb, g, wv_tma_err_ptr());
+  if (e != cudaSuccess) { wv_set_error("gemv (ring) launch: %s", cudaGetErrorString(e)); return WV_ECUDA; }
+  return WV_OK;
+}
+// Returns 1 for what the ring kernel does not take: rows under 4 KB or over 8192 columns (x in registers), and more rows of W, counted
+// once for every row of x, than half of the other kernel's warps. Beyond that it is the slower one for f32 (4096 x 4096 13.3 / 14.0 us,
+// 14336 x 4096 41 / 67) and level for the 16-bit types (4096 x 4096, two rows of x 14.8 / 14.3; 14336 x 4096 23.1 / 22.1).
+template <int DT>
+static int launch_ring(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
+  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  if (!wv_tma_err_ptr() || b.cols > 8192 || b.cols % EPV) return 1;
+  RingGeom g{};
+  g.vpr = b.cols / EPV;
+  if (g.vpr < 256) return 1;
+  g.s = 2;
+  while (g.s < RING_WARPS && g.vpr / g.s > (DT == WV_DT_F32 ? 192 : 128)) g.s *= 2;      // slices of some 2 KB; 16-bit: at most 32 values of x a lane
+  g.vw = (g.vpr + g.s - 1) / g.s;
+  const int nv = (g.vw + 31) / 32, sms = sm_count();
+  if ((long long)(re - rb) * batch > 16ll * sms) return 1;
+  int grid = 2 * sms;
+  if (grid > re - rb) grid = re - rb;
+  g.rows_base = (re - rb) / grid;
+  g.rows_rem = (re - rb) % grid;
+  const unsigned red = (unsigned)(g.rows_base + 1) * g.s * 4u, avail = 110u * 1024u;
+  g.slot_bytes = ((unsigned)g.vw * 16u + 127u) & ~127u;
+  if (red > avail / 2) return 1;
+  g.nslot = (int)((avail - red) / (g.slot_bytes * RING_WARPS));
+  if (g.nslot > RING_SLOTS) g.nslot = RING_SLOTS;
+  if (g.nslot < 2) return 1;
+  g.red_off = g.slot_bytes * g.nslot * RING_WARPS;
+  const size_t smem = g.red_off + red;
+  if (nv > 8 || (DT != WV_DT_F32 && nv > 5)) return 1;
+  if (nv <= 4) return launch_ring_nv<DT, 4>(b, dx, dy, batch, rb, re, g, smem, grid, st);
+  if constexpr (DT == WV_DT_F32) return launch_ring_nv<DT, 8>(b, dx, dy, batch, rb, re, g, smem, grid, st);
+  else return launch_ring_nv<DT, 5>(b, dx, dy, batch, rb, re, g, smem, grid, st);
+}
+
 template <int DT>
 static int launch_dense(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
+  if (!g_tune_d && !g_tune_grid) {
+    const int rc = launch_ring<DT>(b, dx, dy, batch, rb, re, st);
+    if (rc != 1) return rc;
+  }
   size_t smem = (size_t)b.cols * 4 + 16;
   if (smem > 110 * 1024) { wv_set_error("gemv: cols=%d needs %zu bytes of shared memory for x (max 112640)", b.cols, smem); return WV_ESHAPE; }
   static unsigned attr_mask = 0;
