@@ -909,11 +909,10 @@ int wv_launch_gemv(const WvDevBlob& b, const float* dx, float* dy, int batch, in
   if (pp && batch != 1) return WV_ESHAPE;
   const bool batched = batch >= 2 && !pp && !wv_cur_fuse && !g_tune_r && !wv_tma_tuning_rt() && !batch_loop_forced();   // a kernel forced by a tuning code keeps the batch on it
   // A few rows: up to four per pass over W on the integer-dot kernel, which is more precise than the tensor cores' TF32.
-  // Up to five rows that precision decides: in time the lines cross between four and five rows at 4096 x 4096 (Q4_K 11.3 us for
-  // four rows, 16.6 for five, the tensor-core kernel 15.3 whatever the batch; Q8_0, row by row, 13.6 and 16.7 against 15.6) and
-  // between five and six at 14336 x 4096 (Q4_K 35.9 and 40.4 against 36.3, Q8_0 36.5 and 42.6 against 38.7). At six the
-  // tensor-core kernel is the faster one, but for small matrices (1024 x 4096 in Q8_0 and Q4_0: 8.6 row by row, 10.8 and 10.3 there;
-  // level at eight rows).
+  // Up to five rows that precision decides: in time the lines cross between four and five rows at 4096 x 4096 (Q4_K 10.7 us for
+  // four rows, 15.4 for five, the tensor-core kernel 11.9 whatever the batch; Q8_0, row by row, 13.7 and 16.7 against 11.7) and at
+  // 14336 x 4096 (Q4_K 22.3 and 31.5 against 28.0, Q8_0 30.3 and 36.6 against 28.1). At six the tensor-core kernel is the faster one,
+  // for small matrices too (1024 x 4096 in Q8_0 and Q4_0: 7.9 row by row for five rows, 7.6 and 7.3 there for six).
   if (batched && batch < batch_min()) {
     const int rc = wv_launch_gemv_rows(b, dx, dy, batch, row_begin, row_end, st);
     if (rc != 1) return rc;

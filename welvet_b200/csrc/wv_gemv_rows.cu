@@ -9,8 +9,8 @@
 //
 // Bound: launch overhead at the sizes that stay in L2 (a 4096 x 4096 matrix in Q4_K streams in 1.7 us, and a launch costs
 // 4 us of start-up whatever it moves, which row-by-row launches pay per row); HBM for larger matrices.
-// Four rows against Q4_K: 11.1 us at 4096 x 4096 (18.8 row by row), 24.1 at 14336 x 4096 (34.8), 16.7 at 4096 x 6144 (23.1),
-// 5.3 at 1024 x 1024 (12.6); two rows at 4096 x 4096: 7.6 (9.8). A further row costs 1.7 us at 4096 x 4096: its dp4a.
+// Four rows against Q4_K: 10.7 us at 4096 x 4096 (18.8 row by row), 22.3 at 14336 x 4096 (34.8), 16.1 at 4096 x 6144 (23.1),
+// 5.6 at 1024 x 1024 (12.6); two rows at 4096 x 4096: 7.2 (9.8). A further row costs 1.6 us at 4096 x 4096: its dp2a.
 #include "wv_gemv_tma.cuh"
 
 int wv_act_width();   // wv_gemv_tma.cu: development switch (3 = always take 24-bit records)
