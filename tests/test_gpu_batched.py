@@ -132,6 +132,21 @@ def test_dense_forward_bias_and_activations(wv, rows, cols, batch, nbias):
         assert np.all(np.abs(post - ref) <= 2.0 ** -23 * np.abs(ref) + 2.0 ** -49 * np.abs(p) + 1e-45), act
 
 
+@pytest.mark.parametrize("rows,cols,batch", [(32, 32, 65537), (160, 64, 27000)])
+def test_dense_forward_bias_and_activation_of_large_batches(wv, rows, cols, batch):
+    """More rows than a grid has in y, and more results than the pinned buffer takes at a time (4 Mi floats): every row is the plain
+    product's row with the bias added in float64 and rounded, and its ReLU (both exact)."""
+    d = wv.dense
+    rng = np.random.default_rng(batch)
+    layer = d.NewConfigured(cols, rows, d.ActivationLinear, wv.quant.DTypeFloat32, wv.quant.Format.FormatQ8_0, rng.normal(0, 0.1, rows * cols).astype(np.float32))
+    x = rng.standard_normal((batch, cols), np.float32)
+    y = d.Forward(layer, x)[0]
+    layer.Weights.Bias, layer.Activation = rng.normal(0, 1, rows), d.ActivationReLU
+    pre, post = d.Forward(layer, x)
+    np.testing.assert_array_equal(pre, (y + layer.Weights.Bias).astype(np.float32))
+    np.testing.assert_array_equal(post, np.maximum(pre, 0))
+
+
 def test_host_pointer_calls_from_threads(wv):
     """wv_matvec (host pointers in and out) from six threads at once, as goroutines call Dense in the reference: the
     staging slots keep the calls apart, every result equals the single-threaded one bit for bit."""

@@ -931,6 +931,10 @@ __device__ __forceinline__ double activate(double v, int act) {
 }
 // A thread per output, bias[out] from device memory; both results go straight to mapped host memory. Bound by those stores: 0.9 MB
 // over a 50 GB/s host link are 18 us at 8 rows of 14336 outputs. On the host the same float64 passes took 0.45 of the call's 0.55 ms.
+// A launch takes a slice of the rows: WV_ACT_ROWS of them at most (they are the grid's y, which ends at 65535) and, unless one row is
+// more, WV_ACT_FLOATS results, so that the pinned buffer does not grow with the batch.
+#define WV_ACT_ROWS 32768
+#define WV_ACT_FLOATS (4 << 20)
 __global__ void __launch_bounds__(256) bias_act_kernel(const float* __restrict__ y, const double* __restrict__ bias, int nbias, int act, float* __restrict__ pre,
                                                        float* __restrict__ post, int out) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -959,21 +963,28 @@ extern "C" int wv_matvec_bias_act(uint64_t key, const float* x, const double* bi
   // x and the bias behind it in one pinned buffer, brought over together; W x stays on the device
   const size_t nx = (size_t)batch * in, ny = (size_t)batch * out, xpad = (nx + 3) & ~(size_t)3, nin = xpad + 2 * (size_t)nbias;
   const size_t npad = (nin + 3) & ~(size_t)3;
+  int slice = WV_ACT_FLOATS / out;
+  slice = slice < 1 ? 1 : (slice > WV_ACT_ROWS ? WV_ACT_ROWS : slice);
+  if (slice > batch) slice = batch;
+  const size_t ns = (size_t)slice * out;
   if ((rc = grow_mapped(&slot->ax, &slot->ax_dev, &slot->ax_n, npad)) || (rc = grow(&slot->da, &slot->da_n, npad + ny, false)) ||
-      (rc = grow_mapped(&slot->ay, &slot->ay_dev, &slot->ay_n, 2 * ny))) return rc;
+      (rc = grow_mapped(&slot->ay, &slot->ay_dev, &slot->ay_n, 2 * ns))) return rc;
   memcpy(slot->ax, x, nx * 4);
   if (nbias) memcpy(slot->ax + xpad, bias, (size_t)nbias * 8);
   const int n4 = (int)(npad / 4);
   const int blocks = n4 < 256 ? 1 : (n4 / 256 < 64 ? n4 / 256 : 64);
   stage_in_kernel<<<blocks, 256, 0, slot->st>>>(reinterpret_cast<const float4*>(slot->ax_dev), reinterpret_cast<float4*>(slot->da), n4, nullptr, nullptr, 0);
   rc = cudaGetLastError() == cudaSuccess ? wv_launch_gemv(e.blob, slot->da, slot->da + npad, batch, 0, e.blob.rows, slot->st) : WV_ECUDA;
-  if (!rc && launch_pdl(bias_act_kernel, dim3((out + 255) / 256, batch), dim3(256), 0, slot->st, slot->da + npad,
-                        reinterpret_cast<const double*>(slot->da + xpad), nbias, act, slot->ay_dev, slot->ay_dev + ny, out) != cudaSuccess) rc = WV_ECUDA;
+  for (int r0 = 0; !rc && r0 < batch; r0 += slice) {
+    const int nr = batch - r0 < slice ? batch - r0 : slice;
+    if (launch_pdl(bias_act_kernel, dim3((out + 255) / 256, nr), dim3(256), 0, slot->st, slot->da + npad + (size_t)r0 * out,
+                   reinterpret_cast<const double*>(slot->da + xpad), nbias, act, slot->ay_dev, slot->ay_dev + ns, out) != cudaSuccess) { rc = WV_ECUDA; break; }
+    CUDA_TRY(cudaStreamSynchronize(slot->st));
+    if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec_bias_act: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
+    memcpy(pre + (size_t)r0 * out, slot->ay, (size_t)nr * out * 4);
+    memcpy(post + (size_t)r0 * out, slot->ay + ns, (size_t)nr * out * 4);
+  }
   if (rc) { wv_set_error("wv_matvec_bias_act: launch failed (%d): %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
-  CUDA_TRY(cudaStreamSynchronize(slot->st));
-  if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec_bias_act: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
-  memcpy(pre, slot->ay, ny * 4);
-  memcpy(post, slot->ay + ny, ny * 4);
   return WV_OK;
 }
 
