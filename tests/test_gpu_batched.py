@@ -147,6 +147,26 @@ def test_dense_forward_bias_and_activation_of_large_batches(wv, rows, cols, batc
     np.testing.assert_array_equal(post, np.maximum(pre, 0))
 
 
+def test_calls_that_fail_between_two_launches(wv):
+    """Rows wider than FormatNone takes: x is on its way to the device when the GEMV's launch is refused. Both host calls report it
+    and the staging slot serves the next call."""
+    d, none = wv.dense, wv.quant.Format.FormatNone
+    rng = np.random.default_rng(11)
+    wide = d.NewConfigured(32768, 4, d.ActivationLinear, wv.quant.DTypeFloat32, none, rng.normal(0, 1, 4 * 32768).astype(np.float32))
+    layer = d.NewConfigured(64, 24, d.ActivationLinear, wv.quant.DTypeFloat32, none, rng.normal(0, 1, 24 * 64).astype(np.float32))
+    x = rng.standard_normal((40, 64), np.float32)
+    want = d.Forward(layer, x)[0]
+    for act in (d.ActivationLinear, d.ActivationReLU):
+        wide.Activation = layer.Activation = act
+        for batch in (1, 40):
+            with pytest.raises(wv._lib.WelvetError) as e:
+                d.Forward(wide, np.ones((batch, 32768), np.float32))
+            assert e.value.code == wv._lib.WV_ESHAPE
+            pre, post = d.Forward(layer, x)
+            np.testing.assert_array_equal(pre, want)
+            np.testing.assert_array_equal(post, want if act == d.ActivationLinear else np.maximum(want, 0))
+
+
 def test_host_pointer_calls_from_threads(wv):
     """wv_matvec (host pointers in and out) from six threads at once, as goroutines call Dense in the reference: the
     staging slots keep the calls apart, every result equals the single-threaded one bit for bit."""

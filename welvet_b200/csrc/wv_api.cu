@@ -857,6 +857,12 @@ static int take_slot(int batch, StageSlot** out) {
   return WV_OK;
 }
 
+// A call that fails between two of its launches: the first may still read the slot's buffers, which the next caller overwrites.
+static void abandon(StageSlot& slot, const char* who, int rc) {
+  wv_set_error("%s: launch failed (%d): %s", who, rc, cudaGetErrorString(cudaGetLastError()));
+  cudaStreamSynchronize(slot.st);
+}
+
 extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int in, int out) {
   int rc = ensure_init();
   if (rc) return rc;
@@ -906,7 +912,7 @@ extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int 
   }
   if (!launched) {
     rc = enqueue();
-    if (rc) { wv_set_error("wv_matvec: launch failed (%d): %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
+    if (rc) { abandon(*slot, "wv_matvec", rc); return rc; }
   }
   CUDA_TRY(cudaStreamSynchronize(slot->st));
   if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
@@ -984,8 +990,8 @@ extern "C" int wv_matvec_bias_act(uint64_t key, const float* x, const double* bi
     memcpy(pre + (size_t)r0 * out, slot->ay, (size_t)nr * out * 4);
     memcpy(post + (size_t)r0 * out, slot->ay + ns, (size_t)nr * out * 4);
   }
-  if (rc) { wv_set_error("wv_matvec_bias_act: launch failed (%d): %s", rc, cudaGetErrorString(cudaGetLastError())); return rc; }
-  return WV_OK;
+  if (rc) abandon(*slot, "wv_matvec_bias_act", rc);
+  return rc;
 }
 
 extern "C" int wv_device_status(void) {
