@@ -439,7 +439,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         bool bad = *(volatile int*)&s_abort != 0;
         const int s = stage_of(i, grp), use = i >> rsh;
         if (!bad && use > 0 && !mbar_wait(empty_bar(s), (use - 1) & 1, TCG_SPIN)) { atomicCAS_system(err, 0, 500 + s); *(volatile int*)&s_abort = 1; bad = true; }
-        if (__any_sync(0xffffffffu, bad)) { dead = true; break; }     // the whole warp leaves together (it meets at __syncwarp below)
+        if (__any_sync(0xffffffffu, bad)) { dead = true; break; }     // the whole warp leaves together (the stores below are warp-wide)
         tcg_fence_after();                    // the MMAs that read this stage before have been waited for
         float a[16];
         tcg_convert<F>(cur[u], s_tbl, [&](int p, const float (&v)[4]) {      // pieces come in rising order
@@ -449,6 +449,7 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
         });
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tcg_fence_before();
+        __syncwarp();                                 // every lane's stores come before the one arrival
         if (lane == 0) mbar_arrive(full_bar(s));      // one arrival per warp
         made = i + 1;
       }
