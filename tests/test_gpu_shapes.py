@@ -253,3 +253,38 @@ def test_plain_rows_at_the_limits_of_the_ring_kernel(wv, dt, rows, cols, batch):
         assert L.wv_device_status() == 0
     finally:
         L.wv_blob_evict(key)
+
+
+@pytest.mark.parametrize("dt,rows,cols", [(1, 4096, 4096), (1, 2500, 5000), (1, 2400, 8192), (2, 2400, 2056), (2, 4096, 4096), (3, 3001, 8192)])
+def test_plain_rows_do_not_depend_on_the_launch(wv, dt, rows, cols):
+    """FormatNone: a row's bits are the same in the whole matrix, in a shard of its rows and with any number of rows of x, on either
+    side of the line between the two kernels (2368 rows, counted once for every row of x)."""
+    import torch
+    from welvet_b200 import _lib
+    L, check = _lib.lib(), _lib.check
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    w = torch.randn(rows, cols, device="cuda", generator=gen) * 0.02
+    x = torch.randn(3, cols, device="cuda", generator=gen)
+    cuts = [0, 7, rows // 3, rows // 3 + 1200, rows]
+    keys = [0x7100 + i for i in range(len(cuts))]
+    torch.cuda.synchronize()
+
+    def call(key, n, batch):
+        y = torch.full((batch, n), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), batch, cols, n, None))
+        torch.cuda.synchronize()
+        return y
+    try:
+        check(L.wv_pack_upload_dev(keys[-1], 0, dt, 0, w.data_ptr(), rows, cols, None))
+        for key, a, b in zip(keys, cuts, cuts[1:]):
+            check(L.wv_pack_upload_dev(key, 0, dt, 0, w[a].data_ptr(), b - a, cols, None))
+        whole = call(keys[-1], rows, 3)
+        assert torch.equal(call(keys[-1], rows, 1), whole[:1])
+        for batch in (1, 2, 3):
+            parts = [call(key, b - a, batch) for key, a, b in zip(keys, cuts, cuts[1:])]
+            assert torch.equal(torch.cat(parts, 1), whole[:batch])
+        assert L.wv_device_status() == 0
+    finally:
+        for key in keys:
+            L.wv_blob_evict(key)

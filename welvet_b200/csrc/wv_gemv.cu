@@ -319,14 +319,48 @@ gemv_idot_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, float* __rest
 // ------------------------------------------------------------------ FormatNone f32 / f16 / bf16
 // Plain streaming GEMV (the reference's DotTile / DotF16Packed / DotBF16Packed rows,
 // layers/dense/simd.go:201-284): two 512-thread CTAs per SM, a warp owns whole rows, lanes
-// read consecutive 16-byte vectors, U vectors per lane per step with the next step's loads
-// issued before the current step's arithmetic (2*U*512 bytes per warp in flight).
+// read consecutive 16-byte vectors, four per lane per step with the next step's loads
+// issued before the current step's arithmetic (4 KB per warp in flight).
+//
+// The order of summation is the same here and in gemv_ring_kernel below, whatever the launch, so that a row's bits do not depend on
+// which of the two a launch takes (on how many rows of W a rank holds, or how many rows x has): a row is cut into slices
+// of 128 vectors (2 KB); in a slice lane l adds vectors l, l + 32, .. to two running sums, and those and lane l ^ 16's
+// are added; the slices' sums are added lane by lane in rising order, and the sixteen lanes' by butterfly.
+// (The whole butterfly for every slice cost up to 12 % here: f16 14336 x 4096 22.3 -> 24.9 us.)
+#define PLAIN_SLICE 128
+template <int DT> struct PlainVec { static constexpr int N = DT == WV_DT_F32 ? 4 : 8; };      // elements per 16-byte vector
+template <int DT>
+__device__ __forceinline__ void plain_fma(const uint4& q, const float* x, float (&acc)[2]) {
+  const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    if constexpr (DT == WV_DT_F32) acc[e & 1] = fmaf(__uint_as_float(w[e]), x[e], acc[e & 1]);
+    else {
+      float f0, f1;
+      if constexpr (DT == WV_DT_BF16) { f0 = __uint_as_float(w[e] << 16); f1 = __uint_as_float(w[e] & 0xffff0000u); }
+      else { const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&w[e])); f0 = hf.x; f1 = hf.y; }
+      acc[0] = fmaf(f0, x[2 * e], acc[0]);
+      acc[1] = fmaf(f1, x[2 * e + 1], acc[1]);
+    }
+  }
+}
+__device__ __forceinline__ float plain_slice_sum(const float (&acc)[2]) {      // lanes l and l + 16 get the same
+  const float a = acc[0] + acc[1];
+  return a + __shfl_xor_sync(0xffffffffu, a, 16);
+}
+__device__ __forceinline__ float plain_row_sum(float t) {
+#pragma unroll
+  for (int o = 8; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
 #define WV_DENSE_THREADS 512
-template <int DT, int U>
+template <int DT>
+
 __global__ void __launch_bounds__(WV_DENSE_THREADS, 2)
 gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y, int row_begin, int row_end) {
-  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;  // elements per 16-byte vector
-  constexpr int NW = WV_DENSE_THREADS / 32;
+  constexpr int EPV = PlainVec<DT>::N;
+  constexpr int NW = WV_DENSE_THREADS / 32, U = PLAIN_SLICE / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* xs = reinterpret_cast<float*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -336,98 +370,84 @@ gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restr
   const int c_lo = (int)(((long long)blockIdx.x * nrows) / gridDim.x), c_hi = (int)(((long long)(blockIdx.x + 1) * nrows) / gridDim.x);
   const int r_lo = c_lo + (int)(((long long)warp * (c_hi - c_lo)) / NW), r_hi = c_lo + (int)(((long long)(warp + 1) * (c_hi - c_lo)) / NW);
   const int vpr = b.cols / EPV;
-  const int steps_per_row = (vpr + 32 * U - 1) / (32 * U);
-  const int nsteps = (r_hi - r_lo) * steps_per_row;
-  const uint4* wbase = reinterpret_cast<const uint4*>(b.lo) + (size_t)row_begin * vpr;
-  auto load_step = [&](uint4 (&w)[U], int step) {
-    const int row = r_lo + step / steps_per_row, v0 = (step % steps_per_row) * 32 * U;
+  const uint4* wbase = reinterpret_cast<const uint4*>(b.lo) + (size_t)row_begin * vpr + lane;
+  int lrow = r_lo, lv = 0;      // where the next step to be loaded starts
+  auto load_step = [&](uint4 (&w)[U]) {
+    const uint4* p = wbase + (size_t)lrow * vpr + lv;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int v = v0 + u * 32 + lane;
-      w[u] = (step < nsteps && v < vpr) ? __ldg(wbase + (size_t)row * vpr + v) : make_uint4(0, 0, 0, 0);
-    }
+    for (int u = 0; u < U; u++) w[u] = (lrow < r_hi && lv + u * 32 + lane < vpr) ? __ldg(p + u * 32) : make_uint4(0, 0, 0, 0);
+    lv += PLAIN_SLICE;
+    if (lv >= vpr) { lv = 0; lrow++; }
   };
   uint4 nxt[U];
-  load_step(nxt, 0);   // weights do not depend on the previous kernel
+  load_step(nxt);   // weights do not depend on the previous kernel
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int c = tid; c < b.cols; c += WV_DENSE_THREADS) xs[c] = xb[c];
   __syncthreads();
-  float acc = 0.f;
-  for (int step = 0; step < nsteps; step++) {
+  float sum = 0.f;
+  int v0 = 0;
+  for (int row = r_lo; row < r_hi; ) {
     uint4 cur[U];
 #pragma unroll
     for (int u = 0; u < U; u++) cur[u] = nxt[u];
-    load_step(nxt, step + 1);
-    const int v0 = (step % steps_per_row) * 32 * U;
+    load_step(nxt);
+    float acc[2] = {0.f, 0.f};
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int v = v0 + u * 32 + lane;
       if (v < vpr) {
+        float xe[EPV];
         const float4* xp = reinterpret_cast<const float4*>(xs + (size_t)v * EPV);
-        const float4 xa = xp[0];
-        const uint4 q = cur[u];
-        if constexpr (DT == WV_DT_F32) {
-          acc = fmaf(__uint_as_float(q.x), xa.x, acc); acc = fmaf(__uint_as_float(q.y), xa.y, acc);
-          acc = fmaf(__uint_as_float(q.z), xa.z, acc); acc = fmaf(__uint_as_float(q.w), xa.w, acc);
-        } else {
-          const float4 xc = xp[1];
-          const unsigned ws[4] = {q.x, q.y, q.z, q.w};
-          const float xe[8] = {xa.x, xa.y, xa.z, xa.w, xc.x, xc.y, xc.z, xc.w};
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            float f0, f1;
-            if constexpr (DT == WV_DT_BF16) { f0 = __uint_as_float(ws[i] << 16); f1 = __uint_as_float(ws[i] & 0xffff0000u); }
-            else {
-              const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&ws[i]));
-              f0 = hf.x; f1 = hf.y;
-            }
-            acc = fmaf(f0, xe[2 * i], acc); acc = fmaf(f1, xe[2 * i + 1], acc);
-          }
-        }
+        for (int e = 0; e < EPV; e += 4) { const float4 t = xp[e / 4]; xe[e] = t.x; xe[e + 1] = t.y; xe[e + 2] = t.z; xe[e + 3] = t.w; }
+        plain_fma<DT>(cur[u], xe, acc);
       }
     }
-    if ((step + 1) % steps_per_row == 0) {
-#pragma unroll
-      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) yb[r_lo + step / steps_per_row] = acc;
-      acc = 0.f;
+    sum += plain_slice_sum(acc);
+    v0 += PLAIN_SLICE;
+    if (v0 >= vpr) {
+      sum = plain_row_sum(sum);
+      if (lane == 0) yb[row] = sum;
+      sum = 0.f;
+      v0 = 0;
+      row++;
     }
   }
 }
 
 // ------------------------------------------------------------------ FormatNone through a shared-memory ring
 // The same product for few rows of 4 to 32 KB. Bound: latency. The kernel above gives a warp whole rows, with two steps of 2 KB in
-// flight, so that few rows leave most of its warps without work. Here S of a CTA's sixteen warps share a row: a warp's slice of
-// the columns is fixed, so its part of x stays in registers, and a ring of its own brings in the slice of one row after the
-// other (lane 0 requests, before the wait for the preceding kernel what the ring holds; the warp reads: nothing to wait for but
-// its own copies; slices of some 2 KB, since a copy costs about 45 ns whatever its size). The slices' sums of a band meet in
-// shared memory at the end. Two CTAs fill an SM: with one for each SM, two of them went to the SMs that the preceding kernel left
+// flight, so that few rows leave most of its warps without work. Here a warp takes one slice of every row (two, C = 2, where a row
+// has more than eight and there are rows enough: half as many copies, each of which costs about 45 ns whatever its size), as many
+// rows side by side as sixteen warps have room for: its part of x stays in registers, and a ring of its own brings in the slice of
+// one row after the other (lane 0 requests, before the wait for the preceding kernel what the ring holds; the warp reads: nothing
+// to wait for but its own copies). The slices' sums of a band meet in shared memory at the end, sixteen lanes to a slice.
+// Two CTAs fill an SM: with one for each SM, two of them went to the SMs that the preceding kernel left
 // first and others stayed empty (a 4096 x 4096 f32 launch behind one of Q4_K: 30 us instead of 13).
-// us per launch, the kernel above / this one: f32 512 x 8192 11.5 / 4.0, 2368 x 2048 6.1 / 4.7; f16 1000 x 8192 8.3 / 4.7, 1500 x 3000
-// 4.8 / 3.8, 2000 x 2048 3.7 / 3.6.
+// us per launch, the kernel above / this one: f32 512 x 8192 11.5 / 3.9, 2368 x 2048 5.9 / 4.5, 2368 x 8192 15.0 / 12.6 (one slice a
+// warp 14.2); f16 1000 x 8192 8.3 / 4.6, 1400 x 3000 4.6 / 3.3, 2000 x 2048 3.8 / 3.3.
 #define RING_WARPS 16
 #define RING_SLOTS 16
-struct RingGeom { int vpr, vw, s, nslot; unsigned slot_bytes, red_off; int rows_base, rows_rem; };      // vectors per row and slice, slices per row, slots per warp
-template <int DT, int NV>      // NV: 16-byte vectors of a slice per lane at most
+struct RingGeom { int vpr, ns, s, ngrp, nslot; unsigned red_off; int rows_base, rows_rem; };      // vectors and slices of a row, warps to a row, rows side by side, slots per warp
+template <int DT, int C>      // C: consecutive slices a warp takes of its rows
 __global__ void __launch_bounds__(RING_WARPS * 32, 2)
 gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float* __restrict__ y, int rows, int cols, int row_begin, const RingGeom g, int* __restrict__ err) {
-  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  constexpr int EPV = PlainVec<DT>::N, US = PLAIN_SLICE / 32, NV = C * US;
+  constexpr unsigned SLOT = C * PLAIN_SLICE * 16;
   extern __shared__ __align__(128) unsigned char ring_smem[];
   __shared__ __align__(8) unsigned long long s_full[RING_WARPS][RING_SLOTS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bid = blockIdx.x, band = g.rows_base + (bid < g.rows_rem ? 1 : 0), c_lo = row_begin + bid * g.rows_base + min(bid, g.rows_rem);
-  const int sl = warp % g.s, grp = warp / g.s, ngrp = RING_WARPS / g.s;
-  const int v0 = sl * g.vw, nv = max(0, min(g.vw, g.vpr - v0));      // this warp's vectors of a row
-  const int n = nv > 0 && band > grp ? (band - grp + ngrp - 1) / ngrp : 0;      // and its rows: grp, grp + ngrp, ..
-  unsigned char* ring = ring_smem + (size_t)warp * g.nslot * g.slot_bytes;
+  const int ngrp = g.ngrp, sl = warp % g.s, grp = warp / g.s;
+  const int v0 = sl * C * PLAIN_SLICE, nv = min(C * PLAIN_SLICE, g.vpr - v0);      // this warp's vectors of a row
+  const int n = grp < ngrp && band > grp ? (band - grp + ngrp - 1) / ngrp : 0;      // and its rows: grp, grp + ngrp, ..; warps past the last group have none
+  unsigned char* ring = ring_smem + (size_t)warp * g.nslot * SLOT;
   const unsigned ring_s = smem_u32(ring);
-  const unsigned char* src = static_cast<const unsigned char*>(w) + ((size_t)(c_lo + grp) * g.vpr + v0) * 16;
-  const size_t step = (size_t)ngrp * g.vpr * 16;
   auto request = [&](int i, int slot) {      // lane 0
     const unsigned bar = smem_u32(&s_full[warp][slot]);
     mbar_expect_tx(bar, (unsigned)nv * 16u);
-    bulk_g2s(ring_s + (unsigned)slot * g.slot_bytes, src + (size_t)i * step, (unsigned)nv * 16u, bar);
+    bulk_g2s(ring_s + (unsigned)slot * SLOT, static_cast<const uint4*>(w) + (size_t)(c_lo + grp + i * ngrp) * g.vpr + v0, (unsigned)nv * 16u, bar);
   };
   if (lane == 0) {
     for (int q = 0; q < g.nslot; q++) mbar_init(smem_u32(&s_full[warp][q]), 1);
@@ -438,66 +458,56 @@ gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float*
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const float* xb = x + (size_t)blockIdx.y * cols;
-  float xr[NV * EPV];
+  float xr[NV * EPV];      // lanes past the slice hold some of its x; they are not used
+  const bool x16 = (reinterpret_cast<uintptr_t>(xb) & 15) == 0;
+  if (x16) {               // no test between the loads: they travel together (one by one, f16 256 x 6144 took 3.3 us instead of 2.8)
 #pragma unroll
-  for (int u = 0; u < NV; u++) {
-    const int v = u * 32 + lane;
-    const bool on = v < nv;
-    const float* xp = xb + (size_t)(v0 + (on ? v : 0)) * EPV;
+    for (int u = 0; u < NV; u++)
 #pragma unroll
-    for (int e = 0; e < EPV; e += 4) {
-      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (on) {
-        if ((reinterpret_cast<uintptr_t>(xb) & 15) == 0) t = __ldg(reinterpret_cast<const float4*>(xp + e));
-        else t = make_float4(__ldg(xp + e), __ldg(xp + e + 1), __ldg(xp + e + 2), __ldg(xp + e + 3));
+      for (int e = 0; e < EPV; e += 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(xb + (size_t)(v0 + min(u * 32 + lane, nv - 1)) * EPV + e));
+        xr[u * EPV + e] = t.x; xr[u * EPV + e + 1] = t.y; xr[u * EPV + e + 2] = t.z; xr[u * EPV + e + 3] = t.w;
       }
-      xr[u * EPV + e] = t.x; xr[u * EPV + e + 1] = t.y; xr[u * EPV + e + 2] = t.z; xr[u * EPV + e + 3] = t.w;
-    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < NV; u++)
+#pragma unroll
+      for (int e = 0; e < EPV; e++) xr[u * EPV + e] = __ldg(xb + (size_t)(v0 + min(u * 32 + lane, nv - 1)) * EPV + e);
   }
-  float* red = reinterpret_cast<float*>(ring_smem + g.red_off);      // [band][s]
+  float* red = reinterpret_cast<float*>(ring_smem + g.red_off);      // [band][ns][16]
   int slot = 0;
   unsigned par = 0;
   bool dead = false;
   int i = 0;
   for (; i < n; i++) {
     if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&s_full[warp][slot]), par))) { atomicCAS_system(err, 0, 900 + slot); dead = true; break; }
-    const uint4* p = reinterpret_cast<const uint4*>(ring + (size_t)slot * g.slot_bytes);
-    float acc[2] = {0.f, 0.f};
+    const uint4* p = reinterpret_cast<const uint4*>(ring + (size_t)slot * SLOT);
+    float acc[C][2];
 #pragma unroll
     for (int u = 0; u < NV; u++) {
+      if (u % US == 0) acc[u / US][0] = acc[u / US][1] = 0.f;
       const int v = u * 32 + lane;
-      if (v >= nv) continue;      // what lies behind the slice in the slot may be anything
-      const uint4 q = p[v];
-      const unsigned ws[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        if constexpr (DT == WV_DT_F32) acc[e & 1] = fmaf(__uint_as_float(ws[e]), xr[u * EPV + e], acc[e & 1]);
-        else {
-          float f0, f1;
-          if constexpr (DT == WV_DT_BF16) { f0 = __uint_as_float(ws[e] << 16); f1 = __uint_as_float(ws[e] & 0xffff0000u); }
-          else { const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&ws[e])); f0 = hf.x; f1 = hf.y; }
-          acc[0] = fmaf(f0, xr[u * EPV + 2 * e], acc[0]);
-          acc[1] = fmaf(f1, xr[u * EPV + 2 * e + 1], acc[1]);
-        }
-      }
+      if (v < nv) plain_fma<DT>(p[v], xr + u * EPV, acc[u / US]);      // what lies behind the slices in the slot may be anything
     }
     __syncwarp();                                                  // every lane has read the slot
     if (lane == 0 && i + g.nslot < n) request(i + g.nslot, slot);
-    float a = acc[0] + acc[1];
 #pragma unroll
-    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) red[(grp + i * ngrp) * g.s + sl] = a;
+    for (int c = 0; c < C; c++) {
+      const float a = plain_slice_sum(acc[c]);
+      if (lane < 16 && c * PLAIN_SLICE < nv) red[((grp + i * ngrp) * g.ns + sl * C + c) * 16 + lane] = a;
+    }
     if (++slot == g.nslot) { slot = 0; par ^= 1u; }
   }
   if (dead && lane == 0)      // the copies still in flight
     for (int j = i; j < min(n, i + g.nslot); j++) mbar_wait(smem_u32(&s_full[warp][j % g.nslot]), (unsigned)(j / g.nslot) & 1u);
-  if (nv == 0 && lane == 0) for (int r = grp; r < band; r += ngrp) red[r * g.s + sl] = 0.f;
   __syncthreads();
   float* yb = y + (size_t)blockIdx.y * rows + c_lo;
-  for (int r = tid; r < band; r += RING_WARPS * 32) {
-    float a = red[r * g.s];
-    for (int q = 1; q < g.s; q++) a += red[r * g.s + q];
-    yb[r] = a;
+  for (int r0 = warp * 2; r0 < band; r0 += RING_WARPS * 2) {      // sixteen lanes to a row
+    const int r = r0 + (lane >> 4);
+    float t = 0.f;
+    if (r < band) for (int q = 0; q < g.ns; q++) t += red[(r * g.ns + q) * 16 + (lane & 15)];
+    t = plain_row_sum(t);
+    if (r < band && (lane & 15) == 0) yb[r] = t;
   }
 }
 
@@ -614,9 +624,9 @@ static int launch_format(const WvDevBlob& b, const float* dx, float* dy, int bat
 }
 
 int* wv_tma_err_ptr();
-template <int DT, int NV>
-static int launch_ring_nv(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, const RingGeom& g, size_t smem, int grid, cudaStream_t st) {
-  auto kern = gemv_ring_kernel<DT, NV>;
+template <int DT, int C>
+static int launch_ring_c(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, const RingGeom& g, size_t smem, int grid, cudaStream_t st) {
+  auto kern = gemv_ring_kernel<DT, C>;
   static unsigned attr_mask = 0;
   int dev = 0; cudaGetDevice(&dev);
   if (!(attr_mask & (1u << (dev & 31)))) {
@@ -629,36 +639,38 @@ static int launch_ring_nv(const WvDevBlob& b, const float* dx, float* dy, int ba
   return WV_OK;
 }
 // Returns 1 for what the ring kernel does not take: rows under 4 KB or over 8192 columns (x in registers), and more rows of W, counted
-// once for every row of x, than half of the other kernel's warps. Beyond that it is the slower one for f32 (4096 x 4096 13.3 / 14.0 us,
-// 14336 x 4096 41 / 67) and level for the 16-bit types (4096 x 4096, two rows of x 14.8 / 14.3; 14336 x 4096 23.1 / 22.1).
+// once for every row of x, than half of the other kernel's warps. Beyond that it is the slower one where the matrix is large, as its
+// copies of 2 KB come to some 4.5 TB/s (f32 8192 x 4096 22.2 / 26.8 us, 14336 x 4096 39 / 59; f16 14336 x 5000 28.2 / 32.5), and level
+// or faster below (f32 4096 x 4096 12.6 / 12.6, f16 8.0 / 8.1).
 template <int DT>
 static int launch_ring(const WvDevBlob& b, const float* dx, float* dy, int batch, int rb, int re, cudaStream_t st) {
-  constexpr int EPV = DT == WV_DT_F32 ? 4 : 8;
+  constexpr int EPV = PlainVec<DT>::N;
   if (!wv_tma_err_ptr() || b.cols > 8192 || b.cols % EPV) return 1;
   RingGeom g{};
   g.vpr = b.cols / EPV;
-  if (g.vpr < 256) return 1;
-  g.s = 2;
-  while (g.s < RING_WARPS && g.vpr / g.s > (DT == WV_DT_F32 ? 192 : 128)) g.s *= 2;      // slices of some 2 KB; 16-bit: at most 32 values of x a lane
-  g.vw = (g.vpr + g.s - 1) / g.s;
-  const int nv = (g.vw + 31) / 32, sms = sm_count();
+  if (g.vpr < 2 * PLAIN_SLICE) return 1;
+  const int sms = sm_count();
   if ((long long)(re - rb) * batch > 16ll * sms) return 1;
+  g.ns = (g.vpr + PLAIN_SLICE - 1) / PLAIN_SLICE;      // at most 16, and 8 for the 16-bit types
+  // Two slices a warp from about six rows of twelve slices to a CTA; below, more warps start sooner (256 x 6144 2.4 / 2.9 us, 700 x 6144
+  // 4.0 / 4.2; 1400 x 6144 7.5 / 6.4, 2000 x 4608 8.8 / 6.8 with one / two). The order of summation is the same.
+  const int c = DT == WV_DT_F32 && g.ns > 8 && (re - rb) * g.ns > 88 * sms ? 2 : 1;
+  g.s = (g.ns + c - 1) / c;
   int grid = 2 * sms;
   if (grid > re - rb) grid = re - rb;
   g.rows_base = (re - rb) / grid;
   g.rows_rem = (re - rb) % grid;
-  const unsigned red = (unsigned)(g.rows_base + 1) * g.s * 4u, avail = 110u * 1024u;
-  g.slot_bytes = ((unsigned)g.vw * 16u + 127u) & ~127u;
+  const unsigned red = (unsigned)(g.rows_base + 1) * g.ns * 64u, avail = 110u * 1024u, slot = (unsigned)c * PLAIN_SLICE * 16u;
   if (red > avail / 2) return 1;
-  g.nslot = (int)((avail - red) / (g.slot_bytes * RING_WARPS));
+  g.ngrp = RING_WARPS / g.s;
+  while (g.ngrp > 1 && (avail - red) / (slot * g.s * g.ngrp) < 3) g.ngrp--;
+  g.nslot = (int)((avail - red) / (slot * g.s * g.ngrp));
   if (g.nslot > RING_SLOTS) g.nslot = RING_SLOTS;
   if (g.nslot < 2) return 1;
-  g.red_off = g.slot_bytes * g.nslot * RING_WARPS;
+  g.red_off = slot * g.nslot * g.s * g.ngrp;
   const size_t smem = g.red_off + red;
-  if (nv > 8 || (DT != WV_DT_F32 && nv > 5)) return 1;
-  if (nv <= 4) return launch_ring_nv<DT, 4>(b, dx, dy, batch, rb, re, g, smem, grid, st);
-  if constexpr (DT == WV_DT_F32) return launch_ring_nv<DT, 8>(b, dx, dy, batch, rb, re, g, smem, grid, st);
-  else return launch_ring_nv<DT, 5>(b, dx, dy, batch, rb, re, g, smem, grid, st);
+  if constexpr (DT == WV_DT_F32) if (c == 2) return launch_ring_c<DT, 2>(b, dx, dy, batch, rb, re, g, smem, grid, st);
+  return launch_ring_c<DT, 1>(b, dx, dy, batch, rb, re, g, smem, grid, st);
 }
 
 template <int DT>
@@ -670,9 +682,9 @@ static int launch_dense(const WvDevBlob& b, const float* dx, float* dy, int batc
   size_t smem = (size_t)b.cols * 4 + 16;
   if (smem > 110 * 1024) { wv_set_error("gemv: cols=%d needs %zu bytes of shared memory for x (max 112640)", b.cols, smem); return WV_ESHAPE; }
   static unsigned attr_mask = 0;
-  auto kern = g_tune_d == 8 ? gemv_dense_kernel<DT, 8> : gemv_dense_kernel<DT, 4>;   // vectors per lane per step (tuning hook)
+  auto kern = gemv_dense_kernel<DT>;
   int dev = 0; cudaGetDevice(&dev);
-  const unsigned bit = (1u << dev) << (g_tune_d == 8 ? 16 : 0);
+  const unsigned bit = 1u << dev;
   if (!(attr_mask & bit)) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024) != cudaSuccess) return WV_ECUDA;
     attr_mask |= bit;
