@@ -288,3 +288,37 @@ def test_plain_rows_do_not_depend_on_the_launch(wv, dt, rows, cols):
     finally:
         for key in keys:
             L.wv_blob_evict(key)
+
+
+@pytest.mark.parametrize("dt,rows,cols,row", [(1, 2000, 4096, 1), (1, 2000, 4096, 3), (1, 2000, 6144, 5), (2, 1000, 8192, 2), (2, 40, 2048, 1)])
+def test_plain_rows_after_a_wait_that_runs_out(wv, hooks, dt, rows, cols, row):
+    """The ring kernel of FormatNone with a copy that never comes: the call is reported, the rows that were not summed are NaN and
+    the others have their bits; the next call is sound."""
+    import torch
+    from welvet_b200 import _lib
+    L, check, key = _lib.lib(), _lib.check, 0x7200
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    w, x = torch.randn(rows, cols, device="cuda", generator=gen) * 0.02, torch.randn(cols, device="cuda", generator=gen)
+    torch.cuda.synchronize()
+    check(L.wv_pack_upload_dev(key, 0, dt, 0, w.data_ptr(), rows, cols, None))
+
+    def call():
+        y = torch.zeros(rows, device="cuda")
+        torch.cuda.synchronize()
+        check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), 1, cols, rows, None))
+        torch.cuda.synchronize()
+        return y, L.wv_device_status()
+    try:
+        want, status = call()
+        assert status == 0
+        hooks.wv_set_ring_stall(row, 2000)
+        try:
+            y, status = call()
+        finally:
+            hooks.wv_set_ring_stall(0, 0)
+        assert status == _lib.WV_ETIMEOUT
+        assert bool(y.isnan().any()) and (bool((~y.isnan()).any()) or row == 1) and bool((y.isnan() | (y == want)).all())
+        y, status = call()
+        assert status == 0 and torch.equal(y, want)
+    finally:
+        L.wv_blob_evict(key)

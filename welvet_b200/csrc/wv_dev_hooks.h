@@ -17,6 +17,9 @@ void wv_set_act_width(int limbs);
 // Batched kernel: the first producer warp stops short of its `slice`-th slice (1, 2, ...; 0 = off) and the waits give up after
 // `spin` polls (0 = built-in limit), so that a bounded wait runs out.
 void wv_set_tcg_stall(int slice, int spin);
+// FormatNone ring kernel: the first warp of every CTA never requests its `row`-th row (1, 2, ...; 0 = off) and the waits give up after
+// `spin` polls (0 = built-in limit).
+void wv_set_ring_stall(int row, int spin);
 #ifdef __cplusplus
 }
 #endif

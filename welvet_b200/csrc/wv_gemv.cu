@@ -429,7 +429,23 @@ gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restr
 // warp 14.2); f16 1000 x 8192 8.3 / 4.6, 1400 x 3000 4.6 / 3.3, 2000 x 2048 3.8 / 3.3.
 #define RING_WARPS 16
 #define RING_SLOTS 16
-struct RingGeom { int vpr, ns, s, ngrp, nslot; unsigned red_off; int rows_base, rows_rem; };      // vectors and slices of a row, warps to a row, rows side by side, slots per warp
+struct RingGeom {
+  int vpr, ns, s, ngrp, nslot;      // vectors and slices of a row, warps to a row, rows side by side, slots per warp
+  unsigned red_off;
+  int rows_base, rows_rem;
+#ifdef WV_DEV_HOOKS
+  int stall;                        // > 0: the first warp withholds the request for its stall-th row, so that a wait runs out
+  unsigned spin;
+#endif
+};
+#ifdef WV_DEV_HOOKS
+static int g_ring_stall = 0;
+static unsigned g_ring_spin = TMA_SPIN_LIMIT;
+extern "C" void wv_set_ring_stall(int row, int spin) { g_ring_stall = row; g_ring_spin = spin > 0 ? (unsigned)spin : TMA_SPIN_LIMIT; }
+#define RING_SPIN g.spin
+#else
+#define RING_SPIN TMA_SPIN_LIMIT
+#endif
 template <int DT, int C>      // C: consecutive slices a warp takes of its rows
 __global__ void __launch_bounds__(RING_WARPS * 32, 2)
 gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float* __restrict__ y, int rows, int cols, int row_begin, const RingGeom g, int* __restrict__ err) {
@@ -446,6 +462,9 @@ gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float*
   const unsigned ring_s = smem_u32(ring);
   auto request = [&](int i, int slot) {      // lane 0
     const unsigned bar = smem_u32(&s_full[warp][slot]);
+#ifdef WV_DEV_HOOKS
+    if (warp == 0 && i + 1 == g.stall) return;
+#endif
     mbar_expect_tx(bar, (unsigned)nv * 16u);
     bulk_g2s(ring_s + (unsigned)slot * SLOT, static_cast<const uint4*>(w) + (size_t)(c_lo + grp + i * ngrp) * g.vpr + v0, (unsigned)nv * 16u, bar);
   };
@@ -480,7 +499,7 @@ gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float*
   bool dead = false;
   int i = 0;
   for (; i < n; i++) {
-    if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&s_full[warp][slot]), par))) { atomicCAS_system(err, 0, 900 + slot); dead = true; break; }
+    if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&s_full[warp][slot]), par, RING_SPIN))) { atomicCAS_system(err, 0, 900 + slot); dead = true; break; }
     const uint4* p = reinterpret_cast<const uint4*>(ring + (size_t)slot * SLOT);
     float acc[C][2];
 #pragma unroll
@@ -498,8 +517,13 @@ gemv_ring_kernel(const void* __restrict__ w, const float* __restrict__ x, float*
     }
     if (++slot == g.nslot) { slot = 0; par ^= 1u; }
   }
-  if (dead && lane == 0)      // the copies still in flight
-    for (int j = i; j < min(n, i + g.nslot); j++) mbar_wait(smem_u32(&s_full[warp][j % g.nslot]), (unsigned)(j / g.nslot) & 1u);
+  if (dead) {                 // the copies still in flight; the rows not summed come out as NaN
+    if (lane == 0) for (int j = i; j < min(n, i + g.nslot); j++) mbar_wait(smem_u32(&s_full[warp][j % g.nslot]), (unsigned)(j / g.nslot) & 1u, RING_SPIN);
+    for (; i < n; i++)
+#pragma unroll
+      for (int c = 0; c < C; c++)
+        if (lane < 16 && c * PLAIN_SLICE < nv) red[((grp + i * ngrp) * g.ns + sl * C + c) * 16 + lane] = __uint_as_float(0x7fc00000u);
+  }
   __syncthreads();
   float* yb = y + (size_t)blockIdx.y * rows + c_lo;
   for (int r0 = warp * 2; r0 < band; r0 += RING_WARPS * 2) {      // sixteen lanes to a row
@@ -668,6 +692,9 @@ static int launch_ring(const WvDevBlob& b, const float* dx, float* dy, int batch
   if (g.nslot > RING_SLOTS) g.nslot = RING_SLOTS;
   if (g.nslot < 2) return 1;
   g.red_off = slot * g.nslot * g.s * g.ngrp;
+#ifdef WV_DEV_HOOKS
+  g.stall = g_ring_stall; g.spin = g_ring_spin;
+#endif
   const size_t smem = g.red_off + red;
   if constexpr (DT == WV_DT_F32) if (c == 2) return launch_ring_c<DT, 2>(b, dx, dy, batch, rb, re, g, smem, grid, st);
   return launch_ring_c<DT, 1>(b, dx, dy, batch, rb, re, g, smem, grid, st);
