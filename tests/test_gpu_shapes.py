@@ -322,3 +322,48 @@ def test_plain_rows_after_a_wait_that_runs_out(wv, hooks, dt, rows, cols, row):
         assert status == 0 and torch.equal(y, want)
     finally:
         L.wv_blob_evict(key)
+
+
+@pytest.mark.parametrize("fmt,cols", [("Q5_K", 16384), ("Q5_K", 16128), ("Q6_K", 15872), ("Q6_K", 30720), ("Q5_1", 15104), ("Q8_0", 12672)])
+def test_widths_where_the_staged_x_has_no_padding(wv, fmt, cols):
+    """The one-row kernel at the widths where only an unpadded copy of x leaves three stages (and next to them), alone, with a residual
+    and with the RMSNorm in its prologue, aligned and unaligned, against float64 over the dequantised weights: an activation is off
+    by at most 1 / 65024 of its chunk's largest, to which come 2^-20 of sum |w x| for the float32 steps."""
+    import ctypes as C
+
+    import torch
+    from welvet_b200 import _lib
+    from welvet_b200.decode import MatVecFusedCUDA, RMSNormCUDA
+    L, check, key, rows = _lib.lib(), _lib.check, 0x7300, 1400
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    w = torch.randn(rows * cols, device="cuda", generator=gen) * 0.02
+    torch.cuda.synchronize()
+    check(L.wv_pack_upload_dev(key, O.FMT[fmt], 1, 0, w.data_ptr(), rows, cols, None))
+    try:
+        d = torch.zeros(rows, cols, device="cuda")
+        check(L.wv_unpack_dev(key, d.data_ptr(), None))
+        buf = torch.randn(cols + 1, device="cuda", generator=gen)
+        gamma = 1 + 0.1 * torch.randn(cols, device="cuda", generator=gen)
+        res = torch.randn(rows, device="cuda", generator=gen)
+        torch.cuda.synchronize()
+        d = d.double()
+
+        def close(y, x, plus=0.0):
+            x = x.double()
+            step = x.abs().view(-1, 32).amax(1).repeat_interleave(32) / 65024
+            return bool(((y.double() - plus - d @ x).abs() <= d.abs() @ (1.01 * step + 2.0 ** -20 * x.abs()) + 1e-6).all())
+        for off in (0, 1):
+            x = buf[off:off + cols]
+            y, z, n, xn = (torch.full((k,), float("nan"), device="cuda") for k in (rows, rows, rows, cols))
+            torch.cuda.synchronize()
+            check(L.wv_matvec_dev(key, x.data_ptr(), y.data_ptr(), 1, cols, rows, None))
+            check(L.wv_matvec_dev_add(key, x.data_ptr(), res.data_ptr(), z.data_ptr(), cols, rows, None))
+            RMSNormCUDA(x.data_ptr(), gamma.data_ptr(), xn.data_ptr(), 1, cols, 1e-5)
+            if cols <= 16384:      # the norm needs the whole row of x at once
+                MatVecFusedCUDA((C.c_uint64 * 1)(key), x.data_ptr(), (C.c_void_p * 1)(n.data_ptr()), cols, (C.c_int * 1)(rows), dnorm_gamma=gamma.data_ptr(), norm_eps=1e-5)
+            torch.cuda.synchronize()
+            assert close(y, x) and close(z, x, res.double())
+            assert cols > 16384 or close(n, xn)
+        assert L.wv_device_status() == 0
+    finally:
+        L.wv_blob_evict(key)

@@ -24,7 +24,16 @@
 #include <mutex>
 #include <tuple>
 
-#define TMA_XPITCH 36   // floats per staged chunk of x: the 16-byte accesses of eight neighbouring chunks fall into different banks
+// Staged x: the 16-byte accesses of eight neighbouring chunks have to fall into different banks. Padded: nine 16-byte vectors per chunk, of
+// which eight are used. Packed (PK): eight per chunk, chunk c's piece p at place p ^ (c & 7); a variant of its own, since the exchanged
+// addresses cost up to 1 % (IQ4_NL 4096 x 14336 13.8 -> 14.0 us).
+template <bool PK> __device__ __forceinline__ int x_place(int v) { return PK ? v ^ ((v >> 3) & 7) : v + (v >> 3); }      // of the row's vector v
+// The formats whose tiles are large enough for the padding to take the third of three stages from the ring: Q8_0, Q5_1, Q5_K, Q6_K.
+__host__ __device__ constexpr bool tma_packs_x(int f) {
+  const WvFmtInfo fi = wv_fmt_info(f);
+  const int par = fi.kind == WK_CLASSIC ? (fi.has_min ? 8 : 4) : (fi.kind == WK_KQUANT ? (fi.has_min ? 5 : 3) : (fi.pgroup == 16 ? 8 : 4));
+  return (fi.bits_lo + fi.bits_hi) * 4 + par > 24;      // bytes of 32 weights
+}
 struct TmaGeom {
   int cpr;           // chunks per row
   int nwc;           // column warps per row (ceil(cpr/32))
@@ -37,7 +46,7 @@ struct TmaGeom {
   int rows_base, rows_rem;  // single matrix: CTA b owns rows_base (+1 if b < rows_rem) consecutive rows
   int lead;          // tiles issued before the producer waits for the activation loads to be on their way
   int force3;        // development switch: always use the 24-bit activation records
-  unsigned x_off;    // staged activations: TMA_XPITCH floats per chunk
+  unsigned x_off;    // staged activations
   unsigned red_off;  // float red[2][nrg][nwc][32]
   unsigned gate_off; // gate | up launches: the gate's row sums of this CTA's band (TMA_GATE_ROWS floats)
   unsigned bar_off;  // full[nstage], empty[nstage]
@@ -83,7 +92,7 @@ template <> struct TmaExtArgs<true> { using type = TmaExt; };
 static int* g_err_host = nullptr;
 static int* g_err_dev = nullptr;
 
-template <int F, int RT, bool PREFETCH, bool EXT, bool MP = false, bool NORM = false>   // MP: column passes (rows wider than 16384 columns); NORM: RMSNorm of x in the prologue
+template <int F, int RT, bool PREFETCH, bool EXT, bool MP = false, bool NORM = false, bool PK = false>   // MP: column passes (rows wider than 16384 columns); NORM: RMSNorm of x in the prologue; PK: x_place
 __global__ void __launch_bounds__(TMA_THREADS, 1)
 gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* __restrict__ xf, float* __restrict__ y,
                 int row_begin, int row_end, const TmaGeom g, int* __restrict__ err, const typename TmaExtArgs<EXT>::type ext) {
@@ -305,14 +314,14 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
         const int i0 = tid + u * TMA_CONSUMER_WARPS * 32;
         int i = i0 + rot;
         if (i >= nv) i -= nv;
-        if (i0 < nv) *reinterpret_cast<float4*>(xs + (i >> 3) * TMA_XPITCH + (i & 7) * 4) = v[u];
+        if (i0 < nv) reinterpret_cast<float4*>(xs)[x_place<PK>(i)] = v[u];
       }
     } else {
       if (lane == 0) asm volatile("red.relaxed.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(&s_xissued)) : "memory");
       double ss = 0.0;
       for (int i = tid; i < g.cpr * 32; i += TMA_CONSUMER_WARPS * 32) {
         const float xv1 = __ldg(xrow + i);
-        xs[(i >> 5) * TMA_XPITCH + (i & 31)] = xv1;
+        xs[x_place<PK>(i >> 2) * 4 + (i & 3)] = xv1;
         if constexpr (NORM) ss += (double)xv1 * (double)xv1;
       }
       if constexpr (NORM) {
@@ -497,10 +506,12 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     }
   };
 
-  float4* xc = reinterpret_cast<float4*>(smem + g.x_off) + (size_t)(live ? c : 0) * (TMA_XPITCH / 4);
+  const int xch = live ? c : 0;
+  float4* xc = reinterpret_cast<float4*>(smem + g.x_off) + (size_t)xch * (PK ? 8 : 9);
+  const int xsw = PK ? xch & 7 : 0;
   auto chunk_x = [&](float (&xv)[32]) {      // this lane's chunk
 #pragma unroll
-    for (int q = 0; q < 8; q++) { const float4 t = xc[q]; xv[4 * q] = t.x; xv[4 * q + 1] = t.y; xv[4 * q + 2] = t.z; xv[4 * q + 3] = t.w; }
+    for (int q = 0; q < 8; q++) { const float4 t = xc[q ^ xsw]; xv[4 * q] = t.x; xv[4 * q + 1] = t.y; xv[4 * q + 2] = t.z; xv[4 * q + 3] = t.w; }
   };
   for (cp = 0; cp < npass; cp++) {
   copy_x();
@@ -514,9 +525,9 @@ gemv_tma_kernel(const WvDevBlob b, const uint4* __restrict__ xqg, const float* _
     if (rg == 0 && live) {
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        float4 t = xc[k];
+        float4 t = xc[k ^ xsw];
         t.x = (t.x * inv) * gam[k].x; t.y = (t.y * inv) * gam[k].y; t.z = (t.z * inv) * gam[k].z; t.w = (t.w * inv) * gam[k].w;
-        xc[k] = t;
+        xc[k ^ xsw] = t;
       }
     }
     asm volatile("bar.sync 14, %0;" ::"r"(nactive * 32) : "memory");
@@ -697,15 +708,27 @@ static int launch_tma(const WvDevBlob* bl, int nb, const float* dx, float* const
   unsigned off = 0;
   for (int i = 0; i < 5; i++) { g.off[i] = off; off = align128(off + g.rb[i] * g.tr); }
   g.stage_bytes = off;
-  const unsigned xbytes = align128((unsigned)g.cpr * TMA_XPITCH * 4u);
   const WvFuse* fuse = wv_cur_fuse;
   const bool gated = fuse && fuse->mode == 1;
   const unsigned gate_bytes = gated ? TMA_GATE_ROWS * 4u : 0u;
   const unsigned part_bytes = g.ncp > 1 ? (unsigned)nb * TMA_GATE_ROWS * 4u : 0u;
-  const unsigned fixed = xbytes + align128(2u * g.nrg * g.nwc * 32 * 4 + (fi.table ? 65536u : 0u)) + gate_bytes + part_bytes + 2 * TMA_MAX_STAGES * 8 + 128;
+  const unsigned fixed = align128(2u * g.nrg * g.nwc * 32 * 4 + (fi.table ? 65536u : 0u)) + gate_bytes + part_bytes + 2 * TMA_MAX_STAGES * 8 + 128;
   const unsigned avail = 225u * 1024u;  // 227 KB per CTA minus static shared memory and slack
-  if (g.stage_bytes * 2 + fixed > avail) return 1;
-  int ns = (int)((avail - fixed) / g.stage_bytes);
+  unsigned xbytes = align128((unsigned)g.cpr * 144u);
+  auto stages = [&](unsigned xb) { return fixed + xb < avail ? (int)((avail - fixed - xb) / g.stage_bytes) : 0; };
+  int ns = stages(xbytes);
+  // Without padding where that gives the ring a third stage and the CTA has tiles for it. us per launch, two stages / three: Q5_K 4096 x
+  // 16384 12.3 / 11.0, Q5_1 4096 x 15360 12.1 / 11.1, Q8_0 4096 x 12800 11.5 / 11.0; 512 x 16384 (one tile) 4.8 / 5.0. A fourth and
+  // further stages gain nothing (Q6_K 4096 x 12800, three / four: 9.9 / 10.2).
+  bool packed = false;
+  if constexpr (tma_packs_x(F) && RT == 4 && !PF) {
+    const int sms = wv_sm_count();
+    int tiles = 0;
+    for (int i = 0; i < nb; i++) tiles += ((nb == 1 ? re - rb_ : bl[i].rows) / sms + g.tr) / g.tr;
+    packed = g.ncp == 1 && ns < 3 && tiles > 2 && stages((unsigned)g.cpr * 128u) > ns;
+    if (packed) { xbytes = (unsigned)g.cpr * 128u; ns = stages(xbytes); }
+  }
+  if (ns < 2) return 1;
   if (ns > TMA_MAX_STAGES) ns = TMA_MAX_STAGES;
   if (g_tma_stages % 100 > 1 && g_tma_stages % 100 < ns) ns = g_tma_stages % 100;
   g.lead = g_tma_stages >= 100 ? g_tma_stages / 100 : 1;
@@ -739,20 +762,25 @@ static int launch_tma(const WvDevBlob* bl, int nb, const float* dx, float* const
   }
   if (nb == 1 && !wv_cur_peers && !fuse && g.ncp == 1) {
     auto kern = gemv_tma_kernel<F, RT, PF, false>;
-    static unsigned attr_mask = 0;
-    if (!(attr_mask & (1u << dev))) {
+    if constexpr (tma_packs_x(F) && RT == 4 && !PF) if (packed) kern = gemv_tma_kernel<F, RT, PF, false, false, false, true>;
+    static unsigned attr_mask[2] = {0, 0};
+    if (!(attr_mask[packed] & (1u << dev))) {
       if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) { wv_set_error("gemv (tma): cannot raise the shared-memory limit"); return WV_ECUDA; }
-      attr_mask |= 1u << dev;
+      attr_mask[packed] |= 1u << dev;
     }
     e = launch_pdl(kern, dim3(grid, batch), dim3(TMA_THREADS), smem, st, b, xq, dx, dys[0], rb_, re, g, g_err_dev, TmaNoExt{});
   } else {
     if constexpr (RT == 4 && !PF) {   // the grouped / peer-storing variant exists for the default configuration only
       const bool norm = fuse && fuse->norm_gamma;
       if (norm && g.ncp > 1) return WV_ESHAPE;      // the fused norm needs the whole row of x at once
-      const int variant = g.ncp > 1 ? 1 : (norm ? 2 : 0);
+      const int variant = g.ncp > 1 ? 1 : (norm ? 2 : 0) + (packed ? 3 : 0);
       auto kern = variant == 1 ? gemv_tma_kernel<F, RT, PF, true, true, false>
                 : variant == 2 ? gemv_tma_kernel<F, RT, PF, true, false, true> : gemv_tma_kernel<F, RT, PF, true, false, false>;
-      static unsigned attr_mask[3] = {0, 0, 0};
+      if constexpr (tma_packs_x(F)) {
+        if (variant == 3) kern = gemv_tma_kernel<F, RT, PF, true, false, false, true>;
+        if (variant == 5) kern = gemv_tma_kernel<F, RT, PF, true, false, true, true>;
+      }
+      static unsigned attr_mask[6] = {0, 0, 0, 0, 0, 0};
       if (!(attr_mask[variant] & (1u << dev))) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) { wv_set_error("gemv (tma): cannot raise the shared-memory limit"); return WV_ECUDA; }
         attr_mask[variant] |= 1u << dev;
