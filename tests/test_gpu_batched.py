@@ -132,6 +132,20 @@ def test_dense_forward_bias_and_activations(wv, rows, cols, batch, nbias):
         assert np.all(np.abs(post - ref) <= 2.0 ** -23 * np.abs(ref) + 2.0 ** -49 * np.abs(p) + 1e-45), act
 
 
+@pytest.mark.parametrize("as_type", [float, np.float32, np.int64, int])
+def test_dense_forward_activation_value_types(wv, as_type):
+    """An activation equal to one of the eight values is that activation, whatever numeric type a program read it into."""
+    d = wv.dense
+    rng = np.random.default_rng(3)
+    layer = d.NewConfigured(64, 24, d.ActivationLinear, wv.quant.DTypeFloat32, wv.quant.Format.FormatQ8_0, rng.normal(0, 1, 24 * 64).astype(np.float32))
+    x = rng.standard_normal((3, 64), np.float32)
+    y = d.Forward(layer, x)[0]
+    layer.Activation = as_type(d.ActivationReLU2)
+    pre, post = d.Forward(layer, x)
+    np.testing.assert_array_equal(pre, y)
+    np.testing.assert_array_equal(post, np.where(y < 0, 0, y.astype(np.float64) ** 2).astype(np.float32))
+
+
 @pytest.mark.parametrize("rows,cols,batch", [(32, 32, 65537), (160, 64, 27000)])
 def test_dense_forward_bias_and_activation_of_large_batches(wv, rows, cols, batch):
     """More rows than a grid has in y, and more results than the pinned buffer takes at a time (4 Mi floats): every row is the plain

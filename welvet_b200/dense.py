@@ -126,7 +126,7 @@ def ForwardCUDA(l: Layer, input: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
             return pre, pre
         post = np.empty((batch, out), np.float32)
         b = np.ascontiguousarray(bias, np.float64).reshape(-1) if bias is not None and len(bias) else None
-        check(lib().wv_matvec_bias_act(key, xs.ctypes.data, None if b is None else b.ctypes.data, 0 if b is None else b.size, l.Activation,
+        check(lib().wv_matvec_bias_act(key, xs.ctypes.data, None if b is None else b.ctypes.data, 0 if b is None else b.size, int(l.Activation),
                                        pre.ctypes.data, post.ctypes.data, batch, in_, out))
         return pre, post
     y = np.empty(batch * out, np.float32)
