@@ -422,3 +422,28 @@ def test_batched_graphs_come_and_go(wv):
         torch.cuda.synchronize()
         assert torch.equal(got, y), batch
     assert L.wv_device_status() == 0
+
+
+@pytest.mark.parametrize("fmt,rows,cols", [("Q4_0", 333, 512), ("Q4_K", 700, 2048), ("Q8_0", 130, 254)])
+def test_dense_forward_one_row_again_and_again(wv, fmt, rows, cols):
+    """A layer with bias and activation called row by row: from the second call on one graph launch serves it. New x and new bias values
+    every time, two activations and two bias lengths in turn, a larger batch that moves the slot's buffers and a matrix that is
+    evicted and uploaded again in between. The bits are the plain product's plus the bias."""
+    d = wv.dense
+    rng = np.random.default_rng(rows)
+    layer = d.NewConfigured(cols, rows, d.ActivationReLU, wv.quant.DTypeFloat32, wv.quant.Format["Format" + fmt], rng.normal(0, 0.1, rows * cols).astype(np.float32))
+    for step in range(30):
+        x = rng.standard_normal((40 if step == 12 else 1, cols), np.float32)
+        if step % 10 == 0:
+            layer.Activation = (d.ActivationReLU, d.ActivationLeakyReLU, d.ActivationReLU)[step // 10]
+        bias = rng.normal(0, 1, rows if step < 24 else 7)
+        layer.Weights.Bias, act = None, layer.Activation
+        layer.Activation = d.ActivationLinear
+        want = d.Forward(layer, x)[0].astype(np.float64)
+        want[:, :len(bias)] += bias
+        layer.Weights.Bias, layer.Activation = bias, act
+        if step == 16:
+            wv._lib.lib().wv_blob_evict(wv.quant.EnsureResident(layer.Weights.Packed))
+        pre, post = d.Forward(layer, x)
+        np.testing.assert_array_equal(pre, want.astype(np.float32))
+        np.testing.assert_array_equal(post, d.Activate(pre, act).astype(np.float32))

@@ -792,7 +792,13 @@ static int grow(float** p, size_t* cap, size_t n, bool pinned) {
 // of two kernel launches leaves more of the GPU to the other callers. A graph is built on the second call for a matrix
 // (the first one may still set kernel attributes), only for the batch-1 kernels that use no scratch from the shared
 // arena, and is dropped when the key is re-uploaded or the slot's buffers move.
-struct SlotGraph { uint64_t gen = 0; cudaGraphExec_t exec = nullptr; int seen = 0; };
+struct SlotGraph { uint64_t gen = 0, form = 0; cudaGraphExec_t exec = nullptr; int seen = 0; };      // form: what else the launches depend on
+struct SlotGraphs : std::unordered_map<uint64_t, SlotGraph> {
+  void drop() {
+    for (auto& kv : *this) if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+    clear();
+  }
+};
 struct StageSlot {
   std::mutex mu;
   cudaStream_t st = nullptr;
@@ -800,11 +806,7 @@ struct StageSlot {
   size_t hx_n = 0, dx_n = 0, hy_n = 0;
   float *ax = nullptr, *ax_dev = nullptr, *da = nullptr, *ay = nullptr, *ay_dev = nullptr;   // wv_matvec_bias_act: its inputs, device side, results
   size_t ax_n = 0, da_n = 0, ay_n = 0;
-  std::unordered_map<uint64_t, SlotGraph> graphs;
-  void drop_graphs() {
-    for (auto& kv : graphs) if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
-    graphs.clear();
-  }
+  SlotGraphs graphs, act_graphs;      // wv_matvec's and wv_matvec_bias_act's
 };
 #define WV_STAGE_SLOTS 8
 static StageSlot g_slots[WV_STAGE_SLOTS];
@@ -863,6 +865,31 @@ static void abandon(StageSlot& slot, const char* who, int rc) {
   cudaStreamSynchronize(slot.st);
 }
 
+// Enqueues a batch-1 call's launches on the slot's stream, as one graph launch from the second time on.
+template <class E>
+static int enqueue_one_row(StageSlot& slot, SlotGraphs& graphs, uint64_t key, const Entry& e, uint64_t form, E&& enqueue) {
+  if (!e.blob.fast || e.blob.format == WV_NONE || e.blob.cols > 16384) return enqueue();
+  if (graphs.size() >= 512 && !graphs.count(key)) graphs.drop();   // bound what a slot keeps
+  SlotGraph& sg = graphs[key];
+  if (sg.gen != e.gen || sg.form != form) { if (sg.exec) cudaGraphExecDestroy(sg.exec); sg = SlotGraph{}; sg.gen = e.gen; sg.form = form; }
+  if (!sg.exec && sg.seen == 1) {
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamBeginCapture(slot.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      const int crc = enqueue();
+      const cudaError_t ce = cudaStreamEndCapture(slot.st, &graph);
+      if (crc == WV_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&sg.exec, graph, 0) != cudaSuccess) sg.exec = nullptr;
+      if (graph) cudaGraphDestroy(graph);
+    }
+    cudaGetLastError();
+    if (!sg.exec) sg.seen = 2;      // could not be captured: this matrix stays on plain launches
+  }
+  if (sg.exec) {
+    if (cudaGraphLaunch(sg.exec, slot.st) == cudaSuccess) return WV_OK;
+    cudaGetLastError(); cudaGraphExecDestroy(sg.exec); sg.exec = nullptr; sg.seen = 2;
+  } else if (sg.seen == 0) sg.seen = 1;
+  return enqueue();
+}
+
 extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int in, int out) {
   int rc = ensure_init();
   if (rc) return rc;
@@ -874,7 +901,7 @@ extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int 
   StageSlot* slot = nullptr;
   if ((rc = take_slot(batch, &slot))) return rc;
   std::lock_guard<std::mutex> lk(slot->mu, std::adopt_lock);
-  if (slot->hx_n < nx || slot->dx_n < nx || slot->hy_n < ny) slot->drop_graphs();   // the buffers are about to move
+  if (slot->hx_n < nx || slot->dx_n < nx || slot->hy_n < ny) slot->graphs.drop();   // the buffers are about to move
   if ((rc = grow_mapped(&slot->hx, &slot->hx_dev, &slot->hx_n, nx)) || (rc = grow(&slot->dx, &slot->dx_n, nx, false)) ||
       (rc = grow_mapped(&slot->hy, &slot->hy_dev, &slot->hy_n, ny))) return rc;
   memcpy(slot->hx, x, nx * 4);
@@ -888,32 +915,8 @@ extern "C" int wv_matvec(uint64_t key, const float* x, float* y, int batch, int 
     if (cudaGetLastError() != cudaSuccess) return WV_ECUDA;
     return wv_launch_gemv(e.blob, slot->dx, slot->hy_dev, batch, 0, e.blob.rows, slot->st);
   };
-  const bool graphable = batch == 1 && e.blob.fast && e.blob.format != WV_NONE && e.blob.cols <= 16384;
-  bool launched = false;
-  if (graphable) {
-    if (slot->graphs.size() >= 512 && !slot->graphs.count(key)) slot->drop_graphs();   // bound what a slot keeps
-    SlotGraph& sg = slot->graphs[key];
-    if (sg.gen != e.gen) { if (sg.exec) cudaGraphExecDestroy(sg.exec); sg = SlotGraph{}; sg.gen = e.gen; }
-    if (!sg.exec && sg.seen == 1) {
-      cudaGraph_t graph = nullptr;
-      if (cudaStreamBeginCapture(slot->st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const int crc = enqueue();
-        const cudaError_t ce = cudaStreamEndCapture(slot->st, &graph);
-        if (crc == WV_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&sg.exec, graph, 0) != cudaSuccess) sg.exec = nullptr;
-        if (graph) cudaGraphDestroy(graph);
-      }
-      cudaGetLastError();
-      if (!sg.exec) sg.seen = 2;      // could not be captured: this matrix stays on plain launches
-    }
-    if (sg.exec) {
-      if (cudaGraphLaunch(sg.exec, slot->st) == cudaSuccess) launched = true;
-      else { cudaGetLastError(); cudaGraphExecDestroy(sg.exec); sg.exec = nullptr; sg.seen = 2; }
-    } else if (sg.seen == 0) sg.seen = 1;
-  }
-  if (!launched) {
-    rc = enqueue();
-    if (rc) { abandon(*slot, "wv_matvec", rc); return rc; }
-  }
+  rc = batch == 1 ? enqueue_one_row(*slot, slot->graphs, key, e, 0, enqueue) : enqueue();
+  if (rc) { abandon(*slot, "wv_matvec", rc); return rc; }
   CUDA_TRY(cudaStreamSynchronize(slot->st));
   if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
   memcpy(y, slot->hy, ny * 4);
@@ -935,20 +938,26 @@ __device__ __forceinline__ double activate(double v, int act) {
   }
   return v;
 }
-// A thread per output, bias[out] from device memory; both results go straight to mapped host memory. Bound by those stores: 0.9 MB
+// A thread per output; both results go straight to mapped host memory. Bound by those stores: 0.9 MB
 // over a 50 GB/s host link are 18 us at 8 rows of 14336 outputs. On the host the same float64 passes took 0.45 of the call's 0.55 ms.
 // A launch takes a slice of the rows: WV_ACT_ROWS of them at most (they are the grid's y, which ends at 65535) and, unless one row is
 // more, WV_ACT_FLOATS results, so that the pinned buffer does not grow with the batch.
 #define WV_ACT_ROWS 32768
 #define WV_ACT_FLOATS (4 << 20)
-__global__ void __launch_bounds__(256) bias_act_kernel(const float* __restrict__ y, const double* __restrict__ bias, int nbias, int act, float* __restrict__ pre,
-                                                       float* __restrict__ post, int out) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+// The bias of a single row is read from mapped host memory (early), where it lies before the call's first launch, beside the GEMV;
+// several rows read it from device memory. Brought over in front of the GEMV, and with three launches instead of one of a graph, a
+// linear layer with a bias took 30.3 us a call at 256 x 256 and 36.2 at 4096 x 4096 in Q4_0, now 21.4 and 28.8.
+__global__ void __launch_bounds__(256) bias_act_kernel(const float* __restrict__ y, const double* __restrict__ bias, int nbias, int early, int act,
+                                                       float* __restrict__ pre, float* __restrict__ post, int out) {
   const int c = blockIdx.x * 256 + threadIdx.x;
+  double b = 0.0;
+  if (early && c < nbias) b = __ldcv(bias + c);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (c >= out) return;
+  if (!early && c < nbias) b = bias[c];
   const size_t i = (size_t)blockIdx.y * out + c;
   float p = y[i];
-  if (c < nbias) p = (float)((double)p + bias[c]);
+  if (c < nbias) p = (float)((double)p + b);
   pre[i] = p;
   post[i] = (float)activate((double)p, act);
 }
@@ -966,25 +975,39 @@ extern "C" int wv_matvec_bias_act(uint64_t key, const float* x, const double* bi
   StageSlot* slot = nullptr;
   if ((rc = take_slot(batch, &slot))) return rc;
   std::lock_guard<std::mutex> lk(slot->mu, std::adopt_lock);
-  // x and the bias behind it in one pinned buffer, brought over together; W x stays on the device
+  // x and the bias behind it in one pinned buffer, brought over together (a single row's bias stays there); W x stays on the device
+  const bool early = batch == 1;
   const size_t nx = (size_t)batch * in, ny = (size_t)batch * out, xpad = (nx + 3) & ~(size_t)3, nin = xpad + 2 * (size_t)nbias;
   const size_t npad = (nin + 3) & ~(size_t)3;
   int slice = WV_ACT_FLOATS / out;
   slice = slice < 1 ? 1 : (slice > WV_ACT_ROWS ? WV_ACT_ROWS : slice);
   if (slice > batch) slice = batch;
   const size_t ns = (size_t)slice * out;
+  if (slot->ax_n < npad || slot->da_n < npad + ny || slot->ay_n < 2 * ns) slot->act_graphs.drop();
   if ((rc = grow_mapped(&slot->ax, &slot->ax_dev, &slot->ax_n, npad)) || (rc = grow(&slot->da, &slot->da_n, npad + ny, false)) ||
       (rc = grow_mapped(&slot->ay, &slot->ay_dev, &slot->ay_n, 2 * ns))) return rc;
   memcpy(slot->ax, x, nx * 4);
   if (nbias) memcpy(slot->ax + xpad, bias, (size_t)nbias * 8);
-  const int n4 = (int)(npad / 4);
-  const int blocks = n4 < 256 ? 1 : (n4 / 256 < 64 ? n4 / 256 : 64);
-  stage_in_kernel<<<blocks, 256, 0, slot->st>>>(reinterpret_cast<const float4*>(slot->ax_dev), reinterpret_cast<float4*>(slot->da), n4, nullptr, nullptr, 0);
-  rc = cudaGetLastError() == cudaSuccess ? wv_launch_gemv(e.blob, slot->da, slot->da + npad, batch, 0, e.blob.rows, slot->st) : WV_ECUDA;
+  auto product = [&]() -> int {
+    const int n4 = (int)((early ? xpad : npad) / 4);
+    const int blocks = n4 < 256 ? 1 : (n4 / 256 < 64 ? n4 / 256 : 64);
+    stage_in_kernel<<<blocks, 256, 0, slot->st>>>(reinterpret_cast<const float4*>(slot->ax_dev), reinterpret_cast<float4*>(slot->da), n4, nullptr, nullptr, 0);
+    if (cudaGetLastError() != cudaSuccess) return WV_ECUDA;
+    return wv_launch_gemv(e.blob, slot->da, slot->da + npad, batch, 0, e.blob.rows, slot->st);
+  };
+  auto finish = [&](int r0, int nr) -> int {
+    const double* b = reinterpret_cast<const double*>((early ? slot->ax_dev : slot->da) + xpad);
+    return launch_pdl(bias_act_kernel, dim3((out + 255) / 256, nr), dim3(256), 0, slot->st, slot->da + npad + (size_t)r0 * out, b, nbias, (int)early, act,
+                      slot->ay_dev, slot->ay_dev + ns, out) == cudaSuccess ? WV_OK : WV_ECUDA;
+  };
+  auto enqueue = [&]() -> int {      // up to the first slice of the results
+    const int prc = product();
+    return prc ? prc : finish(0, slice);
+  };
+  rc = early ? enqueue_one_row(*slot, slot->act_graphs, key, e, (uint64_t)nbias << 8 | (uint64_t)(act + 1), enqueue) : enqueue();
   for (int r0 = 0; !rc && r0 < batch; r0 += slice) {
     const int nr = batch - r0 < slice ? batch - r0 : slice;
-    if (launch_pdl(bias_act_kernel, dim3((out + 255) / 256, nr), dim3(256), 0, slot->st, slot->da + npad + (size_t)r0 * out,
-                   reinterpret_cast<const double*>(slot->da + xpad), nbias, act, slot->ay_dev, slot->ay_dev + ns, out) != cudaSuccess) { rc = WV_ECUDA; break; }
+    if (r0 && (rc = finish(r0, nr))) break;
     CUDA_TRY(cudaStreamSynchronize(slot->st));
     if (int te = wv_tma_take_error()) { wv_set_error("wv_matvec_bias_act: a bounded device wait ran out (code %d)", te); return WV_ETIMEOUT; }
     memcpy(pre + (size_t)r0 * out, slot->ay, (size_t)nr * out * 4);
