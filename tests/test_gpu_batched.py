@@ -447,3 +447,91 @@ def test_dense_forward_one_row_again_and_again(wv, fmt, rows, cols):
         pre, post = d.Forward(layer, x)
         np.testing.assert_array_equal(pre, want.astype(np.float32))
         np.testing.assert_array_equal(post, d.Activate(pre, act).astype(np.float32))
+
+
+@pytest.mark.parametrize("n,batch", [(256, 8), (1024, 33), (4096, 6), (1280, 256)])
+def test_batched_calls_in_a_chain(wv, n, batch):
+    """Each batched call's X is the Y of the call right before it on the stream, with another batched call behind: the kernel that rounds
+    X lets the next one start before its own wait. The same bits as with a synchronisation behind every call."""
+    L, check = wv._lib.lib(), wv._lib.check
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    keys = [0x7400, 0x7401, 0x7402]
+    x = torch.randn(batch, n, device="cuda", generator=gen)
+    stream = torch.cuda.Stream()
+
+    def chain(wait):
+        ys = [torch.full((batch, n), float("nan"), device="cuda") for _ in range(12)]
+        torch.cuda.synchronize()
+        for i, y in enumerate(ys):
+            check(L.wv_matvec_dev(keys[i % 3], (ys[i - 1] if i else x).data_ptr(), y.data_ptr(), batch, n, n, stream.cuda_stream))
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return torch.stack(ys)
+    try:
+        for key, f in zip(keys, ("Q8_0", "Q4_K", "Q4_0")):
+            w = torch.randn(n, n, device="cuda", generator=gen) / n ** 0.5
+            torch.cuda.synchronize()
+            check(L.wv_pack_upload_dev(key, O.FMT[f], 1, 0, w.data_ptr(), n, n, None))
+        want = chain(True)
+        assert bool(want.isfinite().all())
+        for _ in range(5):
+            assert torch.equal(chain(False), want)
+        assert L.wv_device_status() == 0
+    finally:
+        for key in keys:
+            L.wv_blob_evict(key)
+
+
+@pytest.mark.parametrize("fmt", ["Q4_0", "Q5_K", "Q8_0", "IQ3_S"])
+@pytest.mark.parametrize("shape", [(130, 256), (129, 4352)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_batched_rounds_of_stages(wv, fmt, shape):
+    """Either side of the line between two rounds of pipeline stages and one (192 rows), as in test_batched_column_orders."""
+    rows, cols = shape
+    ob = O.pack(fmt, np.random.default_rng(cols).normal(0, 0.02, rows * cols).astype(np.float32), rows, cols)
+    wd = O.unpack(ob).reshape(rows, cols).astype(np.float64)
+    for batch in (177, 192, 193, 208):
+        x = np.random.default_rng(batch).normal(0, 1, (batch, cols)).astype(np.float32)
+        y, _ = _run(wv, ob, x)
+        assert np.all(np.abs(y - x.astype(np.float64) @ wd.T) <= 9.9e-4 * (np.abs(x).astype(np.float64) @ np.abs(wd).T) + 1e-30), batch
+
+
+@pytest.mark.parametrize("batch", [1, 3, 8])
+def test_dense_forward_non_finite_and_threads(wv, batch):
+    """Bias and activation on the device with infinities and NaN in x and in the bias, from four threads at once: where the float64
+    passes of dense.Activate give an infinity or a NaN the device does, elsewhere the bounds of the test above hold."""
+    import threading
+    d, rows, cols = wv.dense, 300, 512
+    errors = []
+
+    def worker(seed):
+        try:
+            rng = np.random.default_rng(seed)
+            layer = d.NewConfigured(cols, rows, d.ActivationLinear, wv.quant.DTypeFloat32, wv.quant.Format.FormatQ4_0, rng.normal(0, 0.1, rows * cols).astype(np.float32))
+            x = rng.normal(0, 1, (batch, cols)).astype(np.float32)
+            if seed % 2:
+                x[-1, 7] = (np.inf, np.nan)[seed // 2]
+            y = d.Forward(layer, x)[0].astype(np.float64)
+            bias = rng.normal(0, 3, rows)
+            bias[[3, 50, 299]], bias[[7, 8]] = (np.inf, -np.inf, np.nan), (3e38, -3e38)
+            layer.Weights.Bias = bias
+            with np.errstate(all="ignore"):
+                want = (y + bias).astype(np.float32)
+                for act in d._ACTIVATIONS * 3:
+                    layer.Activation = act
+                    pre, post = d.Forward(layer, x)
+                    np.testing.assert_array_equal(pre, want)
+                    p = pre.astype(np.float64)
+                    ref = d.Activate(p, act).astype(np.float32)
+                    ok = np.isfinite(ref)
+                    np.testing.assert_array_equal(post[~ok], ref[~ok])
+                    exact = d.Activate(p, act)[ok]
+                    assert np.all(np.abs(post[ok] - exact) <= 2.0 ** -23 * np.abs(exact) + 2.0 ** -49 * np.abs(p[ok]) + 1e-45), act
+        except BaseException as e:      # noqa: BLE001
+            errors.append(e)
+    threads = [threading.Thread(target=worker, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
