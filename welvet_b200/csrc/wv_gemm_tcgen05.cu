@@ -808,7 +808,7 @@ static int launch_tcg(const WvDevBlob& b, const float* dx, float* dy, int batch,
     int blocks = (int)((n4 + 255) / 256);
     // Two blocks fit beside a CTA of the kernel before. Up to three turns of those they are all resident early; beyond, the copy is
     // what counts (100 rows of 6400 columns 16.0 us a call with 296 blocks, 16.2 with all; 256 of 4096 21.8 and 21.6).
-    const int beside = 2 * 148, all = 8 * 148;
+    const int beside = 2 * wv_sm_count(), all = 8 * wv_sm_count();
     if (blocks > 3 * beside) { if (blocks > all) blocks = all; }
     else if (blocks > beside) blocks = beside;
     rc_.gridDim = dim3(blocks); rc_.blockDim = dim3(256); rc_.stream = st;

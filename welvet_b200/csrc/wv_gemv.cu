@@ -356,7 +356,6 @@ __device__ __forceinline__ float plain_row_sum(float t) {
 
 #define WV_DENSE_THREADS 512
 template <int DT>
-
 __global__ void __launch_bounds__(WV_DENSE_THREADS, 2)
 gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restrict__ y, int row_begin, int row_end) {
   constexpr int EPV = PlainVec<DT>::N;

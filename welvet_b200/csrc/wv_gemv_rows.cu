@@ -349,7 +349,7 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
   if (g.nwc > TMA_CONSUMER_WARPS) return 1;
   // So few rows of W that row by row the CTAs of all activation rows run side by side, or nearly: that takes 3.6 - 4.4 us as long
   // as there is an SM for each and 6.9 - 7.9 us up to two for each, while this kernel spreads the rows of W alone over the chip
-  // and takes 2.4 - 3.2 us and 1.45 us for each of a CTA's activation rows (Q4_K, four rows: 24 x 4096 4.1 against 8.2 us,
+  // and takes 2.4 - 3.2 us and some 1.5 us for each of a CTA's activation rows (Q4_K, four rows: 24 x 4096 4.1 against 8.2 us,
   // 64 x 6144 7.5 against 9.1; three rows, 64 x 4096: 7.6 against 6.9; two rows, 128 x 9216: 7.5 against 6.9).
   const int ny = (batch + ROWS_NB - 1) / ROWS_NB, nb = (batch + ny - 1) / ny;
   const long long side = (long long)(re - rb_) * batch, sms = wv_sm_count();
@@ -404,8 +404,8 @@ static int launch_rows(const WvDevBlob& b, const float* dx, float* dy, int batch
 int wv_launch_gemv_rows(const WvDevBlob& b, const float* dx, float* dy, int batch, int row_begin, int row_end, cudaStream_t st) {
   if (batch < 2 || !b.fast || b.format == WV_NONE || row_end <= row_begin || !wv_tma_err_ptr()) return 1;
   // What runs as 24-bit records on the tensor pipe row by row (gemv_mma_kernel: Q8_0, and the formats with one parameter
-  // group per chunk up to 4096 columns) stays there whatever the shape, since two limbs would be less precise. Three would make
-  // this kernel the slower one where it was tried (Q8_0 at 4096 x 4096, four rows: 17.9 against 13.6 us).
+  // group per chunk up to 4096 columns) stays there whatever the shape, since 16-bit records would be less precise. 24-bit ones would
+  // make this kernel the slower one where it was tried (Q8_0 at 4096 x 4096, four rows: 17.9 against 13.6 us).
   const WvFmtInfo fi = wv_fmt_info(b.format);
   if (b.format == WV_Q8_0 || (b.cols <= 4096 && b.format != WV_IQ3_XXS && fi.kind != WK_KQUANT && fi.pgroup != 16)) return 1;
   switch (b.format) {
