@@ -535,3 +535,43 @@ def test_dense_forward_non_finite_and_threads(wv, batch):
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def test_host_calls_with_scratch_from_threads(wv):
+    """Widths whose kernel takes scratch for the activation records (an odd number of chunks), replayed from graphs of several slots
+    while other calls go round the shared scratch ring more than once: every call's bits are those of the first."""
+    import threading
+    d, L, check = wv.dense, wv._lib.lib(), wv._lib.check
+    rows, cols, errors = 40, 16352, []
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    w, x, y = (torch.randn(n, device="cuda", generator=gen) for n in (rows * cols, cols, rows))
+    torch.cuda.synchronize()
+    check(L.wv_pack_upload_dev(0x7500, O.FMT["Q4_0"], 1, 0, w.data_ptr(), rows, cols, None))
+    stream = torch.cuda.Stream()
+
+    def worker(seed):
+        try:
+            rng = np.random.default_rng(seed)
+            layer = d.NewConfigured(cols, rows, d.ActivationLinear, wv.quant.DTypeFloat32, wv.quant.Format.FormatQ4_0, rng.normal(0, 0.1, rows * cols).astype(np.float32))
+            xs = rng.standard_normal((4, 1, cols), np.float32)
+            bias = rng.normal(0, 1, rows)
+            want = [d.Forward(layer, v)[0] for v in xs]
+            for i in range(400):
+                layer.Weights.Bias, layer.Activation = (bias, d.ActivationReLU) if i % 3 == 0 else (None, d.ActivationLinear)
+                pre, post = d.Forward(layer, xs[i % 4])
+                np.testing.assert_array_equal(pre, (want[i % 4] + bias).astype(np.float32) if i % 3 == 0 else want[i % 4])
+                np.testing.assert_array_equal(post, np.maximum(pre, 0) if i % 3 == 0 else pre)
+        except BaseException as e:      # noqa: BLE001
+            errors.append(e)
+    threads = [threading.Thread(target=worker, args=(s,)) for s in range(3)]
+    for t in threads:
+        t.start()
+    for i in range(1200):
+        check(L.wv_matvec_dev(0x7500, x.data_ptr(), y.data_ptr(), 1, cols, rows, stream.cuda_stream))
+        if i % 50 == 49:
+            stream.synchronize()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    L.wv_blob_evict(0x7500)
+    assert not errors, errors[0]

@@ -32,6 +32,7 @@ extern "C" const char* wv_last_error(void) { return t_err; }
 
 // ---------------------------------------------------------------- session
 int wv_gemv_scratch_init(size_t bytes);  // wv_gemv.cu
+void wv_scratch_own(void* p, size_t bytes);
 int wv_tma_init();                       // wv_gemv_tma.cu
 int wv_tma_take_error();
 struct Entry {
@@ -790,8 +791,8 @@ static int grow(float** p, size_t* cap, size_t n, bool pinned) {
 // A slot also keeps one instantiated CUDA graph per matrix it has served (copy-in kernel + GEMV with the slot's fixed
 // buffers): launches from several host threads are serialised by the driver, so a call that costs one graph launch instead
 // of two kernel launches leaves more of the GPU to the other callers. A graph is built on the second call for a matrix
-// (the first one may still set kernel attributes), only for the batch-1 kernels that use no scratch from the shared
-// arena, and is dropped when the key is re-uploaded or the slot's buffers move.
+// (the first one may still set kernel attributes), for batch 1 up to 16384 columns, with scratch of the slot's own in place of the
+// shared ring's, and is dropped when the key is re-uploaded or the slot's buffers move.
 struct SlotGraph { uint64_t gen = 0, form = 0; cudaGraphExec_t exec = nullptr; int seen = 0; };      // form: what else the launches depend on
 struct SlotGraphs : std::unordered_map<uint64_t, SlotGraph> {
   void drop() {
@@ -807,8 +808,10 @@ struct StageSlot {
   float *ax = nullptr, *ax_dev = nullptr, *da = nullptr, *ay = nullptr, *ay_dev = nullptr;   // wv_matvec_bias_act: its inputs, device side, results
   size_t ax_n = 0, da_n = 0, ay_n = 0;
   SlotGraphs graphs, act_graphs;      // wv_matvec's and wv_matvec_bias_act's
+  void* own = nullptr;                // scratch of the recorded launches: records of 16384 activations take 74 KB
 };
 #define WV_STAGE_SLOTS 8
+#define WV_SLOT_SCRATCH (96u << 10)
 static StageSlot g_slots[WV_STAGE_SLOTS];
 static std::atomic<unsigned> g_slot_rr{0};
 
@@ -874,8 +877,11 @@ static int enqueue_one_row(StageSlot& slot, SlotGraphs& graphs, uint64_t key, co
   if (sg.gen != e.gen || sg.form != form) { if (sg.exec) cudaGraphExecDestroy(sg.exec); sg = SlotGraph{}; sg.gen = e.gen; sg.form = form; }
   if (!sg.exec && sg.seen == 1) {
     cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(slot.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    if (!slot.own && cudaMalloc(&slot.own, WV_SLOT_SCRATCH) != cudaSuccess) slot.own = nullptr;
+    if (slot.own && cudaStreamBeginCapture(slot.st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      wv_scratch_own(slot.own, WV_SLOT_SCRATCH);
       const int crc = enqueue();
+      wv_scratch_own(nullptr, 0);
       const cudaError_t ce = cudaStreamEndCapture(slot.st, &graph);
       if (crc == WV_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&sg.exec, graph, 0) != cudaSuccess) sg.exec = nullptr;
       if (graph) cudaGraphDestroy(graph);

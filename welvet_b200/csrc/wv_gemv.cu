@@ -567,8 +567,19 @@ int wv_gemv_scratch_init(size_t bytes) {
   g_xq_bytes = bytes; g_xq_head = 0;
   return WV_OK;
 }
+// What a host call records in a graph that it replays later takes its scratch from memory of the caller's own (p null: no longer): a
+// slot of the ring would be handed out again while the graph keeps its address.
+static thread_local unsigned char* t_own = nullptr;
+static thread_local size_t t_own_left = 0;
+void wv_scratch_own(void* p, size_t bytes) { t_own = static_cast<unsigned char*>(p); t_own_left = p ? bytes : 0; }
 uint4* wv_scratch_take(size_t bytes) {
   bytes = (bytes + 255) & ~(size_t)255;
+  if (t_own) {
+    if (bytes > t_own_left) return nullptr;
+    uint4* p = reinterpret_cast<uint4*>(t_own);
+    t_own += bytes; t_own_left -= bytes;
+    return p;
+  }
   std::lock_guard<std::mutex> lk(g_xq_mu);
   if (!g_xq_arena || bytes > g_xq_bytes) return nullptr;
   if (g_xq_head + bytes > g_xq_bytes) g_xq_head = 0;
