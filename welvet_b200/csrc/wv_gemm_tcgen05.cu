@@ -18,8 +18,9 @@
 // tensor pipe as well. With W's slices in tensor memory instead of shared memory a chunk takes two stores instead of eight and no
 // proxy fence, and shared memory holds X alone: the rest is L1, where the second half of every 128-byte line of W waits for the
 // next unit (forcing the whole carve-out on the same code: Q8_0, 33 rows, 4096 x 4096 13.8 -> 17.2 us). us per launch, slices of
-// W in shared memory and sums of one row of W at a time / now: Q8_0 4096 x 4096, 33 rows 16.7 / 13.7; Q8_0 14336 x 4096, 8 rows
-// 39.1 / 30.4; Q4_K 4096 x 4096, 128 and 256 rows 18.7 / 16.0 and 24.7 / 22.1; Q4_K 14336 x 4096, 256 rows 55.6 / 47.9.
+// W in shared memory and sums of one row of W at a time / in tensor memory, four rows at a time / and with the early start described
+// at tcg_round_x_kernel, as now: Q8_0 4096 x 4096, 33 rows 16.7 / 13.7 / 12.4; Q8_0 14336 x 4096, 8 rows 39.1 / 30.4 / 27.3; Q4_K
+// 4096 x 4096, 128 rows 18.7 / 16.0 / 15.1 and 256 rows 24.7 / 22.1 / 21.4; Q4_K 14336 x 4096, 256 rows 55.6 / 47.9 / 46.0.
 //
 // Arithmetic: X is rounded to TF32 (round to nearest, 11 significant bits) with its low bits cleared, a weight by adding half a
 // unit of the eleventh bit to it, the rest being the tensor core's truncation, which reads an operand's upper 19 bits only;
@@ -584,8 +585,8 @@ gemm_tcgen05_kernel(const WvDevBlob b, const __grid_constant__ CUtensorMap xmap,
 
 // X rounded to TF32 (round to nearest), element for element. The kernel behind it may start as soon as this one has (it waits for
 // this one's end before it reads X): its set-up and its first slices of W then run beside the preceding kernel's end and this one.
-// us per launch, started after this kernel's own wait / before it: Q8_0 4096 x 4096, 33 rows 13.7 / 12.5; Q5_1 1024 x 1024, 64 rows
-// 8.1 / 7.0; Q8_0 14336 x 4096, 8 rows 30.4 / 28.6; at 256 rows the copy itself counts (22.1 / 21.8, with more blocks 21.6).
+// us per launch, started after this kernel's own wait / before it: Q8_0 4096 x 4096, 33 rows 13.7 / 12.4; Q5_1 1024 x 1024, 64 rows
+// 8.1 / 7.3; Q8_0 14336 x 4096, 8 rows 30.4 / 27.3; at 256 rows the copy itself counts (22.1 / 21.8, with more blocks 21.4).
 __global__ void __launch_bounds__(256) tcg_round_x_kernel(const float4* __restrict__ x, float4* __restrict__ xr, size_t n4) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
