@@ -255,7 +255,7 @@ def test_plain_rows_at_the_limits_of_the_ring_kernel(wv, dt, rows, cols, batch):
         L.wv_blob_evict(key)
 
 
-@pytest.mark.parametrize("dt,rows,cols", [(1, 4096, 4096), (1, 2500, 5000), (1, 2400, 8192), (2, 2400, 2056), (2, 4096, 4096), (3, 3001, 8192)])
+@pytest.mark.parametrize("dt,rows,cols", [(1, 4096, 4096), (1, 2500, 5000), (1, 2500, 3000), (1, 2400, 8192), (2, 2400, 2056), (2, 4096, 4096), (3, 3001, 8192)])
 def test_plain_rows_do_not_depend_on_the_launch(wv, dt, rows, cols):
     """FormatNone: a row's bits are the same in the whole matrix, in a shard of its rows and with any number of rows of x, on either
     side of the line between the two kernels (2368 rows, counted once for every row of x)."""

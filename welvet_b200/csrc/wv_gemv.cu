@@ -417,8 +417,8 @@ gemv_dense_kernel(const WvDevBlob b, const float* __restrict__ x, float* __restr
 
 // ------------------------------------------------------------------ FormatNone through a shared-memory ring
 // The same product for few rows of 4 to 32 KB. Bound: latency. The kernel above gives a warp whole rows, with two steps of 2 KB in
-// flight, so that few rows leave most of its warps without work. Here a warp takes one slice of every row (two, C = 2, where a row
-// has more than eight and there are rows enough: half as many copies, each of which costs about 45 ns whatever its size), as many
+// flight, so that few rows leave most of its warps without work. Here a warp takes one slice of every row (two, C = 2, where
+// f32 rows are long and many: half as many copies, each of which costs about 45 ns whatever its size), as many
 // rows side by side as sixteen warps have room for: its part of x stays in registers, and a ring of its own brings in the slice of
 // one row after the other (lane 0 requests, before the wait for the preceding kernel what the ring holds; the warp reads: nothing
 // to wait for but its own copies). The slices' sums of a band meet in shared memory at the end, sixteen lanes to a slice.
@@ -686,9 +686,11 @@ static int launch_ring(const WvDevBlob& b, const float* dx, float* dy, int batch
   const int sms = sm_count();
   if ((long long)(re - rb) * batch > 16ll * sms) return 1;
   g.ns = (g.vpr + PLAIN_SLICE - 1) / PLAIN_SLICE;      // at most 16, and 8 for the 16-bit types
-  // Two slices a warp from about six rows of twelve slices to a CTA; below, more warps start sooner (256 x 6144 2.4 / 2.9 us, 700 x 6144
-  // 4.0 / 4.2; 1400 x 6144 7.5 / 6.4, 2000 x 4608 8.8 / 6.8 with one / two). The order of summation is the same.
-  const int c = DT == WV_DT_F32 && g.ns > 8 && (re - rb) * g.ns > 88 * sms ? 2 : 1;
+  // Two slices a warp (f32, from six slices on, but for eight, which fill the sixteen warps as they are) where an SM has some 70
+  // slices to sum, 55 of shorter rows; below, more warps start sooner. us per launch, one / two: 256 x 6144 2.4 / 2.9, 1100 x 4608
+  // 4.6 / 4.8, 1400 x 2800 3.9 / 3.9; 1600 x 3000 5.0 / 4.6, 1500 x 3400 5.4 / 4.6, 2300 x 3000 6.5 / 5.7, 900 x 6144 5.3 / 4.7, 2000 x
+  // 4608 8.8 / 6.8. The order of summation is the same.
+  const int c = DT == WV_DT_F32 && g.ns > 5 && g.ns != 8 && (re - rb) * g.ns > (g.ns > 8 ? 70 : 55) * sms ? 2 : 1;
   g.s = (g.ns + c - 1) / c;
   int grid = 2 * sms;
   if (grid > re - rb) grid = re - rb;
